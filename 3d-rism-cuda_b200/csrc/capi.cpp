@@ -112,6 +112,12 @@ void free_device(Context &c) {
   c.d_fkt = nullptr;
   delete c.ky_map;
   c.ky_map = nullptr;
+  for (void *p : {(void *)c.d_RPx, (void *)c.f_RPx, c.d_scr, (void *)c.d_roots, (void *)c.f_roots,
+                  (void *)c.d_bar})
+    if (p) cudaFree(p);
+  c.d_RPx = nullptr; c.f_RPx = nullptr; c.d_scr = nullptr; c.d_roots = nullptr; c.f_roots = nullptr;
+  c.d_bar = nullptr;
+  c.fu64.on = c.fu32.on = false;
   if (c.plan64) cufftDestroy(c.plan64);
   if (c.plan32) cufftDestroy(c.plan32);
   if (c.plan1) cufftDestroy(c.plan1);
@@ -221,7 +227,8 @@ static int alloc_state(Context &c) {
     }
   }
   {
-    const int rc = setup_pipe_r(c);
+    int rc = setup_pipe_r(c);
+    if (rc == RISM3D_OK) rc = setup_fused_iteration(c);
     if (rc != RISM3D_OK) return rc;
   }
   c.plans_ok = true;
@@ -318,8 +325,8 @@ int context_init(Context &c, const rism3d_params *p, int nb, std::string &err) {
   long long nbk = (c.n + 255) / 256;
   c.nred_blocks = (int)(nbk < 148 * 8 ? nbk : 148 * 8);
   ok = ok && cuda_ok(c, cudaMalloc(&c.d_part, sizeof(double) * 64 * c.nred_blocks * nb), "alloc partials") &&
-       cuda_ok(c, cudaMalloc(&c.d_count, sizeof(unsigned) * nb), "alloc counter") &&
-       cuda_ok(c, cudaMemset(c.d_count, 0, sizeof(unsigned) * nb), "zero counter");
+       cuda_ok(c, cudaMalloc(&c.d_count, sizeof(unsigned) * (nb + 1)), "alloc counter") &&
+       cuda_ok(c, cudaMemset(c.d_count, 0, sizeof(unsigned) * (nb + 1)), "zero counter");
   for (Timer *t : {&c.tm_setup, &c.tm_iter, &c.tm_obs}) {
     cudaEventCreate(&t->a);
     cudaEventCreate(&t->b);

@@ -1,0 +1,921 @@
+// One iteration in three kernels, with the 3D transforms folded in (cubic
+// cells whose edge N = R1 R2 has an instantiation, up to four solvent sites):
+//
+//   k_plane_a  update + closure + packing of one xy plane, x- and y-DFT
+//   k_zline    z-DFT, OZ product of every mirror pair, inverse z-DFT
+//   k_plane_r  inverse y- and x-DFT of one xy plane, residual, Gram sums,
+//              and in the last block the stopping test and AN2's 2 x 2 solve
+//
+// What bounds the iteration is bytes: the passes and a library transform move
+// 456 B per point and cycle in FP64 with two sites (passes A / K / R 264, two
+// 3D transforms of three read-write passes each 192), and on small grids the
+// dozen launches cost more than the work.  Folded, the cycle moves 264 B in
+// three launches:
+//   plane A  reads t, U, the new residual and two history grids, writes t and
+//            one history grid (112) and the transform buffer (16);
+//   z lines  read and write the buffer (32) and read half of fk (8);
+//   plane R  reads the buffer, t, U and the two residual histories and writes
+//            the new residual (96), so plane A needs no inverse transform.
+// A plane is worked on by a cluster of CTAs: each transforms its share of the
+// rows, the half-transformed plane is exchanged through L2, and after one
+// cluster barrier each transforms its share of the columns.  (A plane of
+// complex FP64 at N = 256 is 1 MB: more than the distributed shared memory of
+// a portable cluster leaves room for at two CTAs per SM.)
+//
+// The residual goes to whichever of three slots holds no history
+// (DevState.rp): if the update of this cycle is applied, finalize renames
+// that slot, so the history is never copied and a stop leaves it untouched.
+//
+// A line of N = R1 R2 points is transformed in two register stages with one
+// shared-memory exchange (n = t + R2 j, k = s + R1 k2):
+//   A_t[s] = W_N^(t s) sum_j a[t + R2 j] W_R1^(j s),  X[s + R1 k2] = sum_t A_t[s] W_R2^(t k2)
+// and backwards, starting from the groups of equal k mod R1 (so the z kernel
+// goes forth and back with two exchanges in all).
+#pragma once
+
+#include "dft.cuh"
+#include "fused_api.cuh"
+
+namespace rism3d {
+namespace fused {
+
+template <typename T> using CxT = typename Cx<T>::t;
+
+// ---- shapes: N = R1 R2 with R2 even (z lines pair up registers of mirror
+// points), R1 >= R2 where possible; LB lines per batch, NC CTAs per plane
+template <int N> struct Shape;
+template <> struct Shape<32>  { static constexpr int R1 = 8,  R2 = 4,  LB = 16, NC = 2; };
+template <> struct Shape<48>  { static constexpr int R1 = 8,  R2 = 6,  LB = 16, NC = 3; };
+template <> struct Shape<64>  { static constexpr int R1 = 8,  R2 = 8,  LB = 32, NC = 2; };
+template <> struct Shape<96>  { static constexpr int R1 = 12, R2 = 8,  LB = 16, NC = 6; };
+template <> struct Shape<128> { static constexpr int R1 = 16, R2 = 8,  LB = 16, NC = 4; };
+template <> struct Shape<256> { static constexpr int R1 = 16, R2 = 16, LB = 16, NC = 8; };
+
+template <int N> struct Lines {
+  static constexpr int R1 = Shape<N>::R1, R2 = Shape<N>::R2, LB = Shape<N>::LB, NC = Shape<N>::NC;
+  static constexpr int TH = LB * R2;               // threads: one stage-1 item each
+  static constexpr int ST = R2 | 1;                // row-exchange stride (no bank conflicts)
+  static constexpr int LS = R1 * ST;               // shared points of one row
+  static constexpr int SH = N / NC;                // lines per CTA
+  static_assert(R1 * R2 == N && R2 % 2 == 0 && SH % LB == 0, "line split");
+  template <typename T> static constexpr size_t smem() { return sizeof(CxT<T>) * LB * (size_t)LS; }
+  // a whole-phase launch of a small grid has one block per SM at most: all
+  // registers, and all points of a thread in flight at once
+  template <typename T, int V> __host__ __device__ static constexpr int minp() {
+    return (N * NC * ((V + 1) / 2) <= 148) ? 1 : minb<T>();
+  }
+  // resident CTAs asked of the compiler: 128 registers in FP64, 80 in FP32
+  template <typename T> __host__ __device__ static constexpr int minb() {
+    return (sizeof(T) == 8 ? 512 : 768) / TH > 0 ? (sizeof(T) == 8 ? 512 : 768) / TH : 1;
+  }
+};
+
+// Pointwise loops: a thread takes vectors of VW neighbouring points (16 bytes
+// where its R1 points allow), NV of them at a time (WIDE: all) with every load before the
+// first use.  FP64: 4 points x 10 streams = 320 B in flight per thread.
+template <typename T, int R1, bool WIDE> struct Vecs {
+  static constexpr int VW = sizeof(T) == 8 ? 2 : (R1 % 4 == 0 ? 4 : 2);
+  static constexpr int TOT = R1 / VW;              // vectors per thread and row
+  static constexpr int NV = WIDE ? TOT : (sizeof(T) == 8 && TOT % 2 == 0) ? 2 : 1;
+  static constexpr int CH = TOT / NV;              // chunks
+  static_assert(R1 % VW == 0, "points per thread");
+};
+template <int B> struct VecT;
+template <> struct VecT<8> { typedef float2 t; };
+template <> struct VecT<16> { typedef float4 t; };
+// streams of the state: read or written once per kernel, first to leave L2
+template <typename T, int W> __device__ __forceinline__ void ldv(T (&o)[W], const T *p) {
+  typedef typename VecT<sizeof(T) * W>::t B;
+  union { B b; T t[W]; } u;
+  u.b = __ldcs(reinterpret_cast<const B *>(p));
+#pragma unroll
+  for (int k = 0; k < W; ++k) o[k] = u.t[k];
+}
+template <typename T, int W> __device__ __forceinline__ void stv(T *p, const T (&o)[W]) {
+  typedef typename VecT<sizeof(T) * W>::t B;
+  union { B b; T t[W]; } u;
+#pragma unroll
+  for (int k = 0; k < W; ++k) u.t[k] = o[k];
+  __stcs(reinterpret_cast<B *>(p), u.b);
+}
+
+template <typename T> __device__ __forceinline__ void pf(const T *p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;\n"
+               ::: "memory");
+}
+// Threads that share a row: the R2 consecutive threads of stage 1 also do its
+// R1 stage-2 items (s = t, t + R2, ...), so that where R2 divides a warp the
+// row exchange needs no block barrier.
+template <int R2> __device__ __forceinline__ void row_sync() {
+  if (32 % R2 == 0) __syncwarp();
+  else __syncthreads();
+}
+template <int NC> __device__ __forceinline__ void plane_sync() {
+  if (NC > 1) cluster_sync();
+  else __syncthreads();
+}
+
+template <typename T> __device__ __forceinline__ T *rp_slot(const IterArgs<T> &a, int V, int i) {
+  return i < 2 ? a.RP + (size_t)i * V * a.n : a.RPx;
+}
+
+// y-DFT of columns [c0, c0 + SH) of a plane: src[y N + x] -> dst (dst may be
+// src: a column is read whole before it is written)
+template <typename T, int N, bool INV>
+__device__ __forceinline__ void columns(const CxT<T> *src, CxT<T> *dst, int c0, CxT<T> *sm,
+                                        const CxT<T> *roots) {
+  typedef CxT<T> C;
+  using L = Lines<N>;
+  constexpr int R1 = L::R1, R2 = L::R2, LB = L::LB;
+  const int col = threadIdx.x % LB, t = threadIdx.x / LB;
+#pragma unroll 1
+  for (int cb = 0; cb < L::SH; cb += LB) {
+    const C *s0 = src + c0 + cb + col;
+    C v[R1];
+#pragma unroll
+    for (int j = 0; j < R1; ++j) v[j] = __ldcg(s0 + (size_t)(t + R2 * j) * N);
+    dft::run<R1, INV>(v);
+#pragma unroll
+    for (int s = 1; s < R1; ++s) v[s] = dft::cmulw<INV>(v[s], roots[t * s]);
+    __syncthreads();                               // the exchange's last readers are done
+#pragma unroll
+    for (int s = 0; s < R1; ++s) sm[(s * R2 + t) * LB + col] = v[s];
+    __syncthreads();
+#pragma unroll 1
+    for (int i = threadIdx.x; i < LB * R1; i += L::TH) {
+      const int c = i % LB, s = i / LB;
+      C w[R2];
+#pragma unroll
+      for (int k = 0; k < R2; ++k) w[k] = sm[(s * R2 + k) * LB + c];
+      dft::run<R2, INV>(w);
+      C *d0 = dst + c0 + cb + c;
+#pragma unroll
+      for (int k = 0; k < R2; ++k) __stcg(d0 + (size_t)(s + R1 * k) * N, w[k]);
+    }
+  }
+}
+
+// ---------------------------------------------------------------- plane A
+template <typename T, int N, int V, bool REF, bool WIDE>
+__device__ __forceinline__ void planes_a(const IterArgs<T> &a, const DevState *st, CxT<T> *sm,
+                                         const CxT<T> *tw, const CxT<T> *roots, bool hnc) {
+  typedef CxT<T> C;
+  using L = Lines<N>;
+  constexpr int R1 = L::R1, R2 = L::R2, LB = L::LB, ST = L::ST, LS = L::LS;
+  using W = Vecs<T, R1, WIDE>;
+  constexpr int P = (V + 1) / 2, VW = W::VW, NV = W::NV;
+  const int mode = st->mode, slot = st->upd_slot;
+  const T s1 = (T)st->s1, s2 = (T)st->s2, m = (T)st->m;
+  const T *Rn = rp_slot(a, V, st->rp[slot]);       // this cycle's residual
+  const long long n = a.n;
+  const int rank = blockIdx.x % L::NC, ncl = gridDim.x / L::NC;
+  const int row_l = threadIdx.x / R2, t = threadIdx.x % R2;
+  C *line = sm + row_l * LS;
+  for (int plane = blockIdx.x / L::NC; plane < N * P; plane += ncl) {
+    const int p = plane / N, z = plane % N;
+    const bool two = V % 2 == 0 || 2 * p + 1 < V;
+    C *pb = a.buf + (size_t)plane * N * N;
+    __syncthreads();                               // the columns' exchange is free
+#pragma unroll 1
+    for (int rb = 0; rb < L::SH; rb += LB) {
+      const int y = rank * L::SH + rb + row_l;
+      const size_t base = (size_t)(2 * p) * n + ((size_t)z * N + y) * N;
+      T *pt = a.t + base, *py = a.Y + (size_t)slot * V * n + base;
+      const T *pu = a.U + base, *pr = Rn + base, *p0 = a.Y + base, *p1 = a.Y + (size_t)V * n + base;
+      const C tyz = cmul(tw[N + y], tw[2 * N + z]);
+      const int dyz = (y + z) & 1;
+      row_sync<R2>();                              // the exchange's last readers are done
+#pragma unroll 1
+      for (int c = 0; c < W::CH; ++c) {
+        T tv[2][NV][VW], uv[2][NV][VW];
+        int x0[NV];
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+          x0[q] = VW * (t + R2 * (q + NV * c));
+          ldv(tv[0][q], pt + x0[q]);
+          ldv(uv[0][q], pu + x0[q]);
+          if (two) {
+            ldv(tv[1][q], pt + n + x0[q]);
+            ldv(uv[1][q], pu + n + x0[q]);
+          }
+        }
+        if (mode != 0) {
+          T rv[2][NV][VW], y0[2][NV][VW], y1[2][NV][VW];
+#pragma unroll
+          for (int q = 0; q < NV; ++q)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+              if (b && !two) break;
+              ldv(rv[b][q], pr + b * n + x0[q]);
+              ldv(y0[b][q], p0 + b * n + x0[q]);
+              ldv(y1[b][q], p1 + b * n + x0[q]);
+            }
+#pragma unroll
+          for (int q = 0; q < NV; ++q)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+              if (b && !two) break;
+              T yw[VW];
+#pragma unroll
+              for (int k = 0; k < VW; ++k) {
+                // newdt (AN2), anderson_cuda.cu:11-23, or newdt0 (Picard)
+                const T tt = tv[b][q][k], r = rv[b][q][k], yy = tt + m * r;
+                yw[k] = yy;
+                tv[b][q][k] = mode == 2 ? yy + s1 * (y0[b][q][k] - yy) + s2 * (y1[b][q][k] - yy)
+                                        : tt + r;
+              }
+              stv(py + b * n + x0[q], yw);
+              stv(pt + b * n + x0[q], tv[b][q]);
+            }
+        }
+        // closure + c_SR (calculate_cuda.cu:1-29) and the forward pre-twiddle
+        // (timekf, fft3d.cu:41-49): dir * dkf * (c_a + i c_b)
+#pragma unroll
+        for (int q = 0; q < NV; ++q)
+#pragma unroll
+          for (int k = 0; k < VW; ++k) {
+            const int x = x0[q] + k;
+            C cc;
+            cc.x = cfun_rt<REF>(tv[0][q][k], uv[0][q][k], hnc);
+            cc.y = two ? cfun_rt<REF>(tv[1][q][k], uv[1][q][k], hnc) : T(0);
+            const C kf = cmul(tw[x], tyz);
+            const T dir = ((x & 1) ^ dyz) ? T(-1) : T(1);
+            C w;
+            w.x = kf.x * dir;
+            w.y = kf.y * dir;
+            line[(x / R2) * ST + x % R2] = cmul(cc, w);
+          }
+      }
+      row_sync<R2>();
+      // x-DFT; a thread's stage-1 inputs and outputs are its own slots
+      {
+        C v[R1];
+#pragma unroll
+        for (int j = 0; j < R1; ++j) v[j] = line[j * ST + t];
+        dft::run<R1, false>(v);
+#pragma unroll
+        for (int s = 1; s < R1; ++s) v[s] = cmul(v[s], roots[t * s]);
+#pragma unroll
+        for (int s = 0; s < R1; ++s) line[s * ST + t] = v[s];
+      }
+      row_sync<R2>();
+#pragma unroll 1
+      for (int s = t; s < R1; s += R2) {
+        C w[R2];
+#pragma unroll
+        for (int k = 0; k < R2; ++k) w[k] = line[s * ST + k];
+        dft::run<R2, false>(w);
+        C *d = pb + (size_t)y * N + s;
+#pragma unroll
+        for (int k = 0; k < R2; ++k) __stcg(d + R1 * k, w[k]);
+      }
+    }
+    plane_sync<L::NC>();                           // every row of the plane is in L2
+    columns<T, N, false>(pb, pb, rank * L::SH, sm, roots);
+  }
+}
+
+template <typename T, int N, int V, bool REF>
+__global__ void __launch_bounds__(Lines<N>::TH, (Lines<N>::template minb<T>()))
+    k_plane_a(IterArgs<T> a0, bool hnc) {
+  extern __shared__ __align__(16) unsigned char fused_sm[];
+  const IterArgs<T> a = solute_view<T, V>(a0);
+  if (a.st->done) return;
+  planes_a<T, N, V, REF, false>(a, a.st, reinterpret_cast<CxT<T> *>(fused_sm), a.tw, a.roots, hnc);
+}
+
+// ---------------------------------------------------------------- plane R
+// Inverse row DFT of LB rows of the half-transformed plane: row (relative to
+// src) threadIdx.x / R2, the result in line[(x / R2) ST + x % R2], not yet
+// twiddled.
+template <typename T, int N>
+__device__ __forceinline__ void rows_inverse(const CxT<T> *src, CxT<T> *line, int t,
+                                             const CxT<T> *roots) {
+  typedef CxT<T> C;
+  using L = Lines<N>;
+  constexpr int R1 = L::R1, R2 = L::R2, ST = L::ST, NI = (R1 + R2 - 1) / R2;
+  {
+    C v[R1];
+#pragma unroll
+    for (int j = 0; j < R1; ++j) v[j] = __ldcg(src + t + R2 * j);
+    dft::run<R1, true>(v);
+#pragma unroll
+    for (int s = 1; s < R1; ++s) v[s] = dft::cmulw<true>(v[s], roots[t * s]);
+    row_sync<R2>();                                // the exchange's last readers are done
+#pragma unroll
+    for (int s = 0; s < R1; ++s) line[s * ST + t] = v[s];
+  }
+  row_sync<R2>();
+  C w[NI][R2];
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    const int s = t + R2 * i;
+    if (s < R1) {
+#pragma unroll
+      for (int k = 0; k < R2; ++k) w[i][k] = line[s * ST + k];
+      dft::run<R2, true>(w[i]);
+    }
+  }
+  row_sync<R2>();
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    const int s = t + R2 * i;
+    if (s < R1) {
+#pragma unroll
+      for (int k = 0; k < R2; ++k) {
+        const int x = s + R1 * k;
+        line[(x / R2) * ST + x % R2] = w[i][k];
+      }
+    }
+  }
+  row_sync<R2>();
+}
+
+template <typename T, int N, int V, bool REF, bool WIDE>
+__device__ __forceinline__ void planes_r(const IterArgs<T> &a, const DevState *st, CxT<T> *sm,
+                                         const CxT<T> *tw, const CxT<T> *roots, bool hnc) {
+  typedef CxT<T> C;
+  using L = Lines<N>;
+  constexpr int R1 = L::R1, R2 = L::R2, LB = L::LB, ST = L::ST, LS = L::LS, TH = L::TH;
+  using W = Vecs<T, R1, WIDE>;
+  constexpr int P = (V + 1) / 2, VW = W::VW, NV = W::NV;
+  __shared__ double red[(TH + 31) / 32][6];
+  const bool gram = st->count <= 0;
+  const long long n = a.n;
+  const T *RP0 = rp_slot(a, V, st->rp[0]), *RP1 = rp_slot(a, V, st->rp[1]);
+  T *Rn = rp_slot(a, V, st->rp[2]);
+  const int rank = blockIdx.x % L::NC, cl = blockIdx.x / L::NC, ncl = gridDim.x / L::NC;
+  const int row_l = threadIdx.x / R2, t = threadIdx.x % R2;
+  C *line = sm + row_l * LS;
+  C *scr = a.scr + (size_t)cl * N * N;
+  const T invvol = (T)a.invvol;
+  double acc[6] = {0, 0, 0, 0, 0, 0};
+  for (int plane = cl; plane < N * P; plane += ncl) {
+    const int p = plane / N, z = plane % N;
+    const bool two = V % 2 == 0 || 2 * p + 1 < V;
+    columns<T, N, true>(a.buf + (size_t)plane * N * N, scr, rank * L::SH, sm, roots);
+    __syncthreads();                               // the columns' exchange is free
+    plane_sync<L::NC>();                           // every column of the plane is in L2
+#pragma unroll 1
+    for (int rb = 0; rb < L::SH; rb += LB) {
+      const int y = rank * L::SH + rb + row_l;
+      rows_inverse<T, N>(scr + (size_t)y * N, line, t, roots);
+      const size_t base = (size_t)(2 * p) * n + ((size_t)z * N + y) * N;
+      const T *pt = a.t + base, *pu = a.U + base, *p0 = RP0 + base, *p1 = RP1 + base,
+              *pq = REF ? a.R0 + base : nullptr;
+      T *pr = Rn + base;
+      const C tyz = cmul(tw[N + y], tw[2 * N + z]);
+      const int dyz = (y + z) & 1;
+#pragma unroll 1
+      for (int c = 0; c < W::CH; ++c) {
+        T tv[2][NV][VW], uv[2][NV][VW], r0[2][NV][VW], r1[2][NV][VW], qv[2][NV][VW];
+        int x0[NV];
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+          x0[q] = VW * (t + R2 * (q + NV * c));
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            if (b && !two) break;
+            ldv(tv[b][q], pt + b * n + x0[q]);
+            ldv(uv[b][q], pu + b * n + x0[q]);
+            ldv(r0[b][q], p0 + b * n + x0[q]);
+            ldv(r1[b][q], p1 + b * n + x0[q]);
+            if (REF) ldv(qv[b][q], pq + b * n + x0[q]);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+          T rw[2][VW];
+#pragma unroll
+          for (int k = 0; k < VW; ++k) {
+            const int x = x0[q] + k;
+            // inverse post-twiddle (timekb, fft3d.cu:52-60): (1/V) dir conj(dkf)
+            const C kf = cmul(tw[x], tyz);
+            const T sc = invvol * (((x & 1) ^ dyz) ? T(-1) : T(1));
+            C w;
+            w.x = kf.x * sc;
+            w.y = -kf.y * sc;
+            const C h = cmul(line[(x / R2) * ST + x % R2], w);
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+              if (b && !two) break;
+              const T R = residual_rt<REF>(b ? h.y : h.x, tv[b][q][k], uv[b][q][k],
+                                           REF ? qv[b][q][k] : T(0), hnc);
+              rw[b][k] = R;
+              const double r = (double)R;
+              acc[0] += r * r;                     // cal_rms.cu:18
+              if (gram) {                          // theta30, anderson_cuda.cu:33-39
+                const double wt = a.sp->irho[2 * p + b];
+                const double d0 = r - (double)r0[b][q][k], d1 = r - (double)r1[b][q][k];
+                acc[1] += wt * r * d0;
+                acc[2] += wt * r * d1;
+                acc[3] += wt * d0 * d0;
+                acc[4] += wt * d0 * d1;
+                acc[5] += wt * d1 * d1;
+              }
+            }
+          }
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            if (b && !two) break;
+            stv(pr + b * n + x0[q], rw[b]);
+          }
+        }
+      }
+    }
+    if (plane + ncl < N * P) plane_sync<L::NC>();  // the scratch plane is free again
+  }
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    double v = acc[k];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    acc[k] = v;
+  }
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0)
+    for (int k = 0; k < 6; ++k) red[wid][k] = acc[k];
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    double s = 0.0;
+    for (int w = 0; w < TH / 32; ++w) s += red[w][threadIdx.x];
+    a.part[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = s;
+  }
+}
+
+template <typename T, int N, int V, bool REF>
+__global__ void __launch_bounds__(Lines<N>::TH, (Lines<N>::template minb<T>()))
+    k_plane_r(IterArgs<T> a0, bool hnc) {
+  extern __shared__ __align__(16) unsigned char fused_sm[];
+  __shared__ bool last;
+  const IterArgs<T> a = solute_view<T, V>(a0);
+  DevState *st = a.st;
+  if (st->done) {                                  // this solute has stopped
+    if (blockIdx.x == 0 && threadIdx.x == 0) loop_test_all(a0);
+    return;
+  }
+  planes_r<T, N, V, REF, false>(a, st, reinterpret_cast<CxT<T> *>(fused_sm), a.tw, a.roots, hnc);
+  // the last block to finish reduces all block sums and steers the loop
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(a.count, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  finalize_block(st, a.part, gridDim.x, (double)a.n * V, a.hist, a.hist_cap);
+  if (threadIdx.x == 0) {
+    *a.count = 0u;
+    if (st->done) st->after_done = 1;              // nothing is left to do in the loop
+    loop_test_all(a0);
+  }
+}
+
+// Once after the loop: snapshot of h (Re of the last OZ) and g (closure of
+// the t used in that cycle), and when maxstep ended the loop the pending
+// update (iterate.cu:61 runs before the step bound is tested).
+template <typename T, int N, int V, bool REF>
+__global__ void __launch_bounds__(Lines<N>::TH) k_plane_final(IterArgs<T> a0, bool hnc) {
+  typedef CxT<T> C;
+  using L = Lines<N>;
+  constexpr int R2 = L::R2, LB = L::LB, ST = L::ST, LS = L::LS;
+  constexpr int P = (V + 1) / 2;
+  extern __shared__ __align__(16) unsigned char fused_sm[];
+  C *sm = reinterpret_cast<C *>(fused_sm);
+  const IterArgs<T> a = solute_view<T, V>(a0);
+  const DevState *st = a.st;
+  const int done = st->done, mode = st->mode, slot = st->upd_slot;
+  const bool snap = !REF && a.hout, update = done == 3 && mode != 0;
+  if (!snap && !update) return;
+  const T s1 = (T)st->s1, s2 = (T)st->s2, m = (T)st->m;
+  const T *Rn = rp_slot(a, V, st->rp[slot]);       // renamed into the history already
+  const long long n = a.n;
+  const int rank = blockIdx.x % L::NC, cl = blockIdx.x / L::NC, ncl = gridDim.x / L::NC;
+  const int row_l = threadIdx.x / R2, t = threadIdx.x % R2;
+  C *line = sm + row_l * LS;
+  C *scr = a.scr + (size_t)cl * N * N;
+  for (int plane = cl; plane < N * P; plane += ncl) {
+    const int p = plane / N, z = plane % N;
+    columns<T, N, true>(a.buf + (size_t)plane * N * N, scr, rank * L::SH, sm, a.roots);
+    __syncthreads();
+    plane_sync<L::NC>();
+#pragma unroll 1
+    for (int rb = 0; rb < L::SH; rb += LB) {
+      const int y = rank * L::SH + rb + row_l;
+      rows_inverse<T, N>(scr + (size_t)y * N, line, t, a.roots);
+      const C tyz = cmul(a.tw[N + y], a.tw[2 * N + z]);
+#pragma unroll 1
+      for (int x = t; x < N; x += R2) {
+        const C kf = cmul(a.tw[x], tyz);
+        const T sc = (T)a.invvol * (((x + y + z) & 1) ? T(-1) : T(1));
+        C w;
+        w.x = kf.x * sc;
+        w.y = -kf.y * sc;
+        const C h = cmul(line[(x / R2) * ST + x % R2], w);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          if (2 * p + q >= V) break;
+          const size_t iv = (size_t)(2 * p + q) * n + ((size_t)z * N + y) * N + x;
+          const T tv = a.t[iv];
+          if (snap) {
+            a.hout[iv] = (double)(q ? h.y : h.x);
+            a.gout[iv] = (double)closure_rt(tv - a.U[iv], hnc);
+          }
+          if (update) {
+            const T R = Rn[iv], yv = tv + m * R;
+            T tn = tv + R;
+            if (mode == 2) tn = yv + s1 * (a.Y[iv] - yv) + s2 * (a.Y[(size_t)V * n + iv] - yv);
+            a.Y[(size_t)slot * V * n + iv] = yv;
+            a.t[iv] = tn;
+          }
+        }
+      }
+    }
+    if (plane + ncl < N * P) plane_sync<L::NC>();
+  }
+}
+
+// ---------------------------------------------------------------- z lines
+// A block owns CW neighbouring kx columns at one ky < N/2 and their mirrors
+// (kx' = N-1-kx, ky' = N-1-ky), so every k and -k meet in it.  After the
+// forward DFT the owner's points kz = s + R1 k of one thread mirror the
+// points of the neighbouring lane's group R1-1-s, register R2-1-k: each lane
+// takes half of the pairs with one shuffle each way.
+template <typename T, int N, int V>
+struct ZShape {
+  // as many columns as a plane batch has lines: one block size for all kernels
+  static constexpr int COLS = Lines<N>::LB, CW = COLS / 2, TH = Lines<N>::TH;
+  static constexpr int P = (V + 1) / 2;
+  static constexpr int TILES = (N / CW) * (N / 2);
+  static constexpr int MINB = (sizeof(T) == 8 ? 512 : 1024) / TH > 0 ? (sizeof(T) == 8 ? 512 : 1024) / TH : 1;
+  static constexpr size_t smem() { return sizeof(CxT<T>) * (size_t)P * COLS * N; }
+};
+
+template <typename C>
+__device__ __forceinline__ C shfl_pair(unsigned mask, C v) {
+  v.x = __shfl_xor_sync(mask, v.x, 1);
+  v.y = __shfl_xor_sync(mask, v.y, 1);
+  return v;
+}
+
+template <typename T, int N, int V, bool WIDE>
+__device__ __forceinline__ void zline_tile(const IterArgs<T> &a, CxT<T> *sm, const CxT<T> *roots,
+                                           int tile) {
+  typedef CxT<T> C;
+  using Z = ZShape<T, N, V>;
+  constexpr int R1 = Shape<N>::R1, R2 = Shape<N>::R2, CW = Z::CW, COLS = Z::COLS, P = Z::P;
+  static_assert(N % CW == 0 && Z::TH % 32 == 0, "z tiles");
+  const long long n = a.n;
+  const int ky = tile / (N / CW), x0 = (tile % (N / CW)) * CW;
+  // fk and chi of an item's pairs: loaded ahead of the exchange where they fit
+  // in registers, else asked into L2 now
+  constexpr int H = R2 / 2;
+  constexpr bool AHEAD = WIDE && H * (V * V + 2) * sizeof(T) <= 24 * 8;
+  double2 fkv[H];
+  T X[H][V * V];
+  auto pair_kz = [&](int i, int k) {
+    const int side = i & 1, s = (i >> 1) / CW;
+    return side ? N - 1 - (R1 - 1 - s + R1 * k) : s + R1 * k;
+  };
+  auto load_pair = [&](int i, int k, double2 &fk, T (&x)[V * V]) {
+    // beta fk is stored for kz < N/2, the conjugate of the mirror's beyond
+    const int kx = x0 + (i >> 1) % CW, kz = pair_kz(i, k);
+    fk = make_double2(0.0, 0.0);
+    if (!a.nofk) {
+      const bool lo = kz < N / 2;
+      const long long j = kx + (long long)N * (ky + (long long)N * kz);
+      fk = __ldg(a.fkh + (lo ? j : n - 1 - j));
+      if (!lo) fk.y = -fk.y;
+    }
+    chi_cubic<T, V>(a, kx, ky, kz, x);
+  };
+  if constexpr (!AHEAD) {
+    if (!a.nofk)                                   // rows of CW points and their mirrors
+      for (int i = threadIdx.x; i < N; i += Z::TH) {
+        const int kz = i % (N / 2);
+        pf(a.fkh + (i < N / 2 ? x0 + (long long)N * (ky + (long long)N * kz)
+                              : N - x0 - CW + (long long)N * (N - 1 - ky + (long long)N * kz)));
+      }
+  }
+  {
+    const int col = threadIdx.x % COLS, t = threadIdx.x / COLS;
+    const C *g = a.buf + (col < CW ? (size_t)ky * N + x0 + col
+                                   : (size_t)(N - 1 - ky) * N + (N - x0 - 2 * CW) + col);
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      C v[R1];
+#pragma unroll
+      for (int j = 0; j < R1; ++j) v[j] = __ldcg(g + (size_t)p * n + (size_t)(t + R2 * j) * N * N);
+      dft::run<R1, false>(v);
+#pragma unroll
+      for (int s = 1; s < R1; ++s) v[s] = cmul(v[s], roots[t * s]);
+#pragma unroll
+      for (int s = 0; s < R1; ++s) sm[(p * N + s * R2 + t) * COLS + col] = v[s];
+    }
+  }
+  if constexpr (AHEAD)
+    if (threadIdx.x < COLS * R1)
+#pragma unroll
+      for (int k = 0; k < H; ++k) load_pair(threadIdx.x, k, fkv[k], X[k]);
+  __syncthreads();
+#pragma unroll 1
+  for (int i0 = 0; i0 < COLS * R1; i0 += Z::TH) {
+    const int i = i0 + threadIdx.x;
+    const bool act = i < COLS * R1;
+    const unsigned mask = __ballot_sync(0xffffffffu, act);
+    if (!act) continue;
+    const int side = i & 1, o = (i >> 1) % CW, s = (i >> 1) / CW;
+    const int grp = side ? R1 - 1 - s : s, col = side ? COLS - 1 - o : o;
+    C v[P][R2];
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+#pragma unroll
+      for (int k = 0; k < R2; ++k) v[p][k] = sm[(p * N + grp * R2 + k) * COLS + col];
+      dft::run<R2, false>(v[p]);
+    }
+    const int kx = x0 + o;
+#pragma unroll
+    for (int k = 0; k < H; ++k) {
+      // the owner point of this lane's pair k
+      const int kz = pair_kz(i, k);
+      if constexpr (!AHEAD) load_pair(i, k, fkv[0], X[0]);
+      const double2 fk = fkv[AHEAD ? k : 0];
+      C y[P], ym[P], out[P], outm[P];
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        const C q = shfl_pair(mask, v[p][R2 - 1 - k]);
+        y[p] = side ? q : v[p][k];
+        ym[p] = side ? v[p][k] : q;
+      }
+      kspace_product_x<T, V>(a, fk, X[AHEAD ? k : 0], kx, ky, kz, y, ym, out, outm);
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        v[p][k] = side ? outm[p] : out[p];
+        v[p][R2 - 1 - k] = shfl_pair(mask, side ? out[p] : outm[p]);
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      dft::run<R2, true>(v[p]);
+#pragma unroll
+      for (int k = 0; k < R2; ++k)
+        sm[(p * N + grp * R2 + k) * COLS + col] =
+            k ? dft::cmulw<true>(v[p][k], roots[k * grp]) : v[p][k];
+    }
+    if constexpr (AHEAD && R1 > R2)
+      if (i + Z::TH < COLS * R1)
+#pragma unroll
+        for (int k = 0; k < H; ++k) load_pair(i + Z::TH, k, fkv[k], X[k]);
+  }
+  __syncthreads();
+  {
+    const int col = threadIdx.x % COLS, t = threadIdx.x / COLS;
+    C *g = a.buf + (col < CW ? (size_t)ky * N + x0 + col
+                             : (size_t)(N - 1 - ky) * N + (N - x0 - 2 * CW) + col);
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      C v[R1];
+#pragma unroll
+      for (int s = 0; s < R1; ++s) v[s] = sm[(p * N + s * R2 + t) * COLS + col];
+      dft::run<R1, true>(v);
+#pragma unroll
+      for (int j = 0; j < R1; ++j) __stcg(g + (size_t)p * n + (size_t)(t + R2 * j) * N * N, v[j]);
+    }
+  }
+}
+
+template <typename T, int N, int V>
+__global__ void __launch_bounds__(ZShape<T, N, V>::TH, (ZShape<T, N, V>::MINB)) k_zline(IterArgs<T> a0) {
+  extern __shared__ __align__(16) unsigned char fused_sm[];
+  const IterArgs<T> a = solute_view<T, V>(a0);
+  if (a.st->done) return;
+  zline_tile<T, N, V, false>(a, reinterpret_cast<CxT<T> *>(fused_sm), a.roots, blockIdx.x);
+}
+
+// ---------------------------------------------------------------- one launch
+// A whole phase in one launch, for grids whose three kernels take about as
+// long as their launches: the same three stages with a barrier over the
+// solute's blocks between them (all resident: cooperative launch).  Every
+// block keeps its own copy of the loop state and reduces all block sums
+// itself, in the same order, so the stopping test and the 2 x 2 solve need no
+// further exchange.  A block always works on the same planes, so the state
+// arrays are only ever touched by the SM that wrote them; the transform
+// buffer, the exchange planes and the sums go through L2.
+//
+// Arrival count of one solute's blocks, with a bound on the wait: false when
+// the other blocks never came (the caller reports it and returns).
+constexpr unsigned kBarrierPolls = 1u << 24;
+__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned target) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    unsigned v, polls = 0;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+    } while ((int)(v - target) < 0 && ++polls < kBarrierPolls);   // the count may wrap
+    ok = (int)(v - target) >= 0;
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+// byte offset of the tables: after the largest of the stages' exchanges
+template <typename T, int N, int V> __host__ __device__ constexpr size_t tables_at() {
+  const size_t row = sizeof(CxT<T>) * Lines<N>::LB * Lines<N>::LS,
+               z = sizeof(CxT<T>) * (size_t)((V + 1) / 2) * Lines<N>::LB * N;
+  return row > z ? row : z;
+}
+
+template <typename T, int N, int V, bool REF>
+__global__ void __launch_bounds__(Lines<N>::TH, (Lines<N>::template minp<T, V>()))
+    k_phase(IterArgs<T> a0, bool hnc) {
+  typedef CxT<T> C;
+  extern __shared__ __align__(16) unsigned char fused_sm[];
+  constexpr bool WIDE = Lines<N>::template minp<T, V>() == 1 && Lines<N>::template minb<T>() > 1;
+  __shared__ DevState ss;
+  C *sm = reinterpret_cast<C *>(fused_sm);
+  const IterArgs<T> a = solute_view<T, V>(a0);
+  // the phase and root tables, read at every stage, stay in shared memory
+  // (every barrier's acquire empties L1)
+  C *tw = reinterpret_cast<C *>(fused_sm + tables_at<T, N, V>()), *roots = tw + 3 * N;
+  for (int i = threadIdx.x; i < 3 * N; i += blockDim.x) tw[i] = a.tw[i];
+  for (int i = threadIdx.x; i < N; i += blockDim.x) roots[i] = a.roots[i];
+  if (threadIdx.x == 0) ss = *a.st;
+  __syncthreads();
+  unsigned *bar = a.bar + blockIdx.y;
+  const unsigned nblk = gridDim.x;
+  unsigned target = 0;
+  bool ok = true;
+  while (!ss.done) {
+    planes_a<T, N, V, REF, WIDE>(a, &ss, sm, tw, roots, hnc);
+    if (!(ok = grid_barrier(bar, target += nblk))) break;
+#pragma unroll 1
+    for (int tile = blockIdx.x; tile < ZShape<T, N, V>::TILES; tile += nblk) {
+      zline_tile<T, N, V, WIDE>(a, sm, roots, tile);
+      __syncthreads();
+    }
+    if (!(ok = grid_barrier(bar, target += nblk))) break;
+    planes_r<T, N, V, REF, WIDE>(a, &ss, sm, tw, roots, hnc);
+    if (!(ok = grid_barrier(bar, target += nblk))) break;
+    finalize_block(&ss, a.part, (int)nblk, (double)a.n * V, blockIdx.x == 0 ? a.hist : nullptr,
+                   a.hist_cap);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    if (!ok) a.st->fault = 1;
+    if (blockIdx.x == 0) {
+      if (!ok) ss.fault = 1;
+      if (!ok) ss.done = 2;
+      ss.after_done = 1;
+      *a.st = ss;
+    }
+  }
+}
+
+// ---------------------------------------------------------------- launches
+// Clusters of a plane kernel: one per plane, at most what is resident at once
+// (a cluster then walks its planes with one scratch plane).
+template <typename K>
+int plane_clusters(K kernel, int nc, int threads, size_t smem, int planes) {
+  int num = 0;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(nc);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim = {(unsigned)nc, 1, 1};
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&num, kernel, &cfg) != cudaSuccess || num < 1) {
+    cudaGetLastError();
+    return 0;
+  }
+  return num < planes ? num : planes;
+}
+
+template <typename K, typename... A>
+cudaError_t launch_plane(K kernel, int nclusters, int nc, int nb, int threads, size_t smem,
+                         cudaStream_t st, bool cooperative, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(nclusters * nc, nb);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2] = {};
+  int na = 0;
+  if (nc > 1) {
+    at[na].id = cudaLaunchAttributeClusterDimension;
+    at[na++].val.clusterDim = {(unsigned)nc, 1, 1};
+  }
+  if (cooperative) {
+    at[na].id = cudaLaunchAttributeCooperative;
+    at[na++].val.cooperative = 1;
+  }
+  cfg.attrs = at;
+  cfg.numAttrs = na;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// The kernels of one (arithmetic, edge, sites) and their launch shapes
+template <typename T, int N, int V>
+struct Kernels {
+  using L = Lines<N>;
+  using Z = ZShape<T, N, V>;
+  static constexpr int P = (V + 1) / 2;
+  // A phase as one launch, by what a step took on a B200 (us, loop of three
+  // launches / one launch; V = 2): FP64 N = 32 25.7 / 15.8, 64 32.9 / 22.4,
+  // 96 89.8 / 80.3, 128 145 / 130, 256 1022 / 1082; V = 4: 64 47.7 / 38.5,
+  // 96 159 / 171, 128 325 / 352 (the one kernel's registers spill).  FP32 one
+  // launch is never slower: 64 29.5 / 17.7, 128 101 / 84, 256 592 / 575.
+  static constexpr bool ONE = sizeof(T) == 4 || N <= 64 || (N <= 128 && V <= 2);
+  template <typename K> static cudaError_t allow(K k, size_t b) {
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
+  }
+  static constexpr size_t phase_smem() {
+    return tables_at<T, N, V>() + 4 * N * sizeof(CxT<T>);
+  }
+  // attributes and cluster counts; false when the device cannot run them
+  static bool setup(FusedPlan &f, int nb) {
+    const size_t s = L::template smem<T>();
+    cudaError_t e = allow(k_plane_a<T, N, V, false>, s);
+    if (e == cudaSuccess) e = allow(k_plane_r<T, N, V, false>, s);
+    if (e == cudaSuccess) e = allow(k_plane_final<T, N, V, false>, s);
+    if constexpr (ONE)
+      if (e == cudaSuccess) e = allow(k_phase<T, N, V, false>, phase_smem());
+    if (e == cudaSuccess) e = allow(k_zline<T, N, V>, Z::smem());
+    if constexpr (sizeof(T) == 4) {
+      if (e == cudaSuccess) e = allow(k_plane_a<T, N, V, true>, s);
+      if (e == cudaSuccess) e = allow(k_plane_r<T, N, V, true>, s);
+      if (e == cudaSuccess) e = allow(k_plane_final<T, N, V, true>, s);
+      if constexpr (ONE)
+        if (e == cudaSuccess) e = allow(k_phase<T, N, V, true>, phase_smem());
+    }
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    f.ca[0] = plane_clusters(k_plane_a<T, N, V, false>, L::NC, L::TH, s, N * P);
+    f.cr[0] = plane_clusters(k_plane_r<T, N, V, false>, L::NC, L::TH, s, N * P);
+    if constexpr (sizeof(T) == 4) {
+      f.ca[1] = plane_clusters(k_plane_a<T, N, V, true>, L::NC, L::TH, s, N * P);
+      f.cr[1] = plane_clusters(k_plane_r<T, N, V, true>, L::NC, L::TH, s, N * P);
+    } else {
+      f.ca[1] = f.ca[0];
+      f.cr[1] = f.cr[0];
+    }
+    f.nc = L::NC;
+    // clusters of one phase launch: resident ones shared by the nb solutes
+    if constexpr (ONE) {
+      f.cp[0] = plane_clusters(k_phase<T, N, V, false>, L::NC, L::TH, phase_smem(), 1 << 30) / nb;
+      f.cp[1] = f.cp[0];
+      if constexpr (sizeof(T) == 4)
+        f.cp[1] = plane_clusters(k_phase<T, N, V, true>, L::NC, L::TH, phase_smem(), 1 << 30) / nb;
+      for (int r = 0; r < 2; ++r) f.cp[r] = f.cp[r] < N * P ? f.cp[r] : N * P;
+    }
+    return f.ca[0] > 0 && f.cr[0] > 0 && f.ca[1] > 0 && f.cr[1] > 0;
+  }
+  // which: 0 plane A, 1 z lines, 2 plane R, 3 the pass after the loop, 4 a
+  // whole phase
+  static cudaError_t launch(const FusedPlan &f, int which, bool ref, int hnc, int nb,
+                            const IterArgs<T> &a, cudaStream_t st) {
+    if (which == 1) {
+      k_zline<T, N, V><<<dim3(Z::TILES, nb), Z::TH, Z::smem(), st>>>(a);
+      return cudaGetLastError();
+    }
+    if constexpr (sizeof(T) == 4) {
+      if (ref) return launch_planes<true>(f, which, hnc != 0, nb, a, st);
+    }
+    return launch_planes<false>(f, which, hnc != 0, nb, a, st);
+  }
+  template <bool REF>
+  static cudaError_t launch_planes(const FusedPlan &f, int which, bool hnc, int nb,
+                                   const IterArgs<T> &a, cudaStream_t st) {
+    const size_t s = L::template smem<T>();
+    if constexpr (ONE)
+      if (which == 4)
+        return launch_plane(k_phase<T, N, V, REF>, f.cp[REF], L::NC, nb, L::TH, phase_smem(),
+                            st, true, a, hnc);
+    const int ncl = which == 0 ? f.ca[REF] : f.cr[REF];
+    return launch_plane(which == 0   ? k_plane_a<T, N, V, REF>
+                        : which == 2 ? k_plane_r<T, N, V, REF>
+                                     : k_plane_final<T, N, V, REF>,
+                        ncl, L::NC, nb, L::TH, s, st, false, a, hnc);
+  }
+};
+
+template <typename T, int N>
+Vtable<T> table_v(int V) {
+  switch (V) {
+    case 1: return {Kernels<T, N, 1>::setup, Kernels<T, N, 1>::launch};
+    case 2: return {Kernels<T, N, 2>::setup, Kernels<T, N, 2>::launch};
+    case 3: return {Kernels<T, N, 3>::setup, Kernels<T, N, 3>::launch};
+    case 4: return {Kernels<T, N, 4>::setup, Kernels<T, N, 4>::launch};
+  }
+  return {nullptr, nullptr};
+}
+
+}  // namespace fused
+}  // namespace rism3d

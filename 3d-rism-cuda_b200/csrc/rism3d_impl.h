@@ -46,6 +46,8 @@ struct DevState {
   int total32;     // of which FP32
   int fallback;    // (solute 0) the FP32 bulk diverged: stage restarts in FP64
   int restart_next;  // (solute 0) FP64 phase starts a fresh AN2 history
+  int rotate;      // 1: plane R's residual slots are renamed, not copied:
+  int rp[3];       // slots of history entries 0 and 1, and the free one
   int fault;       // a device-side wait gave up (a bulk or tile copy never
                    // arrived): the loop was stopped and the solve reports it
   double best;     // best rms of this run (stagnation watch)
@@ -110,6 +112,15 @@ struct FastDiv {
     return (__umulhi(x, m) + x) >> s;
   }
 #endif
+};
+
+// Launch shape of the three-kernel iteration in one arithmetic
+struct FusedPlan {
+  bool on = false;
+  int nc = 1;                 // CTAs per plane cluster
+  int ca[2] = {0, 0};         // clusters of plane A: plain, refinement form
+  int cr[2] = {0, 0};         // clusters of plane R
+  int cp[2] = {0, 0};         // clusters per solute of a whole-phase launch (0: none)
 };
 
 struct Timer {
@@ -217,6 +228,14 @@ struct Context {
   // beta fk in FP32 laid out [nz/2][nx][ny]
   CUtensorMap *ky_map = nullptr;
   float2 *d_fkt = nullptr;
+  // three-kernel iteration (fused.cuh), per arithmetic: third residual slot,
+  // exchange planes, roots of unity of the cell edge
+  FusedPlan fu64, fu32;
+  double *d_RPx = nullptr;
+  float *f_RPx = nullptr;
+  void *d_scr = nullptr;
+  double2 *d_roots = nullptr;
+  float2 *f_roots = nullptr;
   cufftHandle plan1 = 0;     // one Z2Z transform of the cell (RMDFT), made on first use
   bool plans_ok = false;
   // one captured iteration per precision, reused by every solve
@@ -227,6 +246,7 @@ struct Context {
   bool no_device_loop = false;
   double *d_hist = nullptr;     // per-iteration rms (verbose single solves)
   int hist_cap = 0;
+  unsigned *d_bar = nullptr;    // arrival counts of whole-phase launches [nb]
   unsigned *d_count = nullptr;  // pass-R block counter (last block finalizes)
 
   // restart guess
@@ -274,6 +294,7 @@ int launch_potential_r(Context &c);               // potential.cu (timing hook)
 int upload_chi(Context &c);                       // solver.cu
 // decide on and set up the fused-axis FP32 passes (plan, roots, limits)
 int setup_fused_axes(Context &c);                 // solver.cu
+int setup_fused_iteration(Context &c);            // solver.cu: three-kernel iteration
 int setup_kspace_tma(Context &c);                 // solver.cu: TMA fused pass K
 int fused_fk_columns(Context &c);                 // solver.cu: fk copy for it
 int setup_pipe_r(Context &c);                     // solver.cu: pipelined pass R

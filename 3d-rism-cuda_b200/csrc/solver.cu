@@ -43,208 +43,15 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "fused_api.cuh"
+#include "passes.cuh"
 #include "rism3d_impl.h"
 #include "tma.cuh"
 #include "xfft.cuh"
 
 namespace rism3d {
 
-template <typename T> struct Cx;
-template <> struct Cx<double> { typedef double2 t; };
-template <> struct Cx<float> { typedef float2 t; };
-
 namespace {
-
-constexpr int kThreads = 256;
-
-template <typename T>
-struct IterArgs {
-  long long n;
-  int nx, ny, nz;
-  FastDiv fdx, fdy;         // division by nx and ny
-  const double *xs;         // chi table per odd-square sum (cubic cells) or null
-  const float *xs32;        // the same table in FP32 (read by the FP32 passes)
-  typename Cx<T>::t *buf;   // [P][N]
-  T *t, *U, *Y, *RP;        // t, U: [V][N]; Y, RP: [2][V][N]
-  const T *R0;              // refinement: base residual [V][N] (t = d, U = x0)
-  double *hout, *gout;      // final snapshot, [V][N] (may be null)
-  const typename Cx<T>::t *tw;  // px[nx] py[ny] pz[nz]
-  double invvol, dv;
-  const double2 *fkh;       // [N/2]
-  const double *chi;        // [ntab][V*V][4]
-  int ntab;
-  double dk;
-  double bx, by, bz;
-  DevState *st;
-  const StageParams *sp;
-  double *part;
-  int nblocks;
-  unsigned *count;          // blocks of pass R done (reset by the last one)
-  double *hist;             // per-iteration rms (single solves, verbose) or null
-  int hist_cap;
-  int nofk;                 // refinement: q cf fk cancels, fk is not read
-  const float2 *xroots;     // fused-axis passes: W_nx^m, m < nx (nx == ny)
-  const float2 *fkt;        // fused-axis pass K (nx = 256): beta fk as [nz/2][nx][ny]
-};
-
-// Batched solves: blockIdx.y selects the solute; every per-solute array is
-// laid out solute-major ([B][...]) and this view offsets the pointers, so
-// the kernel bodies below are the single-solute code unchanged.
-template <typename T, int V>
-__device__ __forceinline__ IterArgs<T> solute_view(const IterArgs<T> &a) {
-  constexpr int P = (V + 1) / 2;
-  IterArgs<T> s = a;
-  const size_t b = blockIdx.y, n = (size_t)a.n;
-  if (b == 0) return s;
-  s.buf = a.buf + b * P * n;
-  s.t = a.t + b * V * n;
-  s.U = a.U + b * V * n;
-  s.Y = a.Y + b * 2 * V * n;
-  s.RP = a.RP + b * 2 * V * n;
-  if (a.hout) { s.hout = a.hout + b * V * n; s.gout = a.gout + b * V * n; }
-  if (a.R0) s.R0 = a.R0 + b * V * n;
-  s.fkh = a.fkh + b * (n / 2);
-  s.st = a.st + b;
-  s.part = a.part + b * 6 * (size_t)a.nblocks;
-  s.count = a.count + b;
-  return s;
-}
-
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-template <typename C> __device__ __forceinline__ C mk(double x, double y);
-template <> __device__ __forceinline__ double2 mk<double2>(double x, double y) {
-  return make_double2(x, y);
-}
-template <> __device__ __forceinline__ float2 mk<float2>(double x, double y) {
-  return make_float2((float)x, (float)y);
-}
-
-// Vector access to PTS (1 or 2) consecutive points of a real or complex
-// array; point pairs start at even indices, so 2-wide accesses are aligned.
-template <typename T> struct V2;
-template <> struct V2<float> { typedef float2 t; typedef float4 c; };
-template <> struct V2<double> { typedef double2 t; typedef double4 c; };
-
-template <int PTS, typename T>
-__device__ __forceinline__ void ldr(const T *__restrict__ p, T (&o)[PTS]) {
-  if (PTS == 1) {
-    o[0] = p[0];
-  } else {
-    const typename V2<T>::t w = *reinterpret_cast<const typename V2<T>::t *>(p);
-    o[0] = w.x;
-    o[PTS - 1] = w.y;
-  }
-}
-template <int PTS, typename T>
-__device__ __forceinline__ void str(T *__restrict__ p, const T (&o)[PTS]) {
-  if (PTS == 1) {
-    p[0] = o[0];
-  } else {
-    typename V2<T>::t w;
-    w.x = o[0];
-    w.y = o[PTS - 1];
-    *reinterpret_cast<typename V2<T>::t *>(p) = w;
-  }
-}
-template <int PTS, typename C>
-__device__ __forceinline__ void ldc(const C *__restrict__ p, C (&o)[PTS]) {
-#pragma unroll
-  for (int k = 0; k < PTS; ++k) o[k] = p[k];
-}
-template <int PTS, typename C>
-__device__ __forceinline__ void stc(C *__restrict__ p, const C (&o)[PTS]) {
-#pragma unroll
-  for (int k = 0; k < PTS; ++k) p[k] = o[k];
-}
-// FP32 complex pairs move as one 16-byte access
-template <>
-__device__ __forceinline__ void ldc<2, float2>(const float2 *__restrict__ p, float2 (&o)[2]) {
-  const float4 w = *reinterpret_cast<const float4 *>(p);
-  o[0] = make_float2(w.x, w.y);
-  o[1] = make_float2(w.z, w.w);
-}
-template <>
-__device__ __forceinline__ void stc<2, float2>(float2 *__restrict__ p, const float2 (&o)[2]) {
-  *reinterpret_cast<float4 *>(p) = make_float4(o[0].x, o[0].y, o[1].x, o[1].y);
-}
-
-__device__ __forceinline__ double fexp(double x) { return exp(x); }
-__device__ __forceinline__ float fexp(float x) { return expf(x); }
-
-// calculate_cuda.cu:1-20: KH g = 1 + x (x >= 0) or e^x; HNC g = e^x.
-template <int CLOS, typename T>
-__device__ __forceinline__ T closure(T x) {
-  if (CLOS == 0) return x >= T(0) ? T(1) + x : fexp(x);
-  return fexp(x);
-}
-
-__device__ __forceinline__ double fexpm1(double x) { return expm1(x); }
-__device__ __forceinline__ float fexpm1(float x) { return expm1f(x); }
-
-// C(x0 + d) - C(x0) to the relative precision of the difference itself
-// (refinement form).  KH: C(x) - 1 = max(x, 0) + expm1(min(x, 0)), so with
-// a = min(x0 + d, 0), b = min(x0, 0)
-//   C(x0 + d) - C(x0) = [max(x0 + d, 0) - max(x0, 0)] + e^b expm1(a - b),
-// where the linear bracket is d itself when both arguments are >= 0 and
-// a - b is d itself when both are < 0: e^x0 expm1(d) on the exponential
-// branch, d on the linear one, and in the two mixed cases (|x0| <= |d|)
-// x - expm1(x0) and expm1(x) - x0.  One exp and one expm1 per call and no
-// branches, so the lanes of a warp never split over the four cases.
-template <int CLOS, typename T>
-__device__ __forceinline__ T closure_diff(T x0, T d) {
-  if (CLOS == 1) return fexp(x0) * fexpm1(d);
-  const T x = x0 + d;
-  const bool pos = x >= T(0), pos0 = x0 >= T(0);
-  const T zero = T(0);
-  const T lin = (pos && pos0) ? d : (fmax(x, zero) - fmax(x0, zero));
-  const T b = fmin(x0, zero);
-  const T da = (!pos && !pos0) ? d : (fmin(x, zero) - b);
-  return lin + fexp(b) * fexpm1(da);
-}
-
-// Residual of the cycle at the current state: plain h + 1 - C(t - U);
-// refinement R0 + h - [C(x0 + d) - C(x0)] (t = d, U = x0, h = L[dc]).
-template <int CLOS, bool REF, typename T>
-__device__ __forceinline__ T residual(T h, T t, T U, T r0) {
-  if (REF) return r0 + h - closure_diff<CLOS>(U, t);
-  return h + T(1) - closure<CLOS>(t - U);
-}
-
-// Packed FFT input: plain c_SR = C(t - U) - 1 - t; refinement dc = dg - d.
-template <int CLOS, bool REF, typename T>
-__device__ __forceinline__ T cfun(T t, T U) {
-  if (REF) return closure_diff<CLOS>(U, t) - t;
-  return closure<CLOS>(t - U) - T(1) - t;
-}
-
-// Point index -> (ix, iy, iz), +-1 checkerboard dir = (-1)^(ix+iy+iz)
-// (set_ir, fft3d.cu:86-94) and dkf = exp(-i pi sum x_d/n_d)
-// (set_kf, fft3d.cu:71-83) as a product of three per-axis phases.
-__device__ __forceinline__ void split_index(long long j, const FastDiv &fdx,
-                                            const FastDiv &fdy, int &ix, int &iy,
-                                            int &iz) {
-  const unsigned u = (unsigned)j;                 // N < 2^31
-  const unsigned r = fdx.div(u);
-  ix = (int)(u - r * fdx.d);
-  iz = (int)fdy.div(r);
-  iy = (int)(r - (unsigned)iz * fdy.d);
-}
-
-template <typename C>
-__device__ __forceinline__ void point_phase(long long j, const FastDiv &fdx,
-                                            const FastDiv &fdy, const C *tw,
-                                            int &ix, int &iy, int &iz, int &dir,
-                                            C &dkf) {
-  split_index(j, fdx, fdy, ix, iy, iz);
-  dir = ((ix + iy + iz) & 1) ? -1 : 1;
-  const int nx = (int)fdx.d, ny = (int)fdy.d;
-  dkf = cmul(cmul(tw[ix], tw[nx + iy]), tw[nx + ny + iz]);
-}
 
 // ---------------------------------------------------------------- pass A
 // One straight-line body per update mode (the mode is device state, read
@@ -425,117 +232,6 @@ __global__ void __launch_bounds__(kThreads, (PassAOccupancy<T, V, CLOS, REF>::bl
 }
 
 // ---------------------------------------------------------------- pass K
-// One mirror pair of k points: j (the owner, j < N/2, grid indices ix iy iz)
-// and jm = N-1-j with k(jm) = -k(j).  y/ym are the forward-transformed
-// packed site pairs at j and jm; out/outm receive the OZ result repacked
-// for the inverse transform.
-// fk is beta fk at the owner point (zero when a.nofk).
-template <typename T, int V>
-__device__ __forceinline__ void kspace_pair_fk(const IterArgs<T> &a, double2 fk, int ix, int iy,
-                                               int iz, const typename Cx<T>::t *y,
-                                               const typename Cx<T>::t *ym,
-                                               typename Cx<T>::t *out, typename Cx<T>::t *outm) {
-  typedef typename Cx<T>::t C;
-  constexpr int P = (V + 1) / 2;
-  const StageParams *sp = a.sp;
-  const int dir = ((ix + iy + iz) & 1) ? -1 : 1;
-  // unpack the site pairs and finish the forward transform
-  // (timeirvol * dv, fft3d.cu:32) and subtract q cf fk (mqvfk)
-  // (in the working precision T: the FP32 passes round F to FP32 anyway)
-  C F[V];
-  const T sc = (T)(a.dv * 0.5 * dir);
-  const T fx = (T)fk.x, fy = (T)fk.y;
-#pragma unroll
-  for (int p = 0; p < P; ++p) {
-    const T qa = (T)sp->qcf[2 * p];
-    F[2 * p] = mk<C>(sc * (y[p].x - ym[p].x) - qa * fx, sc * (y[p].y + ym[p].y) - qa * fy);
-    if (2 * p + 1 < V) {
-      const T qb = (T)sp->qcf[2 * p + 1];
-      F[2 * p + 1] = mk<C>(sc * (y[p].y - ym[p].y) - qb * fx, -sc * (y[p].x + ym[p].x) - qb * fy);
-    }
-  }
-  // chi_ab(|k|) (solvent_spline.cu:36-47, applied per point by oz), in T
-  T X[V * V];
-  if (a.xs) {
-    // cubic cell: |k| = (pi/L) sqrt(s), s = sum of three odd squares
-    const int ox = 2 * ix - a.nx + 1, oy = 2 * iy - a.ny + 1, oz = 2 * iz - a.nz + 1;
-    const unsigned sq = (unsigned)(ox * ox + oy * oy + oz * oz);
-    const size_t row = (size_t)((sq - 3u) >> 3) * V * V;
-    if constexpr (sizeof(T) == 4 && V * V % 4 == 0) {
-      const float4 *xr = reinterpret_cast<const float4 *>(a.xs32 + row);   // 16-byte rows
-#pragma unroll
-      for (int ab = 0; ab < V * V / 4; ++ab) {
-        const float4 q = xr[ab];
-        X[4 * ab] = q.x;
-        X[4 * ab + 1] = q.y;
-        X[4 * ab + 2] = q.z;
-        X[4 * ab + 3] = q.w;
-      }
-    } else if constexpr (sizeof(T) == 4) {
-#pragma unroll
-      for (int ab = 0; ab < V * V; ++ab) X[ab] = a.xs32[row + ab];
-    } else {
-      const double2 *xr = reinterpret_cast<const double2 *>(a.xs + row);
-#pragma unroll
-      for (int ab = 0; ab < V * V / 2; ++ab) {
-        const double2 q = xr[ab];
-        X[2 * ab] = (T)q.x;
-        X[2 * ab + 1] = (T)q.y;
-      }
-      if (V * V % 2) X[V * V - 1] = (T)a.xs[row + V * V - 1];
-    }
-  } else {
-    // general cell: natural spline on knots k_i = dk (i+1) with the
-    // bisection semantics of splint.cc:9-16 on uniform knots
-    const double kx = 2.0 * kPi * (ix - a.nx / 2.0 + 0.5) / a.bx;   // set_g
-    const double ky = 2.0 * kPi * (iy - a.ny / 2.0 + 0.5) / a.by;
-    const double kz = 2.0 * kPi * (iz - a.nz / 2.0 + 0.5) / a.bz;
-    const double kk = sqrt(kx * kx + ky * ky + kz * kz);
-    int k0 = (int)(kk / a.dk) - 1;
-    k0 = k0 < 0 ? 0 : (k0 > a.ntab - 2 ? a.ntab - 2 : k0);
-    while (k0 < a.ntab - 2 && a.dk * (k0 + 2) <= kk) ++k0;
-    while (k0 > 0 && a.dk * (k0 + 1) > kk) --k0;
-    const double tt = kk - a.dk * (k0 + 1);
-    const double2 *cf = reinterpret_cast<const double2 *>(a.chi + (size_t)k0 * V * V * 4);
-#pragma unroll
-    for (int ab = 0; ab < V * V; ++ab) {
-      const double2 lo = cf[2 * ab], hi2 = cf[2 * ab + 1];
-      X[ab] = (T)(((hi2.y * tt + hi2.x) * tt + lo.y) * tt + lo.x);
-    }
-  }
-  C H[V];
-#pragma unroll
-  for (int va = 0; va < V; ++va) {
-    T hr = 0, hi = 0;
-#pragma unroll
-    for (int vb = 0; vb < V; ++vb) {
-      const T x = X[va * V + vb];
-      hr += F[vb].x * x;                       // oz, calculate_cuda.cu:44-58
-      hi += F[vb].y * x;
-    }
-    H[va] = mk<C>(hr, hi);
-  }
-  // repack for the inverse: dir (h_a + i h_b) at k and its mirror
-  // (timeirvol before the inverse, fft3d.cu:34)
-  const T d = (T)dir;
-#pragma unroll
-  for (int p = 0; p < P; ++p) {
-    const C ha = H[2 * p];
-    const C hb = (2 * p + 1 < V) ? H[2 * p + 1] : mk<C>(0.0, 0.0);
-    out[p] = mk<C>(d * (ha.x - hb.y), d * (ha.y + hb.x));
-    outm[p] = mk<C>(-d * (ha.x + hb.y), -d * (hb.x - ha.y));
-  }
-}
-
-template <typename T, int V>
-__device__ __forceinline__ void kspace_pair(const IterArgs<T> &a, long long j, int ix, int iy,
-                                            int iz, const typename Cx<T>::t *y,
-                                            const typename Cx<T>::t *ym,
-                                            typename Cx<T>::t *out, typename Cx<T>::t *outm) {
-  const double2 fk = a.nofk ? make_double2(0.0, 0.0) : a.fkh[j];
-  kspace_pair_fk<T, V>(a, fk, ix, iy, iz, y, ym, out, outm);
-}
-
 template <typename T, int V>
 __global__ void __launch_bounds__(kThreads) k_kspace(IterArgs<T> a0) {
   const IterArgs<T> a = solute_view<T, V>(a0);
@@ -588,9 +284,6 @@ __global__ void __launch_bounds__(kThreads) k_kspace(IterArgs<T> a0) {
 
 
 // ---------------------------------------------------------------- pass R
-__device__ void finalize_block(DevState *st, const double *part, int nblocks,
-                               double nv_points, double *hist, int hist_cap);
-
 template <typename T, int V, int CLOS, bool REF>
 __global__ void __launch_bounds__(kThreads) k_pass_r(IterArgs<T> a0) {
   const IterArgs<T> a = solute_view<T, V>(a0);
@@ -1628,71 +1321,6 @@ __global__ void __launch_bounds__(kThreads) k_pass_a_pipe(IterArgs<T> a0) {
   cp_wait<0>();
 }
 
-// ------------------------------------------------------------- finalize
-// Run by the last block of pass R to finish: fixed-order reduction of the
-// block sums, then the host logic of iterate.cu:52-62 and AN2::calculate
-// (anderson.cu:35-63) on one thread -- no separate launch, no host sync.
-__device__ void finalize_block(DevState *st, const double *part, int nblocks,
-                               double nv_points, double *hist, int hist_cap) {
-  // blocks of any multiple of kThreads threads: threads past the first
-  // kThreads fold their sums into those slots, one group at a time
-  __shared__ double red[6][kThreads];
-  double s[6] = {0, 0, 0, 0, 0, 0};
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
-#pragma unroll
-    for (int k = 0; k < 6; ++k) s[k] += __ldcg(part + (size_t)k * nblocks + b);
-  if (threadIdx.x < kThreads)
-#pragma unroll
-    for (int k = 0; k < 6; ++k) red[k][threadIdx.x] = s[k];
-  __syncthreads();
-  for (int g = kThreads; g < (int)blockDim.x; g += kThreads) {
-    if ((int)threadIdx.x >= g && (int)threadIdx.x < g + kThreads)
-#pragma unroll
-      for (int k = 0; k < 6; ++k) red[k][threadIdx.x - g] += s[k];
-    __syncthreads();
-  }
-  for (int w = min((int)blockDim.x, kThreads) / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w)
-#pragma unroll
-      for (int k = 0; k < 6; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x != 0) return;
-  for (int k = 0; k < 6; ++k) st->sums[k] = red[k][0];
-  const double rms = sqrt(red[0][0] / nv_points);
-  st->rms = rms;
-  if (st->measure) return;
-  st->iter += 1;
-  if (hist && st->iter <= hist_cap) hist[st->iter - 1] = rms;  // iterate.cu:63 output
-  if (!isfinite(rms)) { st->done = 2; st->mode = 0; return; }  // iterate.cu:54-57
-  if (rms <= st->conv) { st->done = 1; st->mode = 0; return; } // :58-59
-  if (st->watch) {                       // a phase that may hand over early
-    if (rms < 0.9 * st->best) { st->best = rms; st->since = 0; }
-    else if (++st->since > 30) { st->done = 4; st->mode = 0; return; }
-  }
-  if (st->count > 0) {                                         // anderson.cu:43-49
-    st->count -= 1;
-    st->mode = 1;
-  } else {                                                     // anderson.cu:50-61
-    // [[a00 a01][a01 a11]] x = [c0 c1], eliminated as leg() does (:87-112)
-    double a00 = red[3][0], a01 = red[4][0], a11 = red[5][0];
-    double c0 = red[1][0], c1 = red[2][0];
-    double p = a00;
-    double a01n = a01 / p;
-    double r = c0 / p;
-    double a11n = a11 - a01 * a01n;
-    double c1n = c1 - a01 * r;
-    double x1 = c1n / a11n;
-    double x0 = r - a01n * x1;
-    st->s1 = x0 + st->mp * ((st->binary == 0) ? 0.0 : 1.0);
-    st->s2 = x1 + st->mp * ((st->binary == 0) ? 1.0 : 0.0);
-    st->mode = 2;
-  }
-  st->upd_slot = st->binary;
-  st->binary = (st->binary == 0) ? 1 : 0;
-  if (st->iter >= st->maxstep) st->done = 3;   // iterate.cu:51 loop bound
-}
-
 // -------------------------------------------- depth-M Anderson (opt-in)
 // RISM3D_MDIIS=M (2..kDmMax): the plain FP32 bulk of a mixed single-solute
 // solve mixes the last M history entries instead of AN2's two.  Slot i holds
@@ -2194,8 +1822,31 @@ void launch_iteration_dm(Context &c, const IterArgs<float> &a, cufftHandle plan)
   k_pass_r_dm<V, CLOS><<<a.nblocks, kThreads, 0, c.stream>>>(a, c.dm_depth);
 }
 
+template <typename T> fused::Vtable<T> fused_table(int N, int V) {
+  return N <= 64 ? fused::table_small<T>(N, V)
+                 : N <= 128 ? fused::table_medium<T>(N, V) : fused::table_large<T>(N, V);
+}
+
+// One iteration (or with which >= 0 one of its kernels) in the three-kernel
+// form (fused.cuh).
+template <typename T>
+void launch_fused(Context &c, const IterArgs<T> &a, bool ref, int which = -1) {
+  const FusedPlan &f = sizeof(T) == 8 ? c.fu64 : c.fu32;
+  const int hnc = c.prm.closure == RISM3D_HNC;
+  const fused::Vtable<T> tab = fused_table<T>(c.nx, c.natv);
+  IterArgs<T> ar = a;
+  ar.nblocks = (which == 4 ? f.cp[ref ? 1 : 0] : f.cr[ref ? 1 : 0]) * f.nc;
+  if (which == 4) cudaMemsetAsync(c.d_bar, 0, sizeof(unsigned) * c.nb, c.stream);
+  for (int k = 0; k < 5; ++k)
+    if (which < 0 ? k < 3 : which == k) tab.launch(f, k, ref, hnc, c.nb, ar, c.stream);
+}
+
 template <typename T, int V, int CLOS, bool REF>
 void launch_iteration(Context &c, const IterArgs<T> &a, cufftHandle plan) {
+  if (a.RPx) {
+    launch_fused<T>(c, a, REF);
+    return;
+  }
   if constexpr (sizeof(T) == 4 && !REF) {
     if (c.dm_depth && (const void *)a.Y == (const void *)c.f_Ydm) {
       launch_iteration_dm<V, CLOS>(c, a, plan);
@@ -2289,22 +1940,8 @@ cudaGraphExec_t capture(Context &c, const IterArgs<T> &a, cufftHandle plan) {
   return x;
 }
 
-// End of one device-side loop body: keep looping while any solute is still
-// running or has not yet had the idle pass after its stop (the snapshot);
-// the body count is bounded by the phase's step limit plus a margin.
 __global__ void k_loop_cond(cudaGraphConditionalHandle h, DevState *st, int nb) {
-  if (threadIdx.x != 0) return;
-  bool more = false;
-  int cap = 1;                 // the largest step budget left to any solute
-  for (int b = 0; b < nb; ++b) {
-    if (!(st[b].done && st[b].after_done >= 1)) more = true;
-    cap = max(cap, st[b].maxstep);
-  }
-  const int loops = ++st[0].loops;
-  st[0].bodies += 1;
-  cap = cap < 1000000 ? cap : 1000000;
-  if (loops >= cap + 4) more = false;
-  cudaGraphSetConditional(h, more ? 1u : 0u);
+  if (threadIdx.x == 0) loop_test(h, st, nb);
 }
 
 // One whole phase as a single graph: a while node whose body is one
@@ -2332,8 +1969,15 @@ cudaGraphExec_t capture_loop(Context &c, const IterArgs<T> &a, cufftHandle plan)
     ok = cudaStreamBeginCaptureToGraph(c.stream, body, nullptr, nullptr, 0,
                                        cudaStreamCaptureModeThreadLocal) == cudaSuccess;
     if (ok) {
-      launch_iteration<T, V, CLOS, REF>(c, a, plan);
-      k_loop_cond<<<1, 32, 0, c.stream>>>(h, a.st, c.nb);
+      if (a.RPx) {                               // plane R runs the loop test
+        IterArgs<T> al = a;
+        al.cond = h;
+        al.loop = 1;
+        launch_iteration<T, V, CLOS, REF>(c, al, plan);
+      } else {
+        launch_iteration<T, V, CLOS, REF>(c, a, plan);
+        k_loop_cond<<<1, 32, 0, c.stream>>>(h, a.st, c.nb);
+      }
       cudaGraph_t out = nullptr;
       ok = cudaStreamEndCapture(c.stream, &out) == cudaSuccess;
     }
@@ -2358,13 +2002,14 @@ enum PhaseKind { kPlain32 = 0, kRefine32 = 1, kFinal64 = 2, kBase64 = 3 };
 // an FP32 divergence (fallback) is skipped: one idle body.  The final FP64
 // phase restarts AN2 from Picard steps when the history was discarded.
 __global__ void k_phase_begin(DevState *st, int nb, int kind, double conv, int maxstep,
-                              int watch, int an2_count) {
+                              int watch, int an2_count, int rotate) {
   const bool fallback = st[0].fallback != 0;
   const bool fresh = fallback || st[0].restart_next != 0;
   __syncthreads();
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
     DevState &s = st[b];
     s.done = 0; s.after_done = 0; s.iter = 0; s.mode = 0;
+    s.rotate = rotate; s.rp[0] = 0; s.rp[1] = 1; s.rp[2] = 2;
     if (kind == kBase64) continue;
     s.conv = conv;
     s.maxstep = max(1, maxstep - s.stage_iter);
@@ -2411,6 +2056,36 @@ __global__ void k_promote_base(long long total, const float *tf, const DevState 
     t[f] = fallback ? 0.0 : (double)tf[f];
 }
 
+// Residual history back in slots 0 and 1 after a three-kernel phase (which
+// renames slots instead of copying them); arrays [B][2][V][N] and [B][V][N].
+template <typename T, int V>
+__global__ void __launch_bounds__(kThreads)
+k_rp_order(long long vn, const DevState *st, T *RP, const T *RPx) {
+  const int r0 = st[blockIdx.y].rp[0], r1 = st[blockIdx.y].rp[1];
+  if (r0 == 0 && r1 == 1) return;
+  RP += blockIdx.y * 2 * (size_t)vn;
+  RPx += blockIdx.y * (size_t)vn;
+  const T *p0 = r0 < 2 ? RP + r0 * (size_t)vn : RPx, *p1 = r1 < 2 ? RP + r1 * (size_t)vn : RPx;
+  for (long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x; f < vn;
+       f += (long long)gridDim.x * blockDim.x) {
+    const T a = p0[f], b = p1[f];
+    RP[f] = a;
+    RP[vn + f] = b;
+  }
+}
+
+template <typename T>
+void set_fused_args(Context &c, IterArgs<T> &a) {
+  const FusedPlan &f = sizeof(T) == 8 ? c.fu64 : c.fu32;
+  a.RPx = (T *)(sizeof(T) == 8 ? (void *)c.d_RPx : (void *)c.f_RPx);
+  a.roots = (const typename Cx<T>::t *)(sizeof(T) == 8 ? (void *)c.d_roots : (void *)c.f_roots);
+  a.scr = (typename Cx<T>::t *)c.d_scr;
+  a.scr_n = (long long)std::max(std::max(f.cr[0], f.cr[1]), std::max(f.cp[0], f.cp[1])) * c.nx * c.nx;
+  a.nb = c.nb;
+  a.gcount = c.d_count + c.nb;
+  a.bar = c.d_bar;
+}
+
 // One phase: the device-side loop graph when available (no host sync), else
 // iterations driven from the host.  Progress lines and the optional trace
 // need the host and synchronise.
@@ -2425,8 +2100,12 @@ int run_phase(Context &c, cufftHandle plan, T *t, T *U, T *Y, T *RP,
   a.gout = snapshot ? c.d_g : nullptr;
   a.tw = (const typename Cx<T>::t *)(sizeof(T) == 8 ? (void *)c.d_tw : (void *)c.d_twf);
   const int nb = c.nb;
+  // the three-kernel iteration (not for the opt-in forms of the FP32 bulk)
+  const bool fused = (sizeof(T) == 8 ? c.fu64.on : c.fu32.on) &&
+                     !(sizeof(T) == 4 && !REF && (c.dm_depth || c.xfused));
+  if (fused) set_fused_args<T>(c, a);
   k_phase_begin<<<1, 128, 0, c.stream>>>(c.d_state, nb, kind, conv, c.prm.maxstep,
-                                         watch ? 1 : 0, c.prm.an2_count);
+                                         watch ? 1 : 0, c.prm.an2_count, fused ? 1 : 0);
   c.launches += 1;
   if (!cufft_ok(c, cufftSetStream(plan, c.stream), "cufftSetStream")) return RISM3D_CUFFT_ERROR;
   if (c.plan32z && !cufft_ok(c, cufftSetStream(c.plan32z, c.stream), "cufftSetStream"))
@@ -2434,18 +2113,26 @@ int run_phase(Context &c, cufftHandle plan, T *t, T *U, T *Y, T *RP,
   int status = RISM3D_OK;
   static const bool trace = getenv("RISM3D_TRACE") && getenv("RISM3D_TRACE")[0] == '1';
   cudaGraphExec_t &lx = REF ? c.loop32r : (sizeof(T) == 8) ? c.loop64 : c.loop32;
-  if (!lx && !c.no_device_loop) {
+  // one launch for the phase (not while iterations are driven from the host)
+  const bool one = fused && !c.no_device_loop &&
+                   (sizeof(T) == 8 ? c.fu64 : c.fu32).cp[REF ? 1 : 0] > 0;
+  if (!one && !lx && !c.no_device_loop) {
     lx = capture_loop<T, V, CLOS, REF>(c, a, plan);
     if (!lx) c.no_device_loop = true;
   }
-  if (lx) {
+  if (one || lx) {
     cudaEvent_t t0 = nullptr, t1 = nullptr;
     if (trace) {
       cudaEventCreate(&t0);
       cudaEventCreate(&t1);
       cudaEventRecord(t0, c.stream);
     }
-    if (!cuda_ok(c, cudaGraphLaunch(lx, c.stream), "phase launch")) return RISM3D_CUDA_ERROR;
+    if (one) {
+      launch_fused<T>(c, a, REF, 4);
+      c.launches += 1;
+    }
+    if (!cuda_ok(c, one ? cudaGetLastError() : cudaGraphLaunch(lx, c.stream), "phase launch"))
+      return RISM3D_CUDA_ERROR;
     if (trace) {
       cudaEventRecord(t1, c.stream);
       DevState s0;
@@ -2501,6 +2188,12 @@ int run_phase(Context &c, cufftHandle plan, T *t, T *U, T *Y, T *RP,
   }
   // the loop's bodies (4 launches each: passes A, K, R and the loop test)
   // are counted from the device record at the end of the solve
+  if (fused) {
+    launch_fused<T>(c, a, REF, 3);
+    k_rp_order<T, V><<<dim3(grid_blocks((long long)V * c.n), nb), kThreads, 0, c.stream>>>(
+        (long long)V * c.n, a.st, a.RP, a.RPx);
+    c.launches += 2;
+  }
   k_phase_end<<<1, 128, 0, c.stream>>>(c.d_state, nb, kind, sizeof(T) == 4 ? 1 : 0);
   c.launches += 1;
   // progress lines of the reference (iterate.cu:63), from the device record
@@ -2522,7 +2215,7 @@ int run_phase(Context &c, cufftHandle plan, T *t, T *U, T *Y, T *RP,
 template <int V, int CLOS>
 int refine_base(Context &c) {
   const int nb = c.nb;
-  k_phase_begin<<<1, 128, 0, c.stream>>>(c.d_state, nb, kBase64, 0.0, 0, 0, 0);
+  k_phase_begin<<<1, 128, 0, c.stream>>>(c.d_state, nb, kBase64, 0.0, 0, 0, 0, 0);
   IterArgs<double> a = make_args<double>(c, true);
   a.buf = c.d_buf; a.t = c.d_t; a.U = c.d_U; a.Y = c.d_Y; a.RP = c.d_RP;
   a.tw = c.d_tw;
@@ -2686,7 +2379,7 @@ int solve_v(Context &c, int chargeup) {
       c.err = "a device-side wait gave up: a bulk or tile copy never arrived";
       status = RISM3D_CUDA_ERROR;
     }
-  c.launches += 4 * bodies;
+  c.launches += (c.fu64.on ? 3 : 4) * bodies;
   c.res.rms = fs[0].rms;
   if (nb > 1) {
     c.bres.assign(nb, rism3d_result{});
@@ -2741,6 +2434,12 @@ int time_kernel_t(Context &c, int which, int reps, double *ms) {
   run.done = 0; run.after_done = 0; run.mode = 2; run.count = 0; run.upd_slot = 0;
   run.measure = 1;
   run.s1 = 0.25; run.s2 = 0.25;
+  // the three-kernel iteration, where the solve runs it (14 is a transform)
+  const bool three = which != 14 && (fp64 ? c.fu64.on : c.fu32.on) &&
+                     !(!fp64 && which < 13 && (c.dm_depth || c.xfused));
+  if (three) set_fused_args<T>(c, a);
+  run.rotate = three ? 1 : 0;
+  run.rp[0] = 0; run.rp[1] = 1; run.rp[2] = 2;
   cudaMemcpy(c.d_state, &run, sizeof(DevState), cudaMemcpyHostToDevice);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
@@ -2751,10 +2450,15 @@ int time_kernel_t(Context &c, int which, int reps, double *ms) {
             bk = wave_blocks(k_kspace<T, V>, a.n / 2, 1);
   cudaEventRecord(e0, c.stream);
   bool fused_done = false;
+  if (three) {                                   // plane A / z lines / plane R
+    const bool ref = which == 13 || which == 15;
+    for (int r = 0; r < reps; ++r) launch_fused<T>(c, a, ref, ref ? which - 13 : which % 10);
+    fused_done = true;
+  }
   if constexpr (sizeof(T) == 4 && V <= 2) {
     // the fused-axis passes the FP32 solve runs (ids as below; 14: one
     // cuFFT transform along z)
-    if (c.xfused && which != 14) {
+    if (c.xfused && which != 14 && !three) {
       if (c.nx == 256) time_fused<V, CLOS, 16>(c, a, which, reps);
       else time_fused<V, CLOS, 8>(c, a, which, reps);
       fused_done = true;
@@ -2862,6 +2566,54 @@ int setup_pipe_r(Context &c) {
   if (e == cudaSuccess) e = c.natv == 1 ? bulk_r_attrs<float, 1>() : bulk_r_attrs<float, 2>();
   if (!cuda_ok(c, e, "bulk pass R attributes")) return RISM3D_CUDA_ERROR;
   c.bulk_r = true;
+  return RISM3D_OK;
+}
+
+// The three-kernel iteration: cubic cells (edges and lengths equal, so that
+// chi comes from the per-|k|^2 table) whose edge has an instantiation, up to
+// four sites.  Other cells, and RISM3D_FUSED=0, keep the passes around the
+// 3D library transforms.
+int setup_fused_iteration(Context &c) {
+  c.fu64 = FusedPlan{};
+  c.fu32 = FusedPlan{};
+  const char *off = getenv("RISM3D_FUSED");
+  if ((off && off[0] == '0') || c.natv > 4 || c.nx != c.ny || c.nx != c.nz ||
+      c.prm.box[0] != c.prm.box[1] || c.prm.box[0] != c.prm.box[2])
+    return RISM3D_OK;
+  const bool mixed = c.prm.precision == RISM3D_MIXED;
+  const fused::Vtable<double> t64 = fused_table<double>(c.nx, c.natv);
+  const fused::Vtable<float> t32 = fused_table<float>(c.nx, c.natv);
+  if (!t64.setup || (mixed && !t32.setup)) return RISM3D_OK;
+  if (!t64.setup(c.fu64, c.nb) || (mixed && !t32.setup(c.fu32, c.nb))) return RISM3D_OK;
+  const int N = c.nx;
+  auto max_cr = [](const FusedPlan &f) {
+    return (size_t)std::max(std::max(f.cr[0], f.cr[1]), std::max(f.cp[0], f.cp[1]));
+  };
+  // block sums: six per CTA of plane R in the partials' room
+  if (6 * max_cr(c.fu64) * c.fu64.nc > 64 * (size_t)c.nred_blocks ||
+      (mixed && 6 * max_cr(c.fu32) * c.fu32.nc > 64 * (size_t)c.nred_blocks))
+    return RISM3D_OK;
+  std::vector<double2> roots(N);
+  std::vector<float2> rootsf(N);
+  for (int m = 0; m < N; ++m) {
+    const double ang = 2.0 * kPi * m / N;
+    roots[m] = make_double2(cos(ang), -sin(ang));
+    rootsf[m] = make_float2((float)roots[m].x, (float)roots[m].y);
+  }
+  const size_t vn = (size_t)c.n * c.nb * c.natv;
+  const size_t scr = std::max(max_cr(c.fu64) * sizeof(double2), max_cr(c.fu32) * sizeof(float2)) *
+                     (size_t)N * N * c.nb;
+  if (!cuda_ok(c, cudaMalloc(&c.d_RPx, sizeof(double) * vn), "alloc residual slot") ||
+      (mixed && !cuda_ok(c, cudaMalloc(&c.f_RPx, sizeof(float) * vn), "alloc residual slot")) ||
+      !cuda_ok(c, cudaMalloc(&c.d_scr, scr), "alloc exchange planes") ||
+      !cuda_ok(c, cudaMalloc(&c.d_bar, sizeof(unsigned) * c.nb), "alloc barrier") ||
+      !cuda_ok(c, cudaMalloc(&c.d_roots, sizeof(double2) * N), "alloc roots") ||
+      !cuda_ok(c, cudaMalloc(&c.f_roots, sizeof(float2) * N), "alloc roots") ||
+      !cuda_ok(c, cudaMemcpy(c.d_roots, roots.data(), sizeof(double2) * N, cudaMemcpyHostToDevice), "copy roots") ||
+      !cuda_ok(c, cudaMemcpy(c.f_roots, rootsf.data(), sizeof(float2) * N, cudaMemcpyHostToDevice), "copy roots"))
+    return RISM3D_CUDA_ERROR;
+  c.fu64.on = true;
+  c.fu32.on = mixed;
   return RISM3D_OK;
 }
 
