@@ -1614,11 +1614,11 @@ __global__ void k_shift_history(long long n, int nv, long long total, const doub
 }
 
 // Refinement base, after one FP64 cycle at t0 (buf holds its inverse
-// transform): R0 = h + 1 - C(t0 - U), x0 = t0 - U, d = 0, and the FP32 AN2
-// history re-expressed as corrections to t0 (Y_i - t0; RP_i unchanged).
+// transform): R0 = h + 1 - C(t0 - U), x0 = t0 - U, d = 0, and the AN2
+// history re-expressed as FP32 corrections to t0 (Y_i - t0; RP_i unchanged).
 template <int V, int CLOS>
 __global__ void __launch_bounds__(kThreads)
-k_refine_base(IterArgs<double> a0, float *R0, float *x0, float *d, float *Yf) {
+k_refine_base(IterArgs<double> a0, float *R0, float *x0, float *d, float *Yf, int again) {
   const IterArgs<double> a = solute_view<double, V>(a0);
   constexpr int P = (V + 1) / 2;
   const long long n = a.n;
@@ -1645,8 +1645,11 @@ k_refine_base(IterArgs<double> a0, float *R0, float *x0, float *d, float *Yf) {
       R0[iv] = (float)(h[v] + 1.0 - closure<CLOS>(x));
       x0[iv] = (float)x;
       d[iv] = 0.0f;
-      Yf[iv] = (float)((double)Yf[iv] - t0);
-      Yf[(size_t)V * n + iv] = (float)((double)Yf[(size_t)V * n + iv] - t0);
+      // the bulk's history is absolute in FP32; a later round's is relative
+      // to the last base, with its absolute FP64 values in Y
+      const size_t i1 = (size_t)V * n + iv;
+      Yf[iv] = (float)((again ? a.Y[iv] : (double)Yf[iv]) - t0);
+      Yf[i1] = (float)((again ? a.Y[i1] : (double)Yf[i1]) - t0);
     }
   }
 }
@@ -2001,8 +2004,10 @@ enum PhaseKind { kPlain32 = 0, kRefine32 = 1, kFinal64 = 2, kBase64 = 3 };
 // budget is what the stage has left (iterate.cu:51).  A refinement after
 // an FP32 divergence (fallback) is skipped: one idle body.  The final FP64
 // phase restarts AN2 from Picard steps when the history was discarded.
+// A second or later refinement round (`again`) is skipped when the stage's
+// steps are used up or an earlier round blew up.
 __global__ void k_phase_begin(DevState *st, int nb, int kind, double conv, int maxstep,
-                              int watch, int an2_count, int rotate) {
+                              int watch, int an2_count, int rotate, int again) {
   const bool fallback = st[0].fallback != 0;
   const bool fresh = fallback || st[0].restart_next != 0;
   __syncthreads();
@@ -2014,21 +2019,26 @@ __global__ void k_phase_begin(DevState *st, int nb, int kind, double conv, int m
     s.conv = conv;
     s.maxstep = max(1, maxstep - s.stage_iter);
     s.watch = watch; s.since = 0; s.best = 1e300; s.loops = 0;
-    if (kind == kRefine32 && fallback) { s.done = 4; s.after_done = 1; }
+    if (kind == kRefine32 &&
+        (fallback || (again && (s.stage_iter >= maxstep || st[0].restart_next)))) {
+      s.done = 4;
+      s.after_done = 1;
+    }
     if (kind == kPlain32) { s.dm_fill = 0; s.dm_last = -1; s.dm_use = 0; }
     if (kind == kFinal64 && fresh) { s.count = an2_count; s.binary = 0; }
   }
 }
 
 // End of a phase: step counters, and the flags the next phases read.
-__global__ void k_phase_end(DevState *st, int nb, int kind, int fp32) {
+__global__ void k_phase_end(DevState *st, int nb, int kind, int fp32, int again, int maxstep) {
   __shared__ int any_div;
   if (threadIdx.x == 0) any_div = 0;
   __syncthreads();
   const bool fallback = st[0].fallback != 0;
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
     DevState &s = st[b];
-    const int steps = kind == kBase64 ? (fallback ? 0 : 1) : s.iter;
+    const bool idle = fallback || (again && (s.stage_iter >= maxstep || st[0].restart_next));
+    const int steps = kind == kBase64 ? (idle ? 0 : 1) : s.iter;
     s.stage_iter += steps;
     s.total_iter += steps;
     if (fp32) s.total32 += steps;
@@ -2037,7 +2047,8 @@ __global__ void k_phase_end(DevState *st, int nb, int kind, int fp32) {
   __syncthreads();
   if (threadIdx.x == 0) {
     if (kind == kPlain32) st[0].fallback = any_div;
-    if (kind == kRefine32 && !fallback) st[0].restart_next = any_div;
+    if (kind == kRefine32 && !fallback && !(again && st[0].restart_next))
+      st[0].restart_next = any_div;
   }
 }
 
@@ -2092,7 +2103,7 @@ void set_fused_args(Context &c, IterArgs<T> &a) {
 template <typename T, int V, int CLOS, bool REF>
 int run_phase(Context &c, cufftHandle plan, T *t, T *U, T *Y, T *RP,
               typename Cx<T>::t *buf, bool snapshot, int kind, double conv, bool watch,
-              const T *R0 = nullptr) {
+              const T *R0 = nullptr, bool again = false) {
   IterArgs<T> a = make_args<T>(c, sizeof(T) == 8);
   a.buf = buf; a.t = t; a.U = U; a.Y = Y; a.RP = RP;
   if (REF) { a.R0 = R0; a.sp = c.d_stage_ref; a.nofk = 1; }
@@ -2105,7 +2116,7 @@ int run_phase(Context &c, cufftHandle plan, T *t, T *U, T *Y, T *RP,
                      !(sizeof(T) == 4 && !REF && (c.dm_depth || c.xfused));
   if (fused) set_fused_args<T>(c, a);
   k_phase_begin<<<1, 128, 0, c.stream>>>(c.d_state, nb, kind, conv, c.prm.maxstep,
-                                         watch ? 1 : 0, c.prm.an2_count, fused ? 1 : 0);
+                                         watch ? 1 : 0, c.prm.an2_count, fused ? 1 : 0, again ? 1 : 0);
   c.launches += 1;
   if (!cufft_ok(c, cufftSetStream(plan, c.stream), "cufftSetStream")) return RISM3D_CUFFT_ERROR;
   if (c.plan32z && !cufft_ok(c, cufftSetStream(c.plan32z, c.stream), "cufftSetStream"))
@@ -2194,7 +2205,8 @@ int run_phase(Context &c, cufftHandle plan, T *t, T *U, T *Y, T *RP,
         (long long)V * c.n, a.st, a.RP, a.RPx);
     c.launches += 2;
   }
-  k_phase_end<<<1, 128, 0, c.stream>>>(c.d_state, nb, kind, sizeof(T) == 4 ? 1 : 0);
+  k_phase_end<<<1, 128, 0, c.stream>>>(c.d_state, nb, kind, sizeof(T) == 4 ? 1 : 0,
+                                       again ? 1 : 0, c.prm.maxstep);
   c.launches += 1;
   // progress lines of the reference (iterate.cu:63), from the device record
   if (status == RISM3D_OK && c.prm.verbose && nb == 1 && c.d_hist) {
@@ -2213,9 +2225,9 @@ int run_phase(Context &c, cufftHandle plan, T *t, T *U, T *Y, T *RP,
 // both transforms, the k-space pass with the stage's fk), then the
 // refinement base: R0, x0, d = 0 and the FP32 history relative to t0.
 template <int V, int CLOS>
-int refine_base(Context &c) {
+int refine_base(Context &c, bool again) {
   const int nb = c.nb;
-  k_phase_begin<<<1, 128, 0, c.stream>>>(c.d_state, nb, kBase64, 0.0, 0, 0, 0, 0);
+  k_phase_begin<<<1, 128, 0, c.stream>>>(c.d_state, nb, kBase64, 0.0, 0, 0, 0, 0, again ? 1 : 0);
   IterArgs<double> a = make_args<double>(c, true);
   a.buf = c.d_buf; a.t = c.d_t; a.U = c.d_U; a.Y = c.d_Y; a.RP = c.d_RP;
   a.tw = c.d_tw;
@@ -2231,8 +2243,9 @@ int refine_base(Context &c) {
   if (!cufft_ok(c, cufftExecZ2Z(c.plan64, (cufftDoubleComplex *)a.buf, (cufftDoubleComplex *)a.buf,
                                 CUFFT_INVERSE), "refine base FFT"))
     return RISM3D_CUFFT_ERROR;
-  k_refine_base<V, CLOS><<<bb, kThreads, 0, c.stream>>>(a, c.f_R0, c.f_x0, c.f_t, c.f_Y);
-  k_phase_end<<<1, 128, 0, c.stream>>>(c.d_state, nb, kBase64, 0);
+  k_refine_base<V, CLOS><<<bb, kThreads, 0, c.stream>>>(a, c.f_R0, c.f_x0, c.f_t, c.f_Y,
+                                                         again ? 1 : 0);
+  k_phase_end<<<1, 128, 0, c.stream>>>(c.d_state, nb, kBase64, 0, again ? 1 : 0, c.prm.maxstep);
   c.launches += 6;
   return cuda_ok(c, cudaGetLastError(), "refine base") ? RISM3D_OK : RISM3D_CUDA_ERROR;
 }
@@ -2322,8 +2335,16 @@ int solve_v(Context &c, int chargeup) {
       k_convert<double, float><<<gb, kThreads, 0, c.stream>>>(2 * vn, c.d_Y, c.f_Y);
       k_convert<double, float><<<gb, kThreads, 0, c.stream>>>(2 * vn, c.d_RP, c.f_RP);
       c.launches += 3;
-      double sw = c.prm.mixed_switch > 0 ? c.prm.mixed_switch : 100.0 * c.prm.convergence;
-      if (sw < c.prm.convergence) sw = c.prm.convergence;
+      // The plain form's residual falls like the FP64 one's down to about
+      // 5e-5 and then drags along its rounding floor (256^3, conv 5e-9: 180
+      // steps to 6.8e-5, 354 more to 1.0e-5), so it hands over at 1e-4 at the
+      // latest.  A refinement in turn drags below about 5e-3 of its base's
+      // residual: it runs in rounds of at most a factor 200, each on a base
+      // of its own (one FP64 cycle).
+      const double conv = c.prm.convergence;
+      double sw = c.prm.mixed_switch > 0 ? c.prm.mixed_switch : std::max(100.0 * conv, 1e-4);
+      if (sw < conv) sw = conv;
+      const int rounds = std::max(1, (int)ceil(log(sw / conv) / log(200.0)));
       st = run_phase<float, V, CLOS, false>(c, c.plan32, c.f_t, c.f_U,
                                            c.dm_depth ? c.f_Ydm : c.f_Y,
                                            c.dm_depth ? c.f_RPdm : c.f_RP, c.f_buf,
@@ -2336,14 +2357,18 @@ int solve_v(Context &c, int chargeup) {
       }
       k_promote_base<<<gb, kThreads, 0, c.stream>>>(vn, c.f_t, c.d_state, c.d_t);
       c.launches += 1;
-      st = refine_base<V, CLOS>(c);
+      for (int r = 0; r < rounds && st == RISM3D_OK; ++r) {
+        const double target = r + 1 == rounds ? conv : sw * pow(conv / sw, (r + 1.0) / rounds);
+        st = refine_base<V, CLOS>(c, r > 0);
+        if (st == RISM3D_OK)
+          st = run_phase<float, V, CLOS, true>(c, c.plan32, c.f_t, c.f_x0, c.f_Y, c.f_RP, c.f_buf,
+                                              false, kRefine32, target, true, c.f_R0, r > 0);
+        if (st != RISM3D_OK) break;
+        k_refine_finish<<<gb, kThreads, 0, c.stream>>>(n, V, vnb, c.f_t, c.f_Y, c.f_RP, c.d_state,
+                                                      c.d_t, c.d_Y, c.d_RP);
+        c.launches += 1;
+      }
       if (st != RISM3D_OK) { status = st; break; }
-      st = run_phase<float, V, CLOS, true>(c, c.plan32, c.f_t, c.f_x0, c.f_Y, c.f_RP, c.f_buf,
-                                          false, kRefine32, c.prm.convergence, true, c.f_R0);
-      if (st != RISM3D_OK) { status = st; break; }
-      k_refine_finish<<<gb, kThreads, 0, c.stream>>>(n, V, vnb, c.f_t, c.f_Y, c.f_RP, c.d_state,
-                                                    c.d_t, c.d_Y, c.d_RP);
-      c.launches += 1;
     }
     st = run_phase<double, V, CLOS, false>(c, c.plan64, c.d_t, c.d_U, c.d_Y, c.d_RP, c.d_buf,
                                           true, kFinal64, c.prm.convergence, false);

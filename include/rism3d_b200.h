@@ -66,7 +66,8 @@ typedef struct {
   double an2_m;           /* AN2 mixing factor */
   double an2_mp;          /* AN2 bias on the newer slot */
   int precision;          /* RISM3D_FP64 or RISM3D_MIXED */
-  double mixed_switch;    /* MIXED: plain FP32 -> FP32 refinement once rms <= this (0 = 100 x convergence) */
+  double mixed_switch;    /* MIXED: plain FP32 -> FP32 refinement once rms <= this (0 = 100 x convergence, at least 1e-4: below
+                             that the plain form drags along its rounding floor) */
   int device;             /* CUDA ordinal (main.cu:57) */
   int verbose;            /* 1: print " Step = n Reside = r" like iterate.cu:63 */
   void *stream;           /* caller-owned cudaStream_t for all work; NULL: the

@@ -131,3 +131,24 @@ def test_batch_of_several_solutes(monkeypatch, chunk):
         assert a["status"] == b["status"] == 0
         assert a["iterations"] == b["iterations"]
         assert abs(a["sfe_sc"] - b["sfe_sc"]) < 1e-6 * abs(b["sfe_sc"])
+
+
+def test_refinement_rounds_reach_a_tight_tolerance(monkeypatch):
+    """Tight mixed solves refine in rounds, each on an FP64 base of its own:
+    few FP64 steps, and the FP64 solution."""
+    a = _solve(monkeypatch, True, 64, WATER, precision=1, convergence=1e-9)
+    b = _solve(monkeypatch, True, 64, WATER, convergence=1e-9)
+    assert a[0]["status"] == 0 and a[0]["rms"] <= 1e-9
+    assert a[0]["iterations"] - a[0]["iterations_fp32"] <= 8
+    # residuals of 1e-9 leave g apart by some 1e2 times that
+    assert _rel(a[1], b[1]) < 1e-6
+    assert abs(a[0]["sfe_sc"] - b[0]["sfe_sc"]) < 1e-7 * abs(b[0]["sfe_sc"])
+
+
+@pytest.mark.parametrize("maxstep", [1, 5, 150])
+def test_step_limit_of_a_mixed_solve(monkeypatch, maxstep):
+    """Rounds after the step limit are skipped: the base, one refinement step
+    and one FP64 step follow it, as with a single round."""
+    a = _solve(monkeypatch, True, 48, WATER, precision=1, convergence=1e-10, maxstep=maxstep)
+    assert a[0]["status"] == 6
+    assert maxstep < a[0]["iterations"] <= maxstep + 3
