@@ -45,17 +45,17 @@
 #include <type_traits>
 #include <vector>
 
+#include "adjoint_state.h"
 #include "rism3d_impl.h"
 #include "halfshift.cuh"
 
 namespace rism3d {
 namespace {
 
-constexpr int kThreads = 256;
 constexpr int kAtomsPerBlock = 128;
 constexpr int kPtsTile = 128;
 constexpr int NOUT = 6;   // dq, dsigma, deps, dRx, dRy, dRz
-constexpr int kDepth = 6; // Anderson history of the adjoint solve
+constexpr int kDepth = fused::kAdjDepth; // Anderson history of the adjoint solve
 constexpr int kDotBlocks = 2368;
 
 struct SiteW {
@@ -542,6 +542,58 @@ template <typename T> struct SolveTol;
 template <> struct SolveTol<double> { static constexpr double tol = 1.0e-10; };
 template <> struct SolveTol<float> { static constexpr double tol = 2.0e-6; };
 
+// The whole Anderson solve as one launch (fused_adjoint.cuh): `done` is set
+// when it ran, with the steps taken; otherwise (no instantiation for the cell,
+// or not on this device) nothing has happened.
+template <int V, typename T, typename CT>
+int adjoint_one_launch(Context &c, const T *G, const T *w, T *xi, T *Lxi, T *ys, T *rs,
+                       double *part, const StageParams *sp0, CT *buf, double eta, double tol,
+                       int maxit, Scratch &S, bool &done, int &it, bool &stalled) {
+  done = false;
+  const FusedPlan &f = c.fu64;
+  if (!f.on || V > 4) return RISM3D_OK;
+  const fused::AdjointLaunch<T> launch = fused::adjoint_table<T>(c.nx, V);
+  fused::AdjointArgs<T> g{};
+  int clusters = 0;
+  if (!launch || !launch(g, &clusters, c.stream)) return RISM3D_OK;
+  const size_t N = c.nx;
+  IterArgs<T> &a = g.it;
+  a.n = c.n; a.nx = c.nx; a.ny = c.ny; a.nz = c.nz;
+  a.xs = c.d_xs; a.xs32 = c.d_xs32;
+  a.buf = buf;
+  a.tw = (const CT *)(sizeof(T) == 8 ? (void *)c.d_tw : (void *)c.d_twf);
+  a.roots = (const CT *)(sizeof(T) == 8 ? (void *)c.d_roots : (void *)c.f_roots);
+  a.invvol = 1.0 / c.vol; a.dv = c.dv;
+  a.fkh = c.d_fkh; a.nofk = 1;
+  a.sp = sp0;
+  a.bar = c.d_bar;
+  a.scr = S.get<CT>((size_t)clusters * N * N);
+  fused::AdjointState h{};
+  h.best = 1e300;
+  h.bnorm = -1.0;
+  g.st = S.get<fused::AdjointState>(1);
+  if (!a.scr || !g.st) { c.err = "adjoint: out of device memory"; return RISM3D_CUDA_ERROR; }
+  g.G = G; g.w = w; g.xi = xi; g.Lxi = Lxi; g.ys = ys; g.rs = rs; g.part = part;
+  g.eta = eta; g.tol = tol; g.maxit = maxit;
+  if (!cuda_ok(c, cudaMemcpyAsync(g.st, &h, sizeof(h), cudaMemcpyHostToDevice, c.stream), "adjoint") ||
+      !cuda_ok(c, cudaMemsetAsync(c.d_bar, 0, sizeof(unsigned), c.stream), "adjoint"))
+    return RISM3D_CUDA_ERROR;
+  if (!launch(g, nullptr, c.stream)) {
+    cuda_ok(c, cudaGetLastError(), "adjoint solve launch");
+    return RISM3D_CUDA_ERROR;
+  }
+  c.launches += 1;
+  if (!cuda_ok(c, cudaMemcpyAsync(&h, g.st, sizeof(h), cudaMemcpyDeviceToHost, c.stream), "adjoint") ||
+      !cuda_ok(c, cudaStreamSynchronize(c.stream), "adjoint"))
+    return RISM3D_CUDA_ERROR;
+  if (h.done == 2) { c.err = "adjoint solve diverged"; return RISM3D_DIVERGED; }
+  if (h.done == 5 || h.fault) { c.err = "adjoint: a device-side wait gave up"; return RISM3D_CUDA_ERROR; }
+  it = h.it;
+  stalled = h.done == 4;
+  done = true;
+  return RISM3D_OK;
+}
+
 // T: arithmetic and storage of the transposed-Jacobian solve (double: the
 // FP64 adjoint; float: the FP32 variant, with FP64 dot products, mixing
 // coefficients and sums).  The right-hand side w = L delta and the mismatch
@@ -623,7 +675,12 @@ int adjoint_v(Context &c, double *dq, double *dsig, double *deps, double *dR) {
   const double eta = 0.5, tol = SolveTol<T>::tol;
   const int maxit = 3000;
   bool stalled = false;
-  for (; it < maxit; ++it) {
+  // one launch where the cell has an instantiation, else driven from here
+  bool one = false;
+  rc = adjoint_one_launch<V, T>(c, G, w, xi, Lxi, ys, rs, dpart, sp0, bufT, eta, tol, maxit, S,
+                                one, it, stalled);
+  if (rc != RISM3D_OK) return rc;
+  for (; !one && it < maxit; ++it) {
     rc = LT.apply(V, xi, Lxi, sp0, st0);
     if (rc != RISM3D_OK) return rc;
     const int nd = ns < kDepth ? ns + 1 : kDepth;      // filled slots incl. this one

@@ -112,9 +112,8 @@ void free_device(Context &c) {
   c.d_fkt = nullptr;
   delete c.ky_map;
   c.ky_map = nullptr;
-  for (void *p : {(void *)c.d_RPx, (void *)c.f_RPx, c.d_scr, (void *)c.d_roots, (void *)c.f_roots,
-                  (void *)c.d_bar})
-    if (p) cudaFree(p);
+  if (c.d_fused) cudaFree(c.d_fused);
+  c.d_fused = nullptr;
   c.d_RPx = nullptr; c.f_RPx = nullptr; c.d_scr = nullptr; c.d_roots = nullptr; c.f_roots = nullptr;
   c.d_bar = nullptr;
   c.fu64.on = c.fu32.on = false;

@@ -158,6 +158,36 @@ __device__ __forceinline__ void columns(const CxT<T> *src, CxT<T> *dst, int c0, 
   }
 }
 
+// x-DFT of a row in its exchange slots (line[(x / R2) ST + x % R2], complete)
+// to dst; a thread's stage-1 inputs and outputs are its own slots.
+template <typename T, int N>
+__device__ __forceinline__ void rows_forward(CxT<T> *line, CxT<T> *dst, int t,
+                                             const CxT<T> *roots) {
+  typedef CxT<T> C;
+  using L = Lines<N>;
+  constexpr int R1 = L::R1, R2 = L::R2, ST = L::ST;
+  {
+    C v[R1];
+#pragma unroll
+    for (int j = 0; j < R1; ++j) v[j] = line[j * ST + t];
+    dft::run<R1, false>(v);
+#pragma unroll
+    for (int s = 1; s < R1; ++s) v[s] = cmul(v[s], roots[t * s]);
+#pragma unroll
+    for (int s = 0; s < R1; ++s) line[s * ST + t] = v[s];
+  }
+  row_sync<R2>();
+#pragma unroll 1
+  for (int s = t; s < R1; s += R2) {
+    C w[R2];
+#pragma unroll
+    for (int k = 0; k < R2; ++k) w[k] = line[s * ST + k];
+    dft::run<R2, false>(w);
+#pragma unroll
+    for (int k = 0; k < R2; ++k) __stcg(dst + s + R1 * k, w[k]);
+  }
+}
+
 // ---------------------------------------------------------------- plane A
 template <typename T, int N, int V, bool REF, bool WIDE>
 __device__ __forceinline__ void planes_a(const IterArgs<T> &a, const DevState *st, CxT<T> *sm,
@@ -250,28 +280,7 @@ __device__ __forceinline__ void planes_a(const IterArgs<T> &a, const DevState *s
           }
       }
       row_sync<R2>();
-      // x-DFT; a thread's stage-1 inputs and outputs are its own slots
-      {
-        C v[R1];
-#pragma unroll
-        for (int j = 0; j < R1; ++j) v[j] = line[j * ST + t];
-        dft::run<R1, false>(v);
-#pragma unroll
-        for (int s = 1; s < R1; ++s) v[s] = cmul(v[s], roots[t * s]);
-#pragma unroll
-        for (int s = 0; s < R1; ++s) line[s * ST + t] = v[s];
-      }
-      row_sync<R2>();
-#pragma unroll 1
-      for (int s = t; s < R1; s += R2) {
-        C w[R2];
-#pragma unroll
-        for (int k = 0; k < R2; ++k) w[k] = line[s * ST + k];
-        dft::run<R2, false>(w);
-        C *d = pb + (size_t)y * N + s;
-#pragma unroll
-        for (int k = 0; k < R2; ++k) __stcg(d + R1 * k, w[k]);
-      }
+      rows_forward<T, N>(line, pb + (size_t)y * N, t, roots);
     }
     plane_sync<L::NC>();                           // every row of the plane is in L2
     columns<T, N, false>(pb, pb, rank * L::SH, sm, roots);

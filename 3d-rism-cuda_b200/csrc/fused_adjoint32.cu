@@ -1,0 +1,20 @@
+// Instantiations of the adjoint's one-launch solve (fused_adjoint.cuh): FP32.
+#include "fused_adjoint.cuh"
+
+namespace rism3d {
+namespace fused {
+
+template <> AdjointLaunch<float> adjoint_table<float>(int N, int V) {
+  switch (N) {
+    case 32: return adjoint_table_v<float, 32>(V);
+    case 48: return adjoint_table_v<float, 48>(V);
+    case 64: return adjoint_table_v<float, 64>(V);
+    case 96: return adjoint_table_v<float, 96>(V);
+    case 128: return adjoint_table_v<float, 128>(V);
+    case 256: return adjoint_table_v<float, 256>(V);
+  }
+  return nullptr;
+}
+
+}  // namespace fused
+}  // namespace rism3d

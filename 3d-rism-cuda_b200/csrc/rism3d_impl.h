@@ -231,6 +231,7 @@ struct Context {
   // three-kernel iteration (fused.cuh), per arithmetic: third residual slot,
   // exchange planes, roots of unity of the cell edge
   FusedPlan fu64, fu32;
+  void *d_fused = nullptr;      // the allocation that holds the following
   double *d_RPx = nullptr;
   float *f_RPx = nullptr;
   void *d_scr = nullptr;

@@ -2618,25 +2618,33 @@ int setup_fused_iteration(Context &c) {
   if (6 * max_cr(c.fu64) * c.fu64.nc > 64 * (size_t)c.nred_blocks ||
       (mixed && 6 * max_cr(c.fu32) * c.fu32.nc > 64 * (size_t)c.nred_blocks))
     return RISM3D_OK;
-  std::vector<double2> roots(N);
-  std::vector<float2> rootsf(N);
+  // one allocation: [roots FP64 | roots FP32 | barrier counts | third residual
+  // slots | exchange planes]
+  std::vector<unsigned char> head((sizeof(double2) + sizeof(float2)) * N + sizeof(unsigned) * c.nb, 0);
+  double2 *roots = (double2 *)head.data();
+  float2 *rootsf = (float2 *)(roots + N);
   for (int m = 0; m < N; ++m) {
     const double ang = 2.0 * kPi * m / N;
     roots[m] = make_double2(cos(ang), -sin(ang));
     rootsf[m] = make_float2((float)roots[m].x, (float)roots[m].y);
   }
-  const size_t vn = (size_t)c.n * c.nb * c.natv;
+  auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+  const size_t vn = (size_t)c.n * c.nb * c.natv, h = up(head.size()), r64 = up(sizeof(double) * vn),
+               r32 = mixed ? up(sizeof(float) * vn) : 0;
   const size_t scr = std::max(max_cr(c.fu64) * sizeof(double2), max_cr(c.fu32) * sizeof(float2)) *
                      (size_t)N * N * c.nb;
-  if (!cuda_ok(c, cudaMalloc(&c.d_RPx, sizeof(double) * vn), "alloc residual slot") ||
-      (mixed && !cuda_ok(c, cudaMalloc(&c.f_RPx, sizeof(float) * vn), "alloc residual slot")) ||
-      !cuda_ok(c, cudaMalloc(&c.d_scr, scr), "alloc exchange planes") ||
-      !cuda_ok(c, cudaMalloc(&c.d_bar, sizeof(unsigned) * c.nb), "alloc barrier") ||
-      !cuda_ok(c, cudaMalloc(&c.d_roots, sizeof(double2) * N), "alloc roots") ||
-      !cuda_ok(c, cudaMalloc(&c.f_roots, sizeof(float2) * N), "alloc roots") ||
-      !cuda_ok(c, cudaMemcpy(c.d_roots, roots.data(), sizeof(double2) * N, cudaMemcpyHostToDevice), "copy roots") ||
-      !cuda_ok(c, cudaMemcpy(c.f_roots, rootsf.data(), sizeof(float2) * N, cudaMemcpyHostToDevice), "copy roots"))
+  unsigned char *base = nullptr;
+  if (!cuda_ok(c, cudaMalloc(&base, h + r64 + r32 + scr), "alloc three-kernel iteration"))
     return RISM3D_CUDA_ERROR;
+  c.d_fused = base;
+  if (!cuda_ok(c, cudaMemcpy(base, head.data(), head.size(), cudaMemcpyHostToDevice), "copy roots"))
+    return RISM3D_CUDA_ERROR;
+  c.d_roots = (double2 *)base;
+  c.f_roots = (float2 *)(c.d_roots + N);
+  c.d_bar = (unsigned *)(c.f_roots + N);
+  c.d_RPx = (double *)(base + h);
+  c.f_RPx = mixed ? (float *)(base + h + r64) : nullptr;
+  c.d_scr = base + h + r64 + r32;
   c.fu64.on = true;
   c.fu32.on = mixed;
   return RISM3D_OK;

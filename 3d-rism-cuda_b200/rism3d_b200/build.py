@@ -20,7 +20,8 @@ CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA, "bin", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 SOURCES = ["solver.cu", "fused_large64.cu", "fused_large32.cu", "fused_medium64.cu",
-           "fused_medium32.cu", "fused_small64.cu", "fused_small32.cu", "potential.cu", "observe.cu", "adjoint.cu", "batch.cu",
+           "fused_medium32.cu", "fused_small64.cu", "fused_small32.cu", "fused_adjoint64.cu",
+           "fused_adjoint32.cu", "potential.cu", "observe.cu", "adjoint.cu", "batch.cu",
            "noalloc.cu", "rmdft.cu", "capi.cpp", "io.cpp", "xrism1d.cpp"]
 
 

@@ -152,3 +152,25 @@ def test_step_limit_of_a_mixed_solve(monkeypatch, maxstep):
     a = _solve(monkeypatch, True, 48, WATER, precision=1, convergence=1e-10, maxstep=maxstep)
     assert a[0]["status"] == 6
     assert maxstep < a[0]["iterations"] <= maxstep + 3
+
+
+@pytest.mark.parametrize("edge,xvk", [(32, WATER), (48, WATER), (64, SALT), (96, WATER), (128, SALT)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_one_launch_adjoint_matches_the_host_driven_solve(monkeypatch, edge, xvk, precision):
+    """FP64: the same Anderson steps, so equal to the solve's own tolerance
+    (1e-10); FP32: two stops within 2e-6 of the residual."""
+    import rism3d_b200 as R
+    import rism3d_b200.synth as S
+    m = S.small_chain(seed=10, natom=10)
+    xyz = m.xyz - 0.5 * (m.xyz.min(axis=0) + m.xyz.max(axis=0))
+    out = []
+    for fused in ("1", "0"):
+        monkeypatch.setenv("RISM3D_FUSED", fused)
+        s = R.Solver((edge,) * 3, (0.5 * edge,) * 3, convergence=1e-8)
+        s.set_solvent_obj(F.read_xvk(os.path.join(GOLDEN, xvk)))
+        s.set_solute(m.sig, m.eps, 0.6 * m.q, xyz)
+        s.solve()
+        out.append(s.grad(precision=precision))
+        s.close()
+    for a, b in zip(*out):
+        assert _rel(a, b) < (1e-9 if precision == 0 else 2e-5)
