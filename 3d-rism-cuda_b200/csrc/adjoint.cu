@@ -550,8 +550,7 @@ int adjoint_one_launch(Context &c, const T *G, const T *w, T *xi, T *Lxi, T *ys,
                        double *part, const StageParams *sp0, CT *buf, double eta, double tol,
                        int maxit, Scratch &S, bool &done, int &it, bool &stalled) {
   done = false;
-  const FusedPlan &f = c.fu64;
-  if (!f.on || V > 4) return RISM3D_OK;
+  if (!c.d_fused || !c.d_xs || c.nx != c.ny || c.nx != c.nz) return RISM3D_OK;   // cubic cells
   const fused::AdjointLaunch<T> launch = fused::adjoint_table<T>(c.nx, V);
   fused::AdjointArgs<T> g{};
   int clusters = 0;

@@ -35,7 +35,11 @@ struct AdjointArgs {
 // this device
 template <typename T>
 using AdjointLaunch = bool (*)(const AdjointArgs<T> &, int *clusters, cudaStream_t);
-template <typename T> AdjointLaunch<T> adjoint_table(int N, int V);   // null: no instantiation
+template <typename T> AdjointLaunch<T> adjoint_table_x(int N, int V);   // 32-72
+template <typename T> AdjointLaunch<T> adjoint_table_y(int N, int V);   // 80-128, 256
+template <typename T> AdjointLaunch<T> adjoint_table(int N, int V) {    // null: no instantiation
+  return N <= 72 ? adjoint_table_x<T>(N, V) : adjoint_table_y<T>(N, V);
+}
 
 }  // namespace fused
 }  // namespace rism3d

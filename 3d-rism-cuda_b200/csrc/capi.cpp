@@ -115,7 +115,7 @@ void free_device(Context &c) {
   if (c.d_fused) cudaFree(c.d_fused);
   c.d_fused = nullptr;
   c.d_RPx = nullptr; c.f_RPx = nullptr; c.d_scr = nullptr; c.d_roots = nullptr; c.f_roots = nullptr;
-  c.d_bar = nullptr;
+  c.d_bar = nullptr; c.d_xo = nullptr; c.d_xo32 = nullptr; c.split64 = c.split32 = false;
   c.fu64.on = c.fu32.on = false;
   if (c.plan64) cufftDestroy(c.plan64);
   if (c.plan32) cufftDestroy(c.plan32);

@@ -98,6 +98,8 @@ template <> struct Split<10> { static constexpr int A = 2; };
 template <> struct Split<12> { static constexpr int A = 3; };
 template <> struct Split<15> { static constexpr int A = 3; };
 template <> struct Split<16> { static constexpr int A = 4; };
+template <> struct Split<18> { static constexpr int A = 2; };
+template <> struct Split<20> { static constexpr int A = 4; };
 
 template <int R, bool INV, typename C> __device__ __forceinline__ void run(C (&v)[R]) {
   typedef typename std::remove_reference<decltype(v[0].x)>::type T;

@@ -41,23 +41,49 @@ namespace fused {
 
 template <typename T> using CxT = typename Cx<T>::t;
 
-// ---- shapes: N = R1 R2 with R2 even (z lines pair up registers of mirror
-// points), R1 >= R2 where possible; LB lines per batch, NC CTAs per plane
+// ---- shapes: N = R1 R2, both even (z lines pair up registers of mirror
+// points, rows move in pairs of points), R1 >= R2.  LB lines per batch of a
+// block, NC CTAs per plane, CW owner columns of a z tile.  LB and NC are
+// chosen so that the planes' CTAs fill the SMs in few, even rounds: a block is
+// 96-256 threads, of which the SM holds 512 in FP64 (128 registers).
 template <int N> struct Shape;
-template <> struct Shape<32>  { static constexpr int R1 = 8,  R2 = 4,  LB = 16, NC = 2; };
-template <> struct Shape<48>  { static constexpr int R1 = 8,  R2 = 6,  LB = 16, NC = 3; };
-template <> struct Shape<64>  { static constexpr int R1 = 8,  R2 = 8,  LB = 32, NC = 2; };
-template <> struct Shape<96>  { static constexpr int R1 = 12, R2 = 8,  LB = 16, NC = 6; };
-template <> struct Shape<128> { static constexpr int R1 = 16, R2 = 8,  LB = 16, NC = 4; };
-template <> struct Shape<256> { static constexpr int R1 = 16, R2 = 16, LB = 16, NC = 8; };
+#define RISM3D_SHAPE(N, r1, r2, lb, nc, cw) \
+  template <> struct Shape<N> { static constexpr int R1 = r1, R2 = r2, LB = lb, NC = nc, CW = cw; };
+RISM3D_SHAPE(32, 8, 4, 16, 2, 8)
+RISM3D_SHAPE(36, 6, 6, 12, 3, 6)
+RISM3D_SHAPE(40, 10, 4, 20, 2, 10)
+RISM3D_SHAPE(48, 8, 6, 16, 3, 8)
+RISM3D_SHAPE(60, 10, 6, 30, 2, 15)
+RISM3D_SHAPE(64, 8, 8, 32, 2, 16)
+RISM3D_SHAPE(72, 12, 6, 36, 2, 18)
+RISM3D_SHAPE(80, 10, 8, 16, 5, 8)
+RISM3D_SHAPE(96, 12, 8, 16, 6, 8)
+RISM3D_SHAPE(100, 10, 10, 10, 5, 5)
+RISM3D_SHAPE(108, 18, 6, 18, 3, 9)
+RISM3D_SHAPE(120, 12, 10, 10, 4, 5)
+RISM3D_SHAPE(128, 16, 8, 16, 4, 8)
+RISM3D_SHAPE(144, 12, 12, 12, 3, 6)
+RISM3D_SHAPE(160, 16, 10, 16, 5, 8)
+RISM3D_SHAPE(180, 18, 10, 15, 4, 6)
+RISM3D_SHAPE(192, 16, 12, 16, 6, 8)
+RISM3D_SHAPE(200, 20, 10, 20, 5, 10)
+RISM3D_SHAPE(216, 18, 12, 18, 6, 9)
+RISM3D_SHAPE(240, 20, 12, 15, 8, 6)
+RISM3D_SHAPE(256, 16, 16, 16, 8, 8)
+#undef RISM3D_SHAPE
 
 template <int N> struct Lines {
-  static constexpr int R1 = Shape<N>::R1, R2 = Shape<N>::R2, LB = Shape<N>::LB, NC = Shape<N>::NC;
-  static constexpr int TH = LB * R2;               // threads: one stage-1 item each
+  static constexpr int R1 = Shape<N>::R1, R2 = Shape<N>::R2, LB = Shape<N>::LB, NC = Shape<N>::NC,
+                       CW = Shape<N>::CW;
+  // threads: one stage-1 item each of a batch of lines or a z tile's columns,
+  // in whole warps
+  static constexpr int ITEMS = (LB > 2 * CW ? LB : 2 * CW) * R2, TH = (ITEMS + 31) / 32 * 32;
   static constexpr int ST = R2 | 1;                // row-exchange stride (no bank conflicts)
   static constexpr int LS = R1 * ST;               // shared points of one row
   static constexpr int SH = N / NC;                // lines per CTA
-  static_assert(R1 * R2 == N && R2 % 2 == 0 && SH % LB == 0, "line split");
+  // every thread has a line in every batch: no tests in the loops
+  static constexpr bool FULL = LB * R2 == TH && SH % LB == 0, ZFULL = 2 * CW * R2 == TH;
+  static_assert(R1 * R2 == N && R1 % 2 == 0 && R2 % 2 == 0 && R1 >= R2 && SH * NC == N, "line split");
   template <typename T> static constexpr size_t smem() { return sizeof(CxT<T>) * LB * (size_t)LS; }
   // a whole-phase launch of a small grid has one block per SM at most: all
   // registers, and all points of a thread in flight at once
@@ -122,51 +148,62 @@ template <typename T> __device__ __forceinline__ T *rp_slot(const IterArgs<T> &a
   return i < 2 ? a.RP + (size_t)i * V * a.n : a.RPx;
 }
 
-// y-DFT of columns [c0, c0 + SH) of a plane: src[y N + x] -> dst (dst may be
-// src: a column is read whole before it is written)
-template <typename T, int N, bool INV>
-__device__ __forceinline__ void columns(const CxT<T> *src, CxT<T> *dst, int c0, CxT<T> *sm,
-                                        const CxT<T> *roots) {
+// DFT along y of ncol columns of a plane: column x of src (row pitch `pitch`)
+// -> column x of dst (dst may be src: a column is read whole before it is
+// written)
+template <typename T, int N, bool INV, bool FULL>
+__device__ __forceinline__ void columns(const CxT<T> *src, CxT<T> *dst, int pitch, int ncol,
+                                        CxT<T> *sm, const CxT<T> *roots) {
   typedef CxT<T> C;
   using L = Lines<N>;
   constexpr int R1 = L::R1, R2 = L::R2, LB = L::LB;
   const int col = threadIdx.x % LB, t = threadIdx.x / LB;
 #pragma unroll 1
-  for (int cb = 0; cb < L::SH; cb += LB) {
-    const C *s0 = src + c0 + cb + col;
+  for (int cb = 0; cb < ncol; cb += LB) {
+    const bool live = FULL || (t < R2 && cb + col < ncol);
     C v[R1];
+    if (live) {
+      const C *s0 = src + cb + col;
 #pragma unroll
-    for (int j = 0; j < R1; ++j) v[j] = __ldcg(s0 + (size_t)(t + R2 * j) * N);
-    dft::run<R1, INV>(v);
+      for (int j = 0; j < R1; ++j) v[j] = __ldcg(s0 + (size_t)(t + R2 * j) * pitch);
+      dft::run<R1, INV>(v);
 #pragma unroll
-    for (int s = 1; s < R1; ++s) v[s] = dft::cmulw<INV>(v[s], roots[t * s]);
+      for (int s = 1; s < R1; ++s) v[s] = dft::cmulw<INV>(v[s], roots[t * s]);
+    }
     __syncthreads();                               // the exchange's last readers are done
+    if (live)
 #pragma unroll
-    for (int s = 0; s < R1; ++s) sm[(s * R2 + t) * LB + col] = v[s];
+      for (int s = 0; s < R1; ++s) sm[(s * R2 + t) * LB + col] = v[s];
     __syncthreads();
 #pragma unroll 1
     for (int i = threadIdx.x; i < LB * R1; i += L::TH) {
       const int c = i % LB, s = i / LB;
-      C w[R2];
+      if (FULL || cb + c < ncol) {
+        C w[R2];
 #pragma unroll
-      for (int k = 0; k < R2; ++k) w[k] = sm[(s * R2 + k) * LB + c];
-      dft::run<R2, INV>(w);
-      C *d0 = dst + c0 + cb + c;
+        for (int k = 0; k < R2; ++k) w[k] = sm[(s * R2 + k) * LB + c];
+        dft::run<R2, INV>(w);
+        C *d0 = dst + cb + c;
 #pragma unroll
-      for (int k = 0; k < R2; ++k) __stcg(d0 + (size_t)(s + R1 * k) * N, w[k]);
+        for (int k = 0; k < R2; ++k) __stcg(d0 + (size_t)(s + R1 * k) * pitch, w[k]);
+      }
     }
   }
 }
 
+// Row batches: thread threadIdx.x < LB R2 works on row threadIdx.x / R2 of its
+// batch where that row exists (live); the others only take part in the row
+// barriers.
+//
 // x-DFT of a row in its exchange slots (line[(x / R2) ST + x % R2], complete)
 // to dst; a thread's stage-1 inputs and outputs are its own slots.
 template <typename T, int N>
-__device__ __forceinline__ void rows_forward(CxT<T> *line, CxT<T> *dst, int t,
+__device__ __forceinline__ void rows_forward(CxT<T> *line, CxT<T> *dst, int t, bool live,
                                              const CxT<T> *roots) {
   typedef CxT<T> C;
   using L = Lines<N>;
   constexpr int R1 = L::R1, R2 = L::R2, ST = L::ST;
-  {
+  if (live) {
     C v[R1];
 #pragma unroll
     for (int j = 0; j < R1; ++j) v[j] = line[j * ST + t];
@@ -177,33 +214,163 @@ __device__ __forceinline__ void rows_forward(CxT<T> *line, CxT<T> *dst, int t,
     for (int s = 0; s < R1; ++s) line[s * ST + t] = v[s];
   }
   row_sync<R2>();
+  if (live) {
 #pragma unroll 1
-  for (int s = t; s < R1; s += R2) {
-    C w[R2];
+    for (int s = t; s < R1; s += R2) {
+      C w[R2];
 #pragma unroll
-    for (int k = 0; k < R2; ++k) w[k] = line[s * ST + k];
-    dft::run<R2, false>(w);
+      for (int k = 0; k < R2; ++k) w[k] = line[s * ST + k];
+      dft::run<R2, false>(w);
 #pragma unroll
-    for (int k = 0; k < R2; ++k) __stcg(dst + s + R1 * k, w[k]);
+      for (int k = 0; k < R2; ++k) __stcg(dst + s + R1 * k, w[k]);
+    }
   }
 }
 
+// Inverse x-DFT of the row src into line[(x / R2) ST + x % R2], not yet
+// twiddled; every thread of the row may read it on return.
+template <typename T, int N>
+__device__ __forceinline__ void rows_inverse(const CxT<T> *src, CxT<T> *line, int t, bool live,
+                                             const CxT<T> *roots) {
+  typedef CxT<T> C;
+  using L = Lines<N>;
+  constexpr int R1 = L::R1, R2 = L::R2, ST = L::ST, NI = (R1 + R2 - 1) / R2;
+  {
+    C v[R1];
+    if (live) {
+#pragma unroll
+      for (int j = 0; j < R1; ++j) v[j] = __ldcg(src + t + R2 * j);
+      dft::run<R1, true>(v);
+#pragma unroll
+      for (int s = 1; s < R1; ++s) v[s] = dft::cmulw<true>(v[s], roots[t * s]);
+    }
+    row_sync<R2>();                                // the exchange's last readers are done
+    if (live)
+#pragma unroll
+      for (int s = 0; s < R1; ++s) line[s * ST + t] = v[s];
+  }
+  row_sync<R2>();
+  C w[NI][R2];
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    const int s = t + R2 * i;
+    if (live && s < R1) {
+#pragma unroll
+      for (int k = 0; k < R2; ++k) w[i][k] = line[s * ST + k];
+      dft::run<R2, true>(w[i]);
+    }
+  }
+  row_sync<R2>();
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    const int s = t + R2 * i;
+    if (live && s < R1) {
+#pragma unroll
+      for (int k = 0; k < R2; ++k) {
+        const int x = s + R1 * k;
+        line[(x / R2) * ST + x % R2] = w[i][k];
+      }
+    }
+  }
+  row_sync<R2>();
+}
+
 // ---------------------------------------------------------------- plane A
+// One row of a batch: the update of the last cycle, closure, packed and
+// twiddled, then its x-DFT to dst.
+template <typename T, int N, int V, bool REF, bool WIDE>
+__device__ __forceinline__ void update_row(const IterArgs<T> &a, const DevState *st, CxT<T> *line,
+                                           int t, bool live, bool two, size_t base, CxT<T> tyz,
+                                           int dyz, CxT<T> *dst, const CxT<T> *tw,
+                                           const CxT<T> *roots, bool hnc) {
+  typedef CxT<T> C;
+  using L = Lines<N>;
+  constexpr int R1 = L::R1, R2 = L::R2, ST = L::ST;
+  using W = Vecs<T, R1, WIDE>;
+  constexpr int VW = W::VW, NV = W::NV;
+  const int mode = st->mode, slot = st->upd_slot;
+  const T s1 = (T)st->s1, s2 = (T)st->s2, m = (T)st->m;
+  const size_t n = (size_t)a.n;
+  row_sync<R2>();                                  // the exchange's last readers are done
+  if (live) {
+    T *pt = a.t + base, *py = a.Y + (size_t)slot * V * n + base;
+    const T *pu = a.U + base, *pr = rp_slot(a, V, st->rp[slot]) + base,   // this cycle's residual
+            *p0 = a.Y + base, *p1 = a.Y + (size_t)V * n + base;
+#pragma unroll 1
+    for (int c = 0; c < W::CH; ++c) {
+      T tv[2][NV][VW], uv[2][NV][VW];
+      int x0[NV];
+#pragma unroll
+      for (int q = 0; q < NV; ++q) {
+        x0[q] = VW * (t + R2 * (q + NV * c));
+        ldv(tv[0][q], pt + x0[q]);
+        ldv(uv[0][q], pu + x0[q]);
+        if (two) {
+          ldv(tv[1][q], pt + n + x0[q]);
+          ldv(uv[1][q], pu + n + x0[q]);
+        }
+      }
+      if (mode != 0) {
+        T rv[2][NV][VW], y0[2][NV][VW], y1[2][NV][VW];
+#pragma unroll
+        for (int q = 0; q < NV; ++q)
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            if (b && !two) break;
+            ldv(rv[b][q], pr + b * n + x0[q]);
+            ldv(y0[b][q], p0 + b * n + x0[q]);
+            ldv(y1[b][q], p1 + b * n + x0[q]);
+          }
+#pragma unroll
+        for (int q = 0; q < NV; ++q)
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            if (b && !two) break;
+            T yw[VW];
+#pragma unroll
+            for (int k = 0; k < VW; ++k) {
+              // newdt (AN2), anderson_cuda.cu:11-23, or newdt0 (Picard)
+              const T tt = tv[b][q][k], r = rv[b][q][k], yy = tt + m * r;
+              yw[k] = yy;
+              tv[b][q][k] = mode == 2 ? yy + s1 * (y0[b][q][k] - yy) + s2 * (y1[b][q][k] - yy)
+                                      : tt + r;
+            }
+            stv(py + b * n + x0[q], yw);
+            stv(pt + b * n + x0[q], tv[b][q]);
+          }
+      }
+      // closure + c_SR (calculate_cuda.cu:1-29) and the forward pre-twiddle
+      // (timekf, fft3d.cu:41-49): dir * dkf * (c_a + i c_b)
+#pragma unroll
+      for (int q = 0; q < NV; ++q)
+#pragma unroll
+        for (int k = 0; k < VW; ++k) {
+          const int x = x0[q] + k;
+          C cc;
+          cc.x = cfun_rt<REF>(tv[0][q][k], uv[0][q][k], hnc);
+          cc.y = two ? cfun_rt<REF>(tv[1][q][k], uv[1][q][k], hnc) : T(0);
+          const C kf = cmul(tw[x], tyz);
+          const T dir = ((x & 1) ^ dyz) ? T(-1) : T(1);
+          C w;
+          w.x = kf.x * dir;
+          w.y = kf.y * dir;
+          line[(x / R2) * ST + x % R2] = cmul(cc, w);
+        }
+    }
+  }
+  row_sync<R2>();
+  rows_forward<T, N>(line, dst, t, live, roots);
+}
+
 template <typename T, int N, int V, bool REF, bool WIDE>
 __device__ __forceinline__ void planes_a(const IterArgs<T> &a, const DevState *st, CxT<T> *sm,
                                          const CxT<T> *tw, const CxT<T> *roots, bool hnc) {
   typedef CxT<T> C;
   using L = Lines<N>;
-  constexpr int R1 = L::R1, R2 = L::R2, LB = L::LB, ST = L::ST, LS = L::LS;
-  using W = Vecs<T, R1, WIDE>;
-  constexpr int P = (V + 1) / 2, VW = W::VW, NV = W::NV;
-  const int mode = st->mode, slot = st->upd_slot;
-  const T s1 = (T)st->s1, s2 = (T)st->s2, m = (T)st->m;
-  const T *Rn = rp_slot(a, V, st->rp[slot]);       // this cycle's residual
-  const long long n = a.n;
+  constexpr int R2 = L::R2, LB = L::LB, P = (V + 1) / 2;
+  const size_t n = (size_t)a.n;
   const int rank = blockIdx.x % L::NC, ncl = gridDim.x / L::NC;
   const int row_l = threadIdx.x / R2, t = threadIdx.x % R2;
-  C *line = sm + row_l * LS;
   for (int plane = blockIdx.x / L::NC; plane < N * P; plane += ncl) {
     const int p = plane / N, z = plane % N;
     const bool two = V % 2 == 0 || 2 * p + 1 < V;
@@ -211,79 +378,16 @@ __device__ __forceinline__ void planes_a(const IterArgs<T> &a, const DevState *s
     __syncthreads();                               // the columns' exchange is free
 #pragma unroll 1
     for (int rb = 0; rb < L::SH; rb += LB) {
-      const int y = rank * L::SH + rb + row_l;
-      const size_t base = (size_t)(2 * p) * n + ((size_t)z * N + y) * N;
-      T *pt = a.t + base, *py = a.Y + (size_t)slot * V * n + base;
-      const T *pu = a.U + base, *pr = Rn + base, *p0 = a.Y + base, *p1 = a.Y + (size_t)V * n + base;
-      const C tyz = cmul(tw[N + y], tw[2 * N + z]);
-      const int dyz = (y + z) & 1;
-      row_sync<R2>();                              // the exchange's last readers are done
-#pragma unroll 1
-      for (int c = 0; c < W::CH; ++c) {
-        T tv[2][NV][VW], uv[2][NV][VW];
-        int x0[NV];
-#pragma unroll
-        for (int q = 0; q < NV; ++q) {
-          x0[q] = VW * (t + R2 * (q + NV * c));
-          ldv(tv[0][q], pt + x0[q]);
-          ldv(uv[0][q], pu + x0[q]);
-          if (two) {
-            ldv(tv[1][q], pt + n + x0[q]);
-            ldv(uv[1][q], pu + n + x0[q]);
-          }
-        }
-        if (mode != 0) {
-          T rv[2][NV][VW], y0[2][NV][VW], y1[2][NV][VW];
-#pragma unroll
-          for (int q = 0; q < NV; ++q)
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-              if (b && !two) break;
-              ldv(rv[b][q], pr + b * n + x0[q]);
-              ldv(y0[b][q], p0 + b * n + x0[q]);
-              ldv(y1[b][q], p1 + b * n + x0[q]);
-            }
-#pragma unroll
-          for (int q = 0; q < NV; ++q)
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-              if (b && !two) break;
-              T yw[VW];
-#pragma unroll
-              for (int k = 0; k < VW; ++k) {
-                // newdt (AN2), anderson_cuda.cu:11-23, or newdt0 (Picard)
-                const T tt = tv[b][q][k], r = rv[b][q][k], yy = tt + m * r;
-                yw[k] = yy;
-                tv[b][q][k] = mode == 2 ? yy + s1 * (y0[b][q][k] - yy) + s2 * (y1[b][q][k] - yy)
-                                        : tt + r;
-              }
-              stv(py + b * n + x0[q], yw);
-              stv(pt + b * n + x0[q], tv[b][q]);
-            }
-        }
-        // closure + c_SR (calculate_cuda.cu:1-29) and the forward pre-twiddle
-        // (timekf, fft3d.cu:41-49): dir * dkf * (c_a + i c_b)
-#pragma unroll
-        for (int q = 0; q < NV; ++q)
-#pragma unroll
-          for (int k = 0; k < VW; ++k) {
-            const int x = x0[q] + k;
-            C cc;
-            cc.x = cfun_rt<REF>(tv[0][q][k], uv[0][q][k], hnc);
-            cc.y = two ? cfun_rt<REF>(tv[1][q][k], uv[1][q][k], hnc) : T(0);
-            const C kf = cmul(tw[x], tyz);
-            const T dir = ((x & 1) ^ dyz) ? T(-1) : T(1);
-            C w;
-            w.x = kf.x * dir;
-            w.y = kf.y * dir;
-            line[(x / R2) * ST + x % R2] = cmul(cc, w);
-          }
-      }
-      row_sync<R2>();
-      rows_forward<T, N>(line, pb + (size_t)y * N, t, roots);
+      const bool live = L::FULL || (row_l < LB && rb + row_l < L::SH);
+      const int y = rank * L::SH + (live ? rb + row_l : 0);
+      update_row<T, N, V, REF, WIDE>(a, st, sm + row_l * L::LS, t, live, two,
+                                     (size_t)(2 * p) * n + ((size_t)z * N + y) * N,
+                                     cmul(tw[N + y], tw[2 * N + z]), (y + z) & 1,
+                                     pb + (size_t)y * N, tw, roots, hnc);
     }
     plane_sync<L::NC>();                           // every row of the plane is in L2
-    columns<T, N, false>(pb, pb, rank * L::SH, sm, roots);
+    C *pc = pb + rank * L::SH;
+    columns<T, N, false, L::FULL>(pc, pc, N, L::SH, sm, roots);
   }
 }
 
@@ -297,146 +401,85 @@ __global__ void __launch_bounds__(Lines<N>::TH, (Lines<N>::template minb<T>()))
 }
 
 // ---------------------------------------------------------------- plane R
-// Inverse row DFT of LB rows of the half-transformed plane: row (relative to
-// src) threadIdx.x / R2, the result in line[(x / R2) ST + x % R2], not yet
-// twiddled.
-template <typename T, int N>
-__device__ __forceinline__ void rows_inverse(const CxT<T> *src, CxT<T> *line, int t,
-                                             const CxT<T> *roots) {
+// The points of one row after the inverse transform (line, not yet twiddled;
+// sites v0 and v0 + 1): residuals, their sums, the new residual slot.
+template <typename T, int N, int V, bool REF, bool WIDE>
+__device__ __forceinline__ void residual_row(const IterArgs<T> &a, const DevState *st,
+                                             const CxT<T> *line, int t, bool two, int v0,
+                                             size_t base, CxT<T> tyz, int dyz, const CxT<T> *tw,
+                                             bool gram, bool hnc, double (&acc)[6]) {
   typedef CxT<T> C;
   using L = Lines<N>;
-  constexpr int R1 = L::R1, R2 = L::R2, ST = L::ST, NI = (R1 + R2 - 1) / R2;
-  {
-    C v[R1];
+  constexpr int R1 = L::R1, R2 = L::R2, ST = L::ST;
+  using W = Vecs<T, R1, WIDE>;
+  constexpr int VW = W::VW, NV = W::NV;
+  const size_t n = (size_t)a.n;
+  const T invvol = (T)a.invvol;
+  const T *pt = a.t + base, *pu = a.U + base, *p0 = rp_slot(a, V, st->rp[0]) + base,
+          *p1 = rp_slot(a, V, st->rp[1]) + base, *pq = REF ? a.R0 + base : nullptr;
+  T *pr = rp_slot(a, V, st->rp[2]) + base;
+#pragma unroll 1
+  for (int c = 0; c < W::CH; ++c) {
+    T tv[2][NV][VW], uv[2][NV][VW], r0[2][NV][VW], r1[2][NV][VW], qv[2][NV][VW];
+    int x0[NV];
 #pragma unroll
-    for (int j = 0; j < R1; ++j) v[j] = __ldcg(src + t + R2 * j);
-    dft::run<R1, true>(v);
+    for (int q = 0; q < NV; ++q) {
+      x0[q] = VW * (t + R2 * (q + NV * c));
 #pragma unroll
-    for (int s = 1; s < R1; ++s) v[s] = dft::cmulw<true>(v[s], roots[t * s]);
-    row_sync<R2>();                                // the exchange's last readers are done
-#pragma unroll
-    for (int s = 0; s < R1; ++s) line[s * ST + t] = v[s];
-  }
-  row_sync<R2>();
-  C w[NI][R2];
-#pragma unroll
-  for (int i = 0; i < NI; ++i) {
-    const int s = t + R2 * i;
-    if (s < R1) {
-#pragma unroll
-      for (int k = 0; k < R2; ++k) w[i][k] = line[s * ST + k];
-      dft::run<R2, true>(w[i]);
+      for (int b = 0; b < 2; ++b) {
+        if (b && !two) break;
+        ldv(tv[b][q], pt + b * n + x0[q]);
+        ldv(uv[b][q], pu + b * n + x0[q]);
+        ldv(r0[b][q], p0 + b * n + x0[q]);
+        ldv(r1[b][q], p1 + b * n + x0[q]);
+        if (REF) ldv(qv[b][q], pq + b * n + x0[q]);
+      }
     }
-  }
-  row_sync<R2>();
 #pragma unroll
-  for (int i = 0; i < NI; ++i) {
-    const int s = t + R2 * i;
-    if (s < R1) {
+    for (int q = 0; q < NV; ++q) {
+      T rw[2][VW];
 #pragma unroll
-      for (int k = 0; k < R2; ++k) {
-        const int x = s + R1 * k;
-        line[(x / R2) * ST + x % R2] = w[i][k];
+      for (int k = 0; k < VW; ++k) {
+        const int x = x0[q] + k;
+        // inverse post-twiddle (timekb, fft3d.cu:52-60): (1/V) dir conj(dkf)
+        const C kf = cmul(tw[x], tyz);
+        const T sc = invvol * (((x & 1) ^ dyz) ? T(-1) : T(1));
+        C w;
+        w.x = kf.x * sc;
+        w.y = -kf.y * sc;
+        const C h = cmul(line[(x / R2) * ST + x % R2], w);
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          if (b && !two) break;
+          const T R = residual_rt<REF>(b ? h.y : h.x, tv[b][q][k], uv[b][q][k],
+                                       REF ? qv[b][q][k] : T(0), hnc);
+          rw[b][k] = R;
+          const double r = (double)R;
+          acc[0] += r * r;                     // cal_rms.cu:18
+          if (gram) {                          // theta30, anderson_cuda.cu:33-39
+            const double wt = a.sp->irho[v0 + b];
+            const double d0 = r - (double)r0[b][q][k], d1 = r - (double)r1[b][q][k];
+            acc[1] += wt * r * d0;
+            acc[2] += wt * r * d1;
+            acc[3] += wt * d0 * d0;
+            acc[4] += wt * d0 * d1;
+            acc[5] += wt * d1 * d1;
+          }
+        }
+      }
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        if (b && !two) break;
+        stv(pr + b * n + x0[q], rw[b]);
       }
     }
   }
-  row_sync<R2>();
 }
 
-template <typename T, int N, int V, bool REF, bool WIDE>
-__device__ __forceinline__ void planes_r(const IterArgs<T> &a, const DevState *st, CxT<T> *sm,
-                                         const CxT<T> *tw, const CxT<T> *roots, bool hnc) {
-  typedef CxT<T> C;
-  using L = Lines<N>;
-  constexpr int R1 = L::R1, R2 = L::R2, LB = L::LB, ST = L::ST, LS = L::LS, TH = L::TH;
-  using W = Vecs<T, R1, WIDE>;
-  constexpr int P = (V + 1) / 2, VW = W::VW, NV = W::NV;
-  __shared__ double red[(TH + 31) / 32][6];
-  const bool gram = st->count <= 0;
-  const long long n = a.n;
-  const T *RP0 = rp_slot(a, V, st->rp[0]), *RP1 = rp_slot(a, V, st->rp[1]);
-  T *Rn = rp_slot(a, V, st->rp[2]);
-  const int rank = blockIdx.x % L::NC, cl = blockIdx.x / L::NC, ncl = gridDim.x / L::NC;
-  const int row_l = threadIdx.x / R2, t = threadIdx.x % R2;
-  C *line = sm + row_l * LS;
-  C *scr = a.scr + (size_t)cl * N * N;
-  const T invvol = (T)a.invvol;
-  double acc[6] = {0, 0, 0, 0, 0, 0};
-  for (int plane = cl; plane < N * P; plane += ncl) {
-    const int p = plane / N, z = plane % N;
-    const bool two = V % 2 == 0 || 2 * p + 1 < V;
-    columns<T, N, true>(a.buf + (size_t)plane * N * N, scr, rank * L::SH, sm, roots);
-    __syncthreads();                               // the columns' exchange is free
-    plane_sync<L::NC>();                           // every column of the plane is in L2
-#pragma unroll 1
-    for (int rb = 0; rb < L::SH; rb += LB) {
-      const int y = rank * L::SH + rb + row_l;
-      rows_inverse<T, N>(scr + (size_t)y * N, line, t, roots);
-      const size_t base = (size_t)(2 * p) * n + ((size_t)z * N + y) * N;
-      const T *pt = a.t + base, *pu = a.U + base, *p0 = RP0 + base, *p1 = RP1 + base,
-              *pq = REF ? a.R0 + base : nullptr;
-      T *pr = Rn + base;
-      const C tyz = cmul(tw[N + y], tw[2 * N + z]);
-      const int dyz = (y + z) & 1;
-#pragma unroll 1
-      for (int c = 0; c < W::CH; ++c) {
-        T tv[2][NV][VW], uv[2][NV][VW], r0[2][NV][VW], r1[2][NV][VW], qv[2][NV][VW];
-        int x0[NV];
-#pragma unroll
-        for (int q = 0; q < NV; ++q) {
-          x0[q] = VW * (t + R2 * (q + NV * c));
-#pragma unroll
-          for (int b = 0; b < 2; ++b) {
-            if (b && !two) break;
-            ldv(tv[b][q], pt + b * n + x0[q]);
-            ldv(uv[b][q], pu + b * n + x0[q]);
-            ldv(r0[b][q], p0 + b * n + x0[q]);
-            ldv(r1[b][q], p1 + b * n + x0[q]);
-            if (REF) ldv(qv[b][q], pq + b * n + x0[q]);
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < NV; ++q) {
-          T rw[2][VW];
-#pragma unroll
-          for (int k = 0; k < VW; ++k) {
-            const int x = x0[q] + k;
-            // inverse post-twiddle (timekb, fft3d.cu:52-60): (1/V) dir conj(dkf)
-            const C kf = cmul(tw[x], tyz);
-            const T sc = invvol * (((x & 1) ^ dyz) ? T(-1) : T(1));
-            C w;
-            w.x = kf.x * sc;
-            w.y = -kf.y * sc;
-            const C h = cmul(line[(x / R2) * ST + x % R2], w);
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-              if (b && !two) break;
-              const T R = residual_rt<REF>(b ? h.y : h.x, tv[b][q][k], uv[b][q][k],
-                                           REF ? qv[b][q][k] : T(0), hnc);
-              rw[b][k] = R;
-              const double r = (double)R;
-              acc[0] += r * r;                     // cal_rms.cu:18
-              if (gram) {                          // theta30, anderson_cuda.cu:33-39
-                const double wt = a.sp->irho[2 * p + b];
-                const double d0 = r - (double)r0[b][q][k], d1 = r - (double)r1[b][q][k];
-                acc[1] += wt * r * d0;
-                acc[2] += wt * r * d1;
-                acc[3] += wt * d0 * d0;
-                acc[4] += wt * d0 * d1;
-                acc[5] += wt * d1 * d1;
-              }
-            }
-          }
-#pragma unroll
-          for (int b = 0; b < 2; ++b) {
-            if (b && !two) break;
-            stv(pr + b * n + x0[q], rw[b]);
-          }
-        }
-      }
-    }
-    if (plane + ncl < N * P) plane_sync<L::NC>();  // the scratch plane is free again
-  }
+// Block sums of R^2 and the Gram terms into this block's row of the partials
+template <int TH>
+__device__ __forceinline__ void block_sums(double (&acc)[6], double *part) {
+  __shared__ double red[TH / 32][6];
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
     double v = acc[k];
@@ -450,7 +493,62 @@ __device__ __forceinline__ void planes_r(const IterArgs<T> &a, const DevState *s
   if (threadIdx.x < 6) {
     double s = 0.0;
     for (int w = 0; w < TH / 32; ++w) s += red[w][threadIdx.x];
-    a.part[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = s;
+    part[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = s;
+  }
+}
+
+template <typename T, int N, int V, bool REF, bool WIDE>
+__device__ __forceinline__ void planes_r(const IterArgs<T> &a, const DevState *st, CxT<T> *sm,
+                                         const CxT<T> *tw, const CxT<T> *roots, bool hnc) {
+  typedef CxT<T> C;
+  using L = Lines<N>;
+  constexpr int R2 = L::R2, LB = L::LB, P = (V + 1) / 2;
+  const bool gram = st->count <= 0;
+  const size_t n = (size_t)a.n;
+  const int rank = blockIdx.x % L::NC, cl = blockIdx.x / L::NC, ncl = gridDim.x / L::NC;
+  const int row_l = threadIdx.x / R2, t = threadIdx.x % R2;
+  C *line = sm + row_l * L::LS;
+  C *scr = a.scr + (size_t)cl * N * N;
+  double acc[6] = {0, 0, 0, 0, 0, 0};
+  for (int plane = cl; plane < N * P; plane += ncl) {
+    const int p = plane / N, z = plane % N;
+    const bool two = V % 2 == 0 || 2 * p + 1 < V;
+    columns<T, N, true, L::FULL>(a.buf + (size_t)plane * N * N + rank * L::SH, scr + rank * L::SH, N, L::SH,
+                        sm, roots);
+    __syncthreads();                               // the columns' exchange is free
+    plane_sync<L::NC>();                           // every column of the plane is in L2
+#pragma unroll 1
+    for (int rb = 0; rb < L::SH; rb += LB) {
+      const bool live = L::FULL || (row_l < LB && rb + row_l < L::SH);
+      const int y = rank * L::SH + (live ? rb + row_l : 0);
+      rows_inverse<T, N>(scr + (size_t)y * N, line, t, live, roots);
+      if (live)
+        residual_row<T, N, V, REF, WIDE>(a, st, line, t, two, 2 * p,
+                                         (size_t)(2 * p) * n + ((size_t)z * N + y) * N,
+                                         cmul(tw[N + y], tw[2 * N + z]), (y + z) & 1, tw, gram,
+                                         hnc, acc);
+    }
+    if (plane + ncl < N * P) plane_sync<L::NC>();  // the scratch plane is free again
+  }
+  block_sums<L::TH>(acc, a.part);
+}
+
+// The last block of a solute to finish reduces all block sums and steers the
+// loop.
+template <typename T>
+__device__ __forceinline__ void finish_cycle(const IterArgs<T> &a0, const IterArgs<T> &a, int V) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(a.count, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  finalize_block(a.st, a.part, gridDim.x, (double)a.n * V, a.hist, a.hist_cap);
+  if (threadIdx.x == 0) {
+    *a.count = 0u;
+    if (a.st->done) a.st->after_done = 1;          // nothing is left to do in the loop
+    loop_test_all(a0);
   }
 }
 
@@ -458,7 +556,6 @@ template <typename T, int N, int V, bool REF>
 __global__ void __launch_bounds__(Lines<N>::TH, (Lines<N>::template minb<T>()))
     k_plane_r(IterArgs<T> a0, bool hnc) {
   extern __shared__ __align__(16) unsigned char fused_sm[];
-  __shared__ bool last;
   const IterArgs<T> a = solute_view<T, V>(a0);
   DevState *st = a.st;
   if (st->done) {                                  // this solute has stopped
@@ -466,97 +563,95 @@ __global__ void __launch_bounds__(Lines<N>::TH, (Lines<N>::template minb<T>()))
     return;
   }
   planes_r<T, N, V, REF, false>(a, st, reinterpret_cast<CxT<T> *>(fused_sm), a.tw, a.roots, hnc);
-  // the last block to finish reduces all block sums and steers the loop
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(a.count, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  finalize_block(st, a.part, gridDim.x, (double)a.n * V, a.hist, a.hist_cap);
-  if (threadIdx.x == 0) {
-    *a.count = 0u;
-    if (st->done) st->after_done = 1;              // nothing is left to do in the loop
-    loop_test_all(a0);
-  }
+  finish_cycle(a0, a, V);
 }
 
 // Once after the loop: snapshot of h (Re of the last OZ) and g (closure of
 // the t used in that cycle), and when maxstep ended the loop the pending
 // update (iterate.cu:61 runs before the step bound is tested).
 template <typename T, int N, int V, bool REF>
+__device__ __forceinline__ void final_row(const IterArgs<T> &a, const CxT<T> *line, int t, int p,
+                                          size_t row, CxT<T> tyz, int dyz, bool snap, bool update,
+                                          bool hnc) {
+  typedef CxT<T> C;
+  constexpr int R2 = Lines<N>::R2, ST = Lines<N>::ST;
+  const DevState *st = a.st;
+  const int mode = st->mode, slot = st->upd_slot;
+  const T s1 = (T)st->s1, s2 = (T)st->s2, m = (T)st->m;
+  const T *Rn = rp_slot(a, V, st->rp[slot]);       // renamed into the history already
+  const size_t n = (size_t)a.n;
+#pragma unroll 1
+  for (int x = t; x < N; x += R2) {
+    const C kf = cmul(a.tw[x], tyz);
+    const T sc = (T)a.invvol * (((x & 1) ^ dyz) ? T(-1) : T(1));
+    C w;
+    w.x = kf.x * sc;
+    w.y = -kf.y * sc;
+    const C h = cmul(line[(x / R2) * ST + x % R2], w);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      if (2 * p + q >= V) break;
+      const size_t iv = (size_t)(2 * p + q) * n + row + x;
+      const T tv = a.t[iv];
+      if (snap) {
+        a.hout[iv] = (double)(q ? h.y : h.x);
+        a.gout[iv] = (double)closure_rt(tv - a.U[iv], hnc);
+      }
+      if (update) {
+        const T R = Rn[iv], yv = tv + m * R;
+        T tn = tv + R;
+        if (mode == 2) tn = yv + s1 * (a.Y[iv] - yv) + s2 * (a.Y[(size_t)V * n + iv] - yv);
+        a.Y[(size_t)slot * V * n + iv] = yv;
+        a.t[iv] = tn;
+      }
+    }
+  }
+}
+
+template <typename T, int N, int V, bool REF>
 __global__ void __launch_bounds__(Lines<N>::TH) k_plane_final(IterArgs<T> a0, bool hnc) {
   typedef CxT<T> C;
   using L = Lines<N>;
-  constexpr int R2 = L::R2, LB = L::LB, ST = L::ST, LS = L::LS;
-  constexpr int P = (V + 1) / 2;
+  constexpr int R2 = L::R2, LB = L::LB, P = (V + 1) / 2;
   extern __shared__ __align__(16) unsigned char fused_sm[];
   C *sm = reinterpret_cast<C *>(fused_sm);
   const IterArgs<T> a = solute_view<T, V>(a0);
-  const DevState *st = a.st;
-  const int done = st->done, mode = st->mode, slot = st->upd_slot;
-  const bool snap = !REF && a.hout, update = done == 3 && mode != 0;
+  const bool snap = !REF && a.hout, update = a.st->done == 3 && a.st->mode != 0;
   if (!snap && !update) return;
-  const T s1 = (T)st->s1, s2 = (T)st->s2, m = (T)st->m;
-  const T *Rn = rp_slot(a, V, st->rp[slot]);       // renamed into the history already
-  const long long n = a.n;
   const int rank = blockIdx.x % L::NC, cl = blockIdx.x / L::NC, ncl = gridDim.x / L::NC;
   const int row_l = threadIdx.x / R2, t = threadIdx.x % R2;
-  C *line = sm + row_l * LS;
+  C *line = sm + row_l * L::LS;
   C *scr = a.scr + (size_t)cl * N * N;
   for (int plane = cl; plane < N * P; plane += ncl) {
     const int p = plane / N, z = plane % N;
-    columns<T, N, true>(a.buf + (size_t)plane * N * N, scr, rank * L::SH, sm, a.roots);
+    columns<T, N, true, L::FULL>(a.buf + (size_t)plane * N * N + rank * L::SH, scr + rank * L::SH, N, L::SH,
+                        sm, a.roots);
     __syncthreads();
     plane_sync<L::NC>();
 #pragma unroll 1
     for (int rb = 0; rb < L::SH; rb += LB) {
-      const int y = rank * L::SH + rb + row_l;
-      rows_inverse<T, N>(scr + (size_t)y * N, line, t, a.roots);
-      const C tyz = cmul(a.tw[N + y], a.tw[2 * N + z]);
-#pragma unroll 1
-      for (int x = t; x < N; x += R2) {
-        const C kf = cmul(a.tw[x], tyz);
-        const T sc = (T)a.invvol * (((x + y + z) & 1) ? T(-1) : T(1));
-        C w;
-        w.x = kf.x * sc;
-        w.y = -kf.y * sc;
-        const C h = cmul(line[(x / R2) * ST + x % R2], w);
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          if (2 * p + q >= V) break;
-          const size_t iv = (size_t)(2 * p + q) * n + ((size_t)z * N + y) * N + x;
-          const T tv = a.t[iv];
-          if (snap) {
-            a.hout[iv] = (double)(q ? h.y : h.x);
-            a.gout[iv] = (double)closure_rt(tv - a.U[iv], hnc);
-          }
-          if (update) {
-            const T R = Rn[iv], yv = tv + m * R;
-            T tn = tv + R;
-            if (mode == 2) tn = yv + s1 * (a.Y[iv] - yv) + s2 * (a.Y[(size_t)V * n + iv] - yv);
-            a.Y[(size_t)slot * V * n + iv] = yv;
-            a.t[iv] = tn;
-          }
-        }
-      }
+      const bool live = L::FULL || (row_l < LB && rb + row_l < L::SH);
+      const int y = rank * L::SH + (live ? rb + row_l : 0);
+      rows_inverse<T, N>(scr + (size_t)y * N, line, t, live, a.roots);
+      if (live)
+        final_row<T, N, V, REF>(a, line, t, p, ((size_t)z * N + y) * N,
+                                cmul(a.tw[N + y], a.tw[2 * N + z]), (y + z) & 1, snap, update, hnc);
     }
     if (plane + ncl < N * P) plane_sync<L::NC>();
   }
 }
 
 // ---------------------------------------------------------------- z lines
-// A block owns CW neighbouring kx columns at one ky < N/2 and their mirrors
-// (kx' = N-1-kx, ky' = N-1-ky), so every k and -k meet in it.  After the
+// A block owns CW neighbouring kx columns at one ky < ny/2 and their mirrors
+// (kx' = nx-1-kx, ky' = ny-1-ky), so every k and -k meet in it.  After the
 // forward DFT the owner's points kz = s + R1 k of one thread mirror the
 // points of the neighbouring lane's group R1-1-s, register R2-1-k: each lane
 // takes half of the pairs with one shuffle each way.
 template <typename T, int N, int V>
 struct ZShape {
-  // as many columns as a plane batch has lines: one block size for all kernels
-  static constexpr int COLS = Lines<N>::LB, CW = COLS / 2, TH = Lines<N>::TH;
+  static constexpr int CW = Lines<N>::CW, COLS = 2 * CW, TH = Lines<N>::TH;
   static constexpr int P = (V + 1) / 2;
-  static constexpr int TILES = (N / CW) * (N / 2);
+  static constexpr int TILES = ((N + CW - 1) / CW) * (N / 2);      // of a cubic cell
   static constexpr int MINB = (sizeof(T) == 8 ? 512 : 1024) / TH > 0 ? (sizeof(T) == 8 ? 512 : 1024) / TH : 1;
   static constexpr size_t smem() { return sizeof(CxT<T>) * (size_t)P * COLS * N; }
 };
@@ -568,15 +663,17 @@ __device__ __forceinline__ C shfl_pair(unsigned mask, C v) {
   return v;
 }
 
-template <typename T, int N, int V, bool WIDE>
+// N = nz; CUBIC: nx = ny = N and chi from the per-|k|^2 table, else the octant
+// table; a tile past the last column repeats it for its spare columns' loads.
+template <typename T, int N, int V, bool WIDE, bool CUBIC>
 __device__ __forceinline__ void zline_tile(const IterArgs<T> &a, CxT<T> *sm, const CxT<T> *roots,
-                                           int tile) {
+                                           int nx, int ny, int tile) {
   typedef CxT<T> C;
   using Z = ZShape<T, N, V>;
   constexpr int R1 = Shape<N>::R1, R2 = Shape<N>::R2, CW = Z::CW, COLS = Z::COLS, P = Z::P;
-  static_assert(N % CW == 0 && Z::TH % 32 == 0, "z tiles");
-  const long long n = a.n;
-  const int ky = tile / (N / CW), x0 = (tile % (N / CW)) * CW;
+  static_assert(!CUBIC || N % CW == 0, "z tiles");
+  const long long n = a.n, plane = (long long)nx * ny;
+  const int tx = (nx + CW - 1) / CW, ky = tile / tx, x0 = (tile % tx) * CW;
   // fk and chi of an item's pairs: loaded ahead of the exchange where they fit
   // in registers, else asked into L2 now
   constexpr int H = R2 / 2;
@@ -589,33 +686,36 @@ __device__ __forceinline__ void zline_tile(const IterArgs<T> &a, CxT<T> *sm, con
   };
   auto load_pair = [&](int i, int k, double2 &fk, T (&x)[V * V]) {
     // beta fk is stored for kz < N/2, the conjugate of the mirror's beyond
-    const int kx = x0 + (i >> 1) % CW, kz = pair_kz(i, k);
+    const int kx = CUBIC ? x0 + (i >> 1) % CW : min(x0 + (i >> 1) % CW, nx - 1), kz = pair_kz(i, k);
     fk = make_double2(0.0, 0.0);
     if (!a.nofk) {
       const bool lo = kz < N / 2;
-      const long long j = kx + (long long)N * (ky + (long long)N * kz);
+      const long long j = kx + (long long)nx * ky + plane * kz;
       fk = __ldg(a.fkh + (lo ? j : n - 1 - j));
       if (!lo) fk.y = -fk.y;
     }
-    chi_cubic<T, V>(a, kx, ky, kz, x);
+    if constexpr (CUBIC) chi_cubic<T, V>(a, kx, ky, kz, x);
+    else chi_octant<T, V>(a, kx, ky, kz, x);
   };
   if constexpr (!AHEAD) {
     if (!a.nofk)                                   // rows of CW points and their mirrors
       for (int i = threadIdx.x; i < N; i += Z::TH) {
         const int kz = i % (N / 2);
-        pf(a.fkh + (i < N / 2 ? x0 + (long long)N * (ky + (long long)N * kz)
-                              : N - x0 - CW + (long long)N * (N - 1 - ky + (long long)N * kz)));
+        pf(a.fkh + plane * kz +
+           (i < N / 2 ? x0 + (long long)nx * ky
+                      : max(nx - x0 - CW, 0) + (long long)nx * (ny - 1 - ky)));
       }
   }
-  {
-    const int col = threadIdx.x % COLS, t = threadIdx.x / COLS;
-    const C *g = a.buf + (col < CW ? (size_t)ky * N + x0 + col
-                                   : (size_t)(N - 1 - ky) * N + (N - x0 - 2 * CW) + col);
+  const int col = threadIdx.x % COLS, t = threadIdx.x / COLS;
+  const int cx = x0 + (col < CW ? col : COLS - 1 - col);           // its owner column
+  const bool live = (Lines<N>::ZFULL || t < R2) && (CUBIC || cx < nx);
+  C *g = a.buf + (col < CW ? (size_t)ky * nx + cx : (size_t)(ny - 1 - ky) * nx + nx - 1 - cx);
+  if (live) {
 #pragma unroll
     for (int p = 0; p < P; ++p) {
       C v[R1];
 #pragma unroll
-      for (int j = 0; j < R1; ++j) v[j] = __ldcg(g + (size_t)p * n + (size_t)(t + R2 * j) * N * N);
+      for (int j = 0; j < R1; ++j) v[j] = __ldcg(g + (size_t)p * n + (size_t)(t + R2 * j) * plane);
       dft::run<R1, false>(v);
 #pragma unroll
       for (int s = 1; s < R1; ++s) v[s] = cmul(v[s], roots[t * s]);
@@ -635,12 +735,12 @@ __device__ __forceinline__ void zline_tile(const IterArgs<T> &a, CxT<T> *sm, con
     const unsigned mask = __ballot_sync(0xffffffffu, act);
     if (!act) continue;
     const int side = i & 1, o = (i >> 1) % CW, s = (i >> 1) / CW;
-    const int grp = side ? R1 - 1 - s : s, col = side ? COLS - 1 - o : o;
+    const int grp = side ? R1 - 1 - s : s, cl = side ? COLS - 1 - o : o;
     C v[P][R2];
 #pragma unroll
     for (int p = 0; p < P; ++p) {
 #pragma unroll
-      for (int k = 0; k < R2; ++k) v[p][k] = sm[(p * N + grp * R2 + k) * COLS + col];
+      for (int k = 0; k < R2; ++k) v[p][k] = sm[(p * N + grp * R2 + k) * COLS + cl];
       dft::run<R2, false>(v[p]);
     }
     const int kx = x0 + o;
@@ -669,7 +769,7 @@ __device__ __forceinline__ void zline_tile(const IterArgs<T> &a, CxT<T> *sm, con
       dft::run<R2, true>(v[p]);
 #pragma unroll
       for (int k = 0; k < R2; ++k)
-        sm[(p * N + grp * R2 + k) * COLS + col] =
+        sm[(p * N + grp * R2 + k) * COLS + cl] =
             k ? dft::cmulw<true>(v[p][k], roots[k * grp]) : v[p][k];
     }
     if constexpr (AHEAD && R1 > R2)
@@ -678,10 +778,7 @@ __device__ __forceinline__ void zline_tile(const IterArgs<T> &a, CxT<T> *sm, con
         for (int k = 0; k < H; ++k) load_pair(i + Z::TH, k, fkv[k], X[k]);
   }
   __syncthreads();
-  {
-    const int col = threadIdx.x % COLS, t = threadIdx.x / COLS;
-    C *g = a.buf + (col < CW ? (size_t)ky * N + x0 + col
-                             : (size_t)(N - 1 - ky) * N + (N - x0 - 2 * CW) + col);
+  if (live) {
 #pragma unroll
     for (int p = 0; p < P; ++p) {
       C v[R1];
@@ -689,7 +786,7 @@ __device__ __forceinline__ void zline_tile(const IterArgs<T> &a, CxT<T> *sm, con
       for (int s = 0; s < R1; ++s) v[s] = sm[(p * N + s * R2 + t) * COLS + col];
       dft::run<R1, true>(v);
 #pragma unroll
-      for (int j = 0; j < R1; ++j) __stcg(g + (size_t)p * n + (size_t)(t + R2 * j) * N * N, v[j]);
+      for (int j = 0; j < R1; ++j) __stcg(g + (size_t)p * n + (size_t)(t + R2 * j) * plane, v[j]);
     }
   }
 }
@@ -699,7 +796,7 @@ __global__ void __launch_bounds__(ZShape<T, N, V>::TH, (ZShape<T, N, V>::MINB)) 
   extern __shared__ __align__(16) unsigned char fused_sm[];
   const IterArgs<T> a = solute_view<T, V>(a0);
   if (a.st->done) return;
-  zline_tile<T, N, V, false>(a, reinterpret_cast<CxT<T> *>(fused_sm), a.roots, blockIdx.x);
+  zline_tile<T, N, V, false, true>(a, reinterpret_cast<CxT<T> *>(fused_sm), a.roots, N, N, blockIdx.x);
 }
 
 // ---------------------------------------------------------------- one launch
@@ -733,7 +830,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned target) {
 // byte offset of the tables: after the largest of the stages' exchanges
 template <typename T, int N, int V> __host__ __device__ constexpr size_t tables_at() {
   const size_t row = sizeof(CxT<T>) * Lines<N>::LB * Lines<N>::LS,
-               z = sizeof(CxT<T>) * (size_t)((V + 1) / 2) * Lines<N>::LB * N;
+               z = sizeof(CxT<T>) * (size_t)((V + 1) / 2) * 2 * Lines<N>::CW * N;
   return row > z ? row : z;
 }
 
@@ -762,7 +859,7 @@ __global__ void __launch_bounds__(Lines<N>::TH, (Lines<N>::template minp<T, V>()
     if (!(ok = grid_barrier(bar, target += nblk))) break;
 #pragma unroll 1
     for (int tile = blockIdx.x; tile < ZShape<T, N, V>::TILES; tile += nblk) {
-      zline_tile<T, N, V, WIDE>(a, sm, roots, tile);
+      zline_tile<T, N, V, WIDE, true>(a, sm, roots, N, N, tile);
       __syncthreads();
     }
     if (!(ok = grid_barrier(bar, target += nblk))) break;
@@ -835,11 +932,11 @@ struct Kernels {
   using Z = ZShape<T, N, V>;
   static constexpr int P = (V + 1) / 2;
   // A phase as one launch, by what a step took on a B200 (us, loop of three
-  // launches / one launch; V = 2): FP64 N = 32 25.7 / 15.8, 64 32.9 / 22.4,
-  // 96 89.8 / 80.3, 128 145 / 130, 256 1022 / 1082; V = 4: 64 47.7 / 38.5,
-  // 96 159 / 171, 128 325 / 352 (the one kernel's registers spill).  FP32 one
-  // launch is never slower: 64 29.5 / 17.7, 128 101 / 84, 256 592 / 575.
-  static constexpr bool ONE = sizeof(T) == 4 || N <= 64 || (N <= 128 && V <= 2);
+  // launches / one launch; V = 2): FP64 N = 32 25 / 16, 64 31 / 23, 80 52 / 41,
+  // 128 152 / 132, 160 336 / 320, 256 1022 / 1082; V = 4: 64 47 / 39, 80 109 /
+  // 93, 128 316 / 354 (the one kernel's registers spill).  FP32 one launch is
+  // never slower: 64 31 / 19, 128 101 / 89, 256 592 / 575.
+  static constexpr bool ONE = sizeof(T) == 4 || N <= 80 || (N <= 160 && V <= 2);
   template <typename K> static cudaError_t allow(K k, size_t b) {
     return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
   }
@@ -918,9 +1015,7 @@ struct Kernels {
 template <typename T, int N>
 Vtable<T> table_v(int V) {
   switch (V) {
-    case 1: return {Kernels<T, N, 1>::setup, Kernels<T, N, 1>::launch};
     case 2: return {Kernels<T, N, 2>::setup, Kernels<T, N, 2>::launch};
-    case 3: return {Kernels<T, N, 3>::setup, Kernels<T, N, 3>::launch};
     case 4: return {Kernels<T, N, 4>::setup, Kernels<T, N, 4>::launch};
   }
   return {nullptr, nullptr};

@@ -1,14 +1,15 @@
-// Instantiations of the three-kernel iteration (fused.cuh): FP32, edges 32, 48, 64.
+// Instantiations of the plane kernels (fused.cuh): FP32, cell edges 32, 36, 40, 48.
 #include "fused.cuh"
 
 namespace rism3d {
 namespace fused {
 
-template <> Vtable<float> table_small<float>(int N, int V) {
+template <> Vtable<float> table_a<float>(int N, int V) {
   switch (N) {
     case 32: return table_v<float, 32>(V);
+    case 36: return table_v<float, 36>(V);
+    case 40: return table_v<float, 40>(V);
     case 48: return table_v<float, 48>(V);
-    case 64: return table_v<float, 64>(V);
   }
   return {nullptr, nullptr};
 }

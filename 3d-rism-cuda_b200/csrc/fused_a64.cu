@@ -1,14 +1,15 @@
-// Instantiations of the three-kernel iteration (fused.cuh): FP64, edges 32, 48, 64.
+// Instantiations of the plane kernels (fused.cuh): FP64, cell edges 32, 36, 40, 48.
 #include "fused.cuh"
 
 namespace rism3d {
 namespace fused {
 
-template <> Vtable<double> table_small<double>(int N, int V) {
+template <> Vtable<double> table_a<double>(int N, int V) {
   switch (N) {
     case 32: return table_v<double, 32>(V);
+    case 36: return table_v<double, 36>(V);
+    case 40: return table_v<double, 40>(V);
     case 48: return table_v<double, 48>(V);
-    case 64: return table_v<double, 64>(V);
   }
   return {nullptr, nullptr};
 }

@@ -93,13 +93,14 @@ __device__ __forceinline__ void adjoint_forward(const AdjointArgs<T> &g, const A
     __syncthreads();                               // the columns' exchange is free
 #pragma unroll 1
     for (int rb = 0; rb < L::SH; rb += LB) {
-      const int y = rank * L::SH + rb + row_l;
+      const bool live = L::FULL || (row_l < LB && rb + row_l < L::SH);
+      const int y = rank * L::SH + (live ? rb + row_l : 0);
       const size_t base = (size_t)(2 * p) * n + ((size_t)z * N + y) * N;
       const C tyz = cmul(tw[N + y], tw[2 * N + z]);
       const int dyz = (y + z) & 1;
       row_sync<R2>();                              // the exchange's last readers are done
 #pragma unroll 1
-      for (int q = 0; q < W::TOT; ++q) {
+      for (int q = 0; q < (live ? W::TOT : 0); ++q) {
         const int x0 = VW * (t + R2 * q);
         T xv[2][VW];
 #pragma unroll
@@ -140,10 +141,10 @@ __device__ __forceinline__ void adjoint_forward(const AdjointArgs<T> &g, const A
         }
       }
       row_sync<R2>();
-      rows_forward<T, N>(line, pb + (size_t)y * N, t, roots);
+      rows_forward<T, N>(line, pb + (size_t)y * N, t, live, roots);
     }
     plane_sync<L::NC>();                           // every row of the plane is in L2
-    columns<T, N, false>(pb, pb, rank * L::SH, sm, roots);
+    columns<T, N, false, L::FULL>(pb + rank * L::SH, pb + rank * L::SH, N, L::SH, sm, roots);
   }
 }
 
@@ -171,18 +172,20 @@ __device__ __forceinline__ void adjoint_residual(const AdjointArgs<T> &g, const 
   for (int plane = cl; plane < N * P; plane += ncl) {
     const int p = plane / N, z = plane % N;
     const bool two = V % 2 == 0 || 2 * p + 1 < V;
-    columns<T, N, true>(a.buf + (size_t)plane * N * N, scr, rank * L::SH, sm, roots);
+    columns<T, N, true, L::FULL>(a.buf + (size_t)plane * N * N + rank * L::SH, scr + rank * L::SH, N, L::SH,
+                        sm, roots);
     __syncthreads();                               // the columns' exchange is free
     plane_sync<L::NC>();                           // every column of the plane is in L2
 #pragma unroll 1
     for (int rb = 0; rb < L::SH; rb += LB) {
-      const int y = rank * L::SH + rb + row_l;
-      rows_inverse<T, N>(scr + (size_t)y * N, line, t, roots);
+      const bool live = L::FULL || (row_l < LB && rb + row_l < L::SH);
+      const int y = rank * L::SH + (live ? rb + row_l : 0);
+      rows_inverse<T, N>(scr + (size_t)y * N, line, t, live, roots);
       const size_t base = (size_t)(2 * p) * n + ((size_t)z * N + y) * N;
       const C tyz = cmul(tw[N + y], tw[2 * N + z]);
       const int dyz = (y + z) & 1;
 #pragma unroll 1
-      for (int q = 0; q < W::TOT; ++q) {
+      for (int q = 0; q < (live ? W::TOT : 0); ++q) {
         const int x0 = VW * (t + R2 * q);
         C h[VW];
 #pragma unroll
@@ -316,7 +319,7 @@ __global__ void __launch_bounds__(Lines<N>::TH, (Lines<N>::template minp<T, V>()
     if (!(ok = grid_barrier(g.it.bar, target += nblk))) break;
 #pragma unroll 1
     for (int tile = blockIdx.x; tile < ZShape<T, N, V>::TILES; tile += nblk) {
-      zline_tile<T, N, V, false>(g.it, sm, roots, tile);
+      zline_tile<T, N, V, false, true>(g.it, sm, roots, N, N, tile);
       __syncthreads();
     }
     if (!(ok = grid_barrier(g.it.bar, target += nblk))) break;
@@ -356,9 +359,7 @@ bool adjoint_launch(const AdjointArgs<T> &g, int *clusters, cudaStream_t st) {
 template <typename T, int N>
 AdjointLaunch<T> adjoint_table_v(int V) {
   switch (V) {
-    case 1: return adjoint_launch<T, N, 1>;
     case 2: return adjoint_launch<T, N, 2>;
-    case 3: return adjoint_launch<T, N, 3>;
     case 4: return adjoint_launch<T, N, 4>;
   }
   return nullptr;

@@ -1,0 +1,26 @@
+// Instantiations of the split form of the folded iteration (fused_split.cuh):
+// FP64, edges 32, 36, 40, 48, 60, 64, 72, 80, 96, 100, 108.
+#include "fused_split.cuh"
+
+namespace rism3d {
+namespace fused {
+
+template <> SplitRun<double> split_table_x<double>(int N, int V, int *lines) {
+  switch (N) {
+    case 32: return split_v<double, 32>(V, lines);
+    case 36: return split_v<double, 36>(V, lines);
+    case 40: return split_v<double, 40>(V, lines);
+    case 48: return split_v<double, 48>(V, lines);
+    case 60: return split_v<double, 60>(V, lines);
+    case 64: return split_v<double, 64>(V, lines);
+    case 72: return split_v<double, 72>(V, lines);
+    case 80: return split_v<double, 80>(V, lines);
+    case 96: return split_v<double, 96>(V, lines);
+    case 100: return split_v<double, 100>(V, lines);
+    case 108: return split_v<double, 108>(V, lines);
+  }
+  return nullptr;
+}
+
+}  // namespace fused
+}  // namespace rism3d

@@ -11,10 +11,6 @@ template <typename T> struct Cx;
 template <> struct Cx<double> { typedef double2 t; };
 template <> struct Cx<float> { typedef float2 t; };
 
-namespace {
-
-constexpr int kThreads = 256;
-
 template <typename T>
 struct IterArgs {
   long long n;
@@ -47,13 +43,19 @@ struct IterArgs {
   T *RPx;                   // third residual slot [V][N]
   typename Cx<T>::t *scr;   // plane exchange, scr_n points per solute
   long long scr_n;
-  const typename Cx<T>::t *roots;   // W_N^m, m < N (the cell edge)
+  const typename Cx<T>::t *roots;   // W_N^m, m < N (the cell edge); non-cubic: [nx] [ny] [nz]
+  const T *xo;              // non-cubic: chi_ab [nz/2][ny/2][nx/2][V*V], by |2 i + 1| per axis
   cudaGraphConditionalHandle cond;  // loop body: the while node to steer
   int loop;                 // 1: plane R runs the loop test itself
   int nb;                   // solutes
   unsigned *gcount;         // solutes whose plane R is done (nb > 1)
   unsigned *bar;            // arrival counts of a whole-phase launch [nb]
 };
+
+namespace {
+
+constexpr int kThreads = 256;
+
 
 // Batched solves: blockIdx.y selects the solute; every per-solute array is
 // laid out solute-major ([B][...]) and this view offsets the pointers, so
@@ -275,6 +277,29 @@ __device__ __forceinline__ void chi_cubic(const IterArgs<T> &a, int ix, int iy, 
   } else {
 #pragma unroll
     for (int ab = 0; ab < V * V; ++ab) X[ab] = (T)a.xs[row + ab];
+  }
+}
+
+// chi_ab(|k|) of a non-cubic cell from its octant table: |k| depends on the
+// distance of each index from the middle alone.
+template <typename T, int V>
+__device__ __forceinline__ void chi_octant(const IterArgs<T> &a, int ix, int iy, int iz,
+                                           T (&X)[V * V]) {
+  const int hx = a.nx / 2, hy = a.ny / 2, hz = a.nz / 2;
+  const int mx = ix < hx ? hx - 1 - ix : ix - hx, my = iy < hy ? hy - 1 - iy : iy - hy,
+            mz = iz < hz ? hz - 1 - iz : iz - hz;
+  const T *row = a.xo + ((size_t)mx + (size_t)hx * (my + (size_t)hy * mz)) * V * V;
+  if constexpr (V * V * sizeof(T) % 16 == 0) {
+#pragma unroll
+    for (int ab = 0; ab < V * V; ab += 16 / (int)sizeof(T)) {
+      union { float4 b; T t[16 / sizeof(T)]; } u;
+      u.b = *reinterpret_cast<const float4 *>(row + ab);
+#pragma unroll
+      for (int e = 0; e < 16 / (int)sizeof(T); ++e) X[ab + e] = u.t[e];
+    }
+  } else {
+#pragma unroll
+    for (int ab = 0; ab < V * V; ++ab) X[ab] = row[ab];
   }
 }
 

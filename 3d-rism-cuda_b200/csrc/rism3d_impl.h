@@ -231,6 +231,9 @@ struct Context {
   // three-kernel iteration (fused.cuh), per arithmetic: third residual slot,
   // exchange planes, roots of unity of the cell edge
   FusedPlan fu64, fu32;
+  bool split64 = false, split32 = false;   // in the split form (else planes)
+  double *d_xo = nullptr;       // chi octants of the split form
+  float *d_xo32 = nullptr;
   void *d_fused = nullptr;      // the allocation that holds the following
   double *d_RPx = nullptr;
   float *f_RPx = nullptr;

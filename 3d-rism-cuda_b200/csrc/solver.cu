@@ -1825,18 +1825,32 @@ void launch_iteration_dm(Context &c, const IterArgs<float> &a, cufftHandle plan)
   k_pass_r_dm<V, CLOS><<<a.nblocks, kThreads, 0, c.stream>>>(a, c.dm_depth);
 }
 
-template <typename T> fused::Vtable<T> fused_table(int N, int V) {
-  return N <= 64 ? fused::table_small<T>(N, V)
-                 : N <= 128 ? fused::table_medium<T>(N, V) : fused::table_large<T>(N, V);
-}
-
 // One iteration (or with which >= 0 one of its kernels) in the three-kernel
 // form (fused.cuh).
 template <typename T>
+void launch_split(Context &c, const IterArgs<T> &a, bool ref, int which) {
+  int lines = 1;
+  const fused::SplitRun<T> run[3] = {fused::split_table<T>(c.nx, c.natv, &lines),
+                                     fused::split_table<T>(c.ny, c.natv, nullptr),
+                                     fused::split_table<T>(c.nz, c.natv, nullptr)};
+  static const int axis[6] = {0, 1, 2, 1, 0, 0};
+  const int hnc = c.prm.closure == RISM3D_HNC;
+  IterArgs<T> ar = a;
+  ar.nblocks = (int)(((long long)c.ny * c.nz * ((c.natv + 1) / 2) + lines - 1) / lines);
+  if (which == 3) run[0](5, 0, ref, hnc, c.nb, ar, c.stream);
+  else
+    for (int k = 0; k < 5; ++k) run[axis[k]](k, axis[k], ref, hnc, c.nb, ar, c.stream);
+}
+
+template <typename T>
 void launch_fused(Context &c, const IterArgs<T> &a, bool ref, int which = -1) {
+  if (sizeof(T) == 8 ? c.split64 : c.split32) {  // which: -1 a cycle, 3 the pass after the loop
+    launch_split<T>(c, a, ref, which);
+    return;
+  }
   const FusedPlan &f = sizeof(T) == 8 ? c.fu64 : c.fu32;
   const int hnc = c.prm.closure == RISM3D_HNC;
-  const fused::Vtable<T> tab = fused_table<T>(c.nx, c.natv);
+  const fused::Vtable<T> tab = fused::table<T>(c.nx, c.natv);
   IterArgs<T> ar = a;
   ar.nblocks = (which == 4 ? f.cp[ref ? 1 : 0] : f.cr[ref ? 1 : 0]) * f.nc;
   if (which == 4) cudaMemsetAsync(c.d_bar, 0, sizeof(unsigned) * c.nb, c.stream);
@@ -2093,6 +2107,7 @@ void set_fused_args(Context &c, IterArgs<T> &a) {
   a.scr = (typename Cx<T>::t *)c.d_scr;
   a.scr_n = (long long)std::max(std::max(f.cr[0], f.cr[1]), std::max(f.cp[0], f.cp[1])) * c.nx * c.nx;
   a.nb = c.nb;
+  a.xo = (const T *)(sizeof(T) == 8 ? (void *)c.d_xo : (void *)c.d_xo32);
   a.gcount = c.d_count + c.nb;
   a.bar = c.d_bar;
 }
@@ -2404,7 +2419,7 @@ int solve_v(Context &c, int chargeup) {
       c.err = "a device-side wait gave up: a bulk or tile copy never arrived";
       status = RISM3D_CUDA_ERROR;
     }
-  c.launches += (c.fu64.on ? 3 : 4) * bodies;
+  c.launches += (c.split64 || c.split32 ? 5 : c.fu64.on ? 3 : 4) * bodies;
   c.res.rms = fs[0].rms;
   if (nb > 1) {
     c.bres.assign(nb, rism3d_result{});
@@ -2460,7 +2475,7 @@ int time_kernel_t(Context &c, int which, int reps, double *ms) {
   run.measure = 1;
   run.s1 = 0.25; run.s2 = 0.25;
   // the three-kernel iteration, where the solve runs it (14 is a transform)
-  const bool three = which != 14 && (fp64 ? c.fu64.on : c.fu32.on) &&
+  const bool three = which != 14 && !(fp64 ? c.split64 : c.split32) && (fp64 ? c.fu64.on : c.fu32.on) &&
                      !(!fp64 && which < 13 && (c.dm_depth || c.xfused));
   if (three) set_fused_args<T>(c, a);
   run.rotate = three ? 1 : 0;
@@ -2594,59 +2609,125 @@ int setup_pipe_r(Context &c) {
   return RISM3D_OK;
 }
 
-// The three-kernel iteration: cubic cells (edges and lengths equal, so that
-// chi comes from the per-|k|^2 table) whose edge has an instantiation, up to
-// four sites.  Other cells, and RISM3D_FUSED=0, keep the passes around the
-// 3D library transforms.
+// chi_ab on the octant of distances from the middle of k space (non-cubic
+// cells of the folded iteration): [nz/2][ny/2][nx/2][V*V], the spline of
+// chi_spline once per entry.
+template <int V>
+__global__ void k_chi_octant(IterArgs<double> a, double *xo, float *xo32) {
+  const int hx = a.nx / 2, hy = a.ny / 2, hz = a.nz / 2;
+  const long long tot = (long long)hx * hy * hz;
+  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < tot;
+       e += (long long)gridDim.x * blockDim.x) {
+    const int mx = (int)(e % hx), my = (int)(e / hx % hy), mz = (int)(e / hx / hy);
+    double X[V * V];
+    chi_spline<double, V>(a, hx + mx, hy + my, hz + mz, X);
+#pragma unroll
+    for (int ab = 0; ab < V * V; ++ab) {
+      xo[e * V * V + ab] = X[ab];
+      if (xo32) xo32[e * V * V + ab] = (float)X[ab];
+    }
+  }
+}
+
+// Called with every solvent table (upload_chi)
+int build_chi_octant(Context &c) {
+  if (!c.d_xo) return RISM3D_OK;
+  IterArgs<double> a = make_args<double>(c, true);
+  const int gb = grid_blocks(c.n / 8);
+  if (c.natv == 2) k_chi_octant<2><<<gb, kThreads, 0, c.stream>>>(a, c.d_xo, c.d_xo32);
+  else k_chi_octant<4><<<gb, kThreads, 0, c.stream>>>(a, c.d_xo, c.d_xo32);
+  c.launches += 1;
+  return cuda_ok(c, cudaGetLastError(), "chi octant") ? RISM3D_OK : RISM3D_CUDA_ERROR;
+}
+
+// The iteration with folded transforms: edges with an instantiation, two or
+// four sites, in the form that is fastest for the cell and the arithmetic
+// (cubic_form).  Other edges and sites, and RISM3D_FUSED=0, keep the passes
+// around the 3D library transforms.
 int setup_fused_iteration(Context &c) {
   c.fu64 = FusedPlan{};
   c.fu32 = FusedPlan{};
+  c.split64 = c.split32 = false;
   const char *off = getenv("RISM3D_FUSED");
-  if ((off && off[0] == '0') || c.natv > 4 || c.nx != c.ny || c.nx != c.nz ||
-      c.prm.box[0] != c.prm.box[1] || c.prm.box[0] != c.prm.box[2])
-    return RISM3D_OK;
+  if (off && off[0] == '0') return RISM3D_OK;
   const bool mixed = c.prm.precision == RISM3D_MIXED;
-  const fused::Vtable<double> t64 = fused_table<double>(c.nx, c.natv);
-  const fused::Vtable<float> t32 = fused_table<float>(c.nx, c.natv);
-  if (!t64.setup || (mixed && !t32.setup)) return RISM3D_OK;
-  if (!t64.setup(c.fu64, c.nb) || (mixed && !t32.setup(c.fu32, c.nb))) return RISM3D_OK;
-  const int N = c.nx;
+  const bool cubic = c.nx == c.ny && c.nx == c.nz && c.prm.box[0] == c.prm.box[1] &&
+                     c.prm.box[0] == c.prm.box[2];
+  const int V = c.natv, edge[3] = {c.nx, c.ny, c.nz};
+  fused::Form f64 = cubic ? fused::cubic_form(c.nx, true) : fused::kSplit,
+              f32 = !mixed ? fused::kLibrary : cubic ? fused::cubic_form(c.nx, false) : fused::kSplit;
+  const fused::Vtable<double> t64 = fused::table<double>(c.nx, V);
+  const fused::Vtable<float> t32 = fused::table<float>(c.nx, V);
+  if (f64 == fused::kPlanes && (!t64.setup || !t64.setup(c.fu64, c.nb))) f64 = fused::kLibrary;
+  if (f32 == fused::kPlanes && (!t32.setup || !t32.setup(c.fu32, c.nb))) f32 = fused::kLibrary;
+  // the split form: kernels of every axis' edge
+  int lines = 1;
+  auto split_ok = [&](auto zero) {
+    typedef decltype(zero) T;
+    IterArgs<T> a{};
+    a.nx = c.nx; a.ny = c.ny; a.nz = c.nz;
+    for (int d = 0; d < 3; ++d) {
+      const fused::SplitRun<T> run = fused::split_table<T>(edge[d], V, d ? nullptr : &lines);
+      if (!run) return false;
+      if (run(-1, d, false, 0, 1, a, c.stream) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+      }
+    }
+    return true;
+  };
+  if (f64 == fused::kSplit && !split_ok(0.0)) f64 = fused::kLibrary;
+  if (f32 == fused::kSplit && !split_ok(0.0f)) f32 = fused::kLibrary;
   auto max_cr = [](const FusedPlan &f) {
     return (size_t)std::max(std::max(f.cr[0], f.cr[1]), std::max(f.cp[0], f.cp[1]));
   };
-  // block sums: six per CTA of plane R in the partials' room
-  if (6 * max_cr(c.fu64) * c.fu64.nc > 64 * (size_t)c.nred_blocks ||
-      (mixed && 6 * max_cr(c.fu32) * c.fu32.nc > 64 * (size_t)c.nred_blocks))
-    return RISM3D_OK;
+  const bool split = f64 == fused::kSplit || f32 == fused::kSplit;
+  const size_t blocks =
+      std::max(std::max(max_cr(c.fu64) * c.fu64.nc, max_cr(c.fu32) * c.fu32.nc),
+               split ? ((size_t)c.ny * c.nz * ((V + 1) / 2) + lines - 1) / lines : 0);
+  const size_t scr = std::max(max_cr(c.fu64) * sizeof(double2), max_cr(c.fu32) * sizeof(float2)) *
+                     (size_t)c.nx * c.nx * c.nb;
+  const size_t oct = split ? (size_t)(c.n / 8) * V * V : 0;
+  if (f64 == fused::kLibrary && f32 == fused::kLibrary) return RISM3D_OK;
+  // block sums: six per block of plane R in the partials' room
+  if (6 * blocks > 64 * (size_t)c.nred_blocks) return RISM3D_OK;
   // one allocation: [roots FP64 | roots FP32 | barrier counts | third residual
-  // slots | exchange planes]
-  std::vector<unsigned char> head((sizeof(double2) + sizeof(float2)) * N + sizeof(unsigned) * c.nb, 0);
+  // slots | exchange planes | chi octants]; one root table per axis
+  const int nr = c.nx + c.ny + c.nz;
+  std::vector<unsigned char> head((sizeof(double2) + sizeof(float2)) * nr + sizeof(unsigned) * c.nb, 0);
   double2 *roots = (double2 *)head.data();
-  float2 *rootsf = (float2 *)(roots + N);
-  for (int m = 0; m < N; ++m) {
-    const double ang = 2.0 * kPi * m / N;
-    roots[m] = make_double2(cos(ang), -sin(ang));
-    rootsf[m] = make_float2((float)roots[m].x, (float)roots[m].y);
+  float2 *rootsf = (float2 *)(roots + nr);
+  for (int d = 0, off0 = 0; d < 3; ++d) {
+    const int N = edge[d];
+    for (int m = 0; m < N; ++m) {
+      const double ang = 2.0 * kPi * m / N;
+      roots[off0 + m] = make_double2(cos(ang), -sin(ang));
+      rootsf[off0 + m] = make_float2((float)roots[off0 + m].x, (float)roots[off0 + m].y);
+    }
+    off0 += N;
   }
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-  const size_t vn = (size_t)c.n * c.nb * c.natv, h = up(head.size()), r64 = up(sizeof(double) * vn),
-               r32 = mixed ? up(sizeof(float) * vn) : 0;
-  const size_t scr = std::max(max_cr(c.fu64) * sizeof(double2), max_cr(c.fu32) * sizeof(float2)) *
-                     (size_t)N * N * c.nb;
+  const size_t vn = (size_t)c.n * c.nb * V, h = up(head.size()), r64 = up(sizeof(double) * vn),
+               r32 = mixed ? up(sizeof(float) * vn) : 0, sc = up(scr), o64 = up(sizeof(double) * oct),
+               o32 = mixed ? up(sizeof(float) * oct) : 0;
   unsigned char *base = nullptr;
-  if (!cuda_ok(c, cudaMalloc(&base, h + r64 + r32 + scr), "alloc three-kernel iteration"))
+  if (!cuda_ok(c, cudaMalloc(&base, h + r64 + r32 + sc + o64 + o32), "alloc folded iteration"))
     return RISM3D_CUDA_ERROR;
   c.d_fused = base;
   if (!cuda_ok(c, cudaMemcpy(base, head.data(), head.size(), cudaMemcpyHostToDevice), "copy roots"))
     return RISM3D_CUDA_ERROR;
   c.d_roots = (double2 *)base;
-  c.f_roots = (float2 *)(c.d_roots + N);
-  c.d_bar = (unsigned *)(c.f_roots + N);
+  c.f_roots = (float2 *)(c.d_roots + nr);
+  c.d_bar = (unsigned *)(c.f_roots + nr);
   c.d_RPx = (double *)(base + h);
   c.f_RPx = mixed ? (float *)(base + h + r64) : nullptr;
   c.d_scr = base + h + r64 + r32;
-  c.fu64.on = true;
-  c.fu32.on = mixed;
+  c.d_xo = oct ? (double *)(base + h + r64 + r32 + sc) : nullptr;
+  c.d_xo32 = oct && mixed ? (float *)(base + h + r64 + r32 + sc + o64) : nullptr;
+  c.split64 = f64 == fused::kSplit;
+  c.split32 = f32 == fused::kSplit;
+  c.fu64.on = f64 != fused::kLibrary;
+  c.fu32.on = f32 != fused::kLibrary;
   return RISM3D_OK;
 }
 
@@ -2868,9 +2949,11 @@ int upload_chi(Context &c) {
   }
   if (c.chi.d_coef) cudaFree(c.chi.d_coef);
   if (!cuda_ok(c, cudaMalloc(&c.chi.d_coef, sizeof(double) * tab.size()), "chi alloc") ||
-      !cuda_ok(c, cudaMemcpyAsync(c.chi.d_coef, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice, c.stream), "chi copy") ||
-      !cuda_ok(c, cudaStreamSynchronize(c.stream), "chi"))
+      !cuda_ok(c, cudaMemcpyAsync(c.chi.d_coef, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice, c.stream), "chi copy"))
     return RISM3D_CUDA_ERROR;
+  const int rc = build_chi_octant(c);
+  if (rc != RISM3D_OK || !cuda_ok(c, cudaStreamSynchronize(c.stream), "chi"))
+    return rc != RISM3D_OK ? rc : RISM3D_CUDA_ERROR;
   return RISM3D_OK;
 }
 

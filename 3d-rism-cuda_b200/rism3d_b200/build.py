@@ -19,10 +19,12 @@ CLI1D = os.path.join(TOP, "bin", "rism1d-b200")
 CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA, "bin", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-SOURCES = ["solver.cu", "fused_large64.cu", "fused_large32.cu", "fused_medium64.cu",
-           "fused_medium32.cu", "fused_small64.cu", "fused_small32.cu", "fused_adjoint64.cu",
-           "fused_adjoint32.cu", "potential.cu", "observe.cu", "adjoint.cu", "batch.cu",
-           "noalloc.cu", "rmdft.cu", "capi.cpp", "io.cpp", "xrism1d.cpp"]
+SOURCES = ["solver.cu", "fused_c64.cu", "fused_b64.cu", "fused_a64.cu", "fused_c32.cu",
+           "fused_b32.cu", "fused_a32.cu", "fused_split_y64.cu", "fused_split_x64.cu",
+           "fused_split_y32.cu", "fused_split_x32.cu", "fused_adjoint_y64.cu",
+           "fused_adjoint_x64.cu", "fused_adjoint_y32.cu", "fused_adjoint_x32.cu",
+           "potential.cu", "observe.cu", "adjoint.cu", "batch.cu", "noalloc.cu",
+           "rmdft.cu", "capi.cpp", "io.cpp", "xrism1d.cpp"]
 
 
 def _ccbin():
