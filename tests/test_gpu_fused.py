@@ -174,3 +174,19 @@ def test_one_launch_adjoint_matches_the_host_driven_solve(monkeypatch, edge, xvk
         s.close()
     for a, b in zip(*out):
         assert _rel(a, b) < (1e-9 if precision == 0 else 2e-5)
+
+
+def test_depth_two_accelerator_is_an2(monkeypatch):
+    """The depth-2 accelerator of the FP32 bulk: where the folded iteration is
+    on it is AN2's own run, to the bit; the depth-M passes themselves match
+    AN2's unfused passes over 20 steps (FP32 rounding, 6e-8, and an
+    amplification below 1e4: 1e-3)."""
+    import rism3d_b200 as R
+    kw = dict(precision=R.MIXED, maxstep=20, convergence=1e-9)
+    for fused, tol in ((True, 0.0), (False, 1e-3)):
+        a = _solve(monkeypatch, fused, 64, WATER, **kw)
+        monkeypatch.setenv("RISM3D_MDIIS", "2")
+        b = _solve(monkeypatch, fused, 64, WATER, **kw)
+        monkeypatch.delenv("RISM3D_MDIIS")
+        assert a[0]["iterations"] == b[0]["iterations"]
+        assert abs(a[0]["rms"] - b[0]["rms"]) <= tol * a[0]["rms"]
