@@ -72,8 +72,24 @@ __device__ __forceinline__ double exp_neg(double x) {
 // within about 40 A.  Per (point, atom) one refined reciprocal square root
 // gives 1/r, r and 1/r^2.  Beyond 40 A the factor e^-r (< 4.3e-18) is
 // dropped: there the reference's q (1 - e^-r) / r already rounds to q / r.
-constexpr int kPts = 2;
+// The kernel is bound by FP64 issue, mostly of the pairs beyond 40 A, so these
+// take as few FP64 operations as they can: one third-order step refines 1/r
+// (5 instead of two Newton steps' 10), r^-6 is shared by the sites, which add
+// r^-6 (A r^-6 - B) (2 each instead of 6), and the distance tests compare bit
+// patterns.  256^3, 846 atoms, V = 2: 33.1 -> 24.1 ms in FP64, 26.4 -> 21.6 mixed.
+constexpr int kPts = 2;          // 4: 256^3 24.1 -> 22.5 ms, but 128^3 2.03 -> 2.09, spills
 constexpr int kBrick = 8;        // brick edge (points); x: 4 threads x kPts
+
+// 1/sqrt(x), x > 0 normal: the hardware approximation y (relative error below
+// 2^-20) and one third-order step y (1 + e/2 + 3 e^2/8), e = 1 - x y^2; what
+// is dropped, 5 e^3 / 16, is below 1e-18.  The approximation's low word is
+// zero, so y y is exact and e has no rounding to speak of.  x = 0 gives NaN.
+__device__ __forceinline__ double rsqrt_3(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y * y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
 
 template <int V, bool MIX>
 __global__ void __launch_bounds__(kThreads)
@@ -82,7 +98,7 @@ k_potential_r(int nx, int ny, int nz, int bricks_x, int bricks_y, double drx, do
               const int *__restrict__ acnt, SiteLJ sites, double ikbt, double ubeta,
               double *__restrict__ u, double *__restrict__ esr, double *__restrict__ fr) {
   __shared__ double4 sa[kTile];           // x y z q
-  __shared__ double2 sl[V][kTile];        // sigma_uv^2, 4 eps_uv / kBT
+  __shared__ double2 sl[V][kTile];        // 4 eps_uv sigma_uv^12 / kBT, 4 eps_uv sigma_uv^6 / kBT
   __shared__ float2 slf[V][kTile];        // the same in FP32 (MIX)
   const long long n = (long long)nx * ny * nz;
   // solute blockIdx.y: its atoms and its [V][N] / [N] grids
@@ -112,7 +128,9 @@ k_potential_r(int nx, int ny, int nz, int bricks_x, int bricks_y, double drx, do
 #pragma unroll
     for (int v = 0; v < V; ++v) acc[k][v] = 0.0;
   }
-  const double cut2 = 1.0e-4;   // (1e-2)^2, cal_LJ.cu:11-12
+  // r^2 tests on bit patterns (the order of non-negative doubles)
+  const long long cut2 = __double_as_longlong(1.0e-4),   // (1e-2)^2, cal_LJ.cu:11-12
+                  far2 = __double_as_longlong(1600.0);
   for (int t0 = 0; t0 < natom; t0 += kTile) {
     __syncthreads();
     for (int i = threadIdx.x; i < kTile; i += blockDim.x) {
@@ -122,8 +140,9 @@ k_potential_r(int nx, int ny, int nz, int bricks_x, int bricks_y, double drx, do
         sa[i] = make_double4(a[0], a[1], a[2], a[3]);
 #pragma unroll
         for (int v = 0; v < V; ++v) {
-          const double sg = (a[4] + sites.sig[v]) * 0.5;                 // cal_LJ.cu:28
-          sl[v][i] = make_double2(sg * sg, 4.0 * sqrt(a[5] * sites.eps[v]) * ikbt);  // :29, :38
+          const double sg = (a[4] + sites.sig[v]) * 0.5, s2 = sg * sg, s6 = s2 * s2 * s2;  // cal_LJ.cu:28
+          const double b6 = 4.0 * sqrt(a[5] * sites.eps[v]) * ikbt * s6;  // :29, :38
+          sl[v][i] = make_double2(b6 * s6, b6);
           slf[v][i] = make_float2((float)sl[v][i].x, (float)sl[v][i].y);
         }
       }
@@ -143,28 +162,25 @@ k_potential_r(int nx, int ny, int nz, int bricks_x, int bricks_y, double drx, do
 #pragma unroll
       for (int k = 0; k < kPts; ++k) {
         const double dx = rx[k] - at.x;
-        const double r2 = dx * dx + dyz;
-        const double ri = rsqrt_nr<MIX ? 1 : 2>(r2);
+        const double r2 = fma(dx, dx, dyz);
+        const long long rb = __double_as_longlong(r2);
+        const double ri = rsqrt_3(r2);           // NaN at r = 0: not used there
         if (MIX) {
-          const float ir2 = r2 < cut2 ? (float)(1.0 / cut2) : (float)(ri * ri);
+          const float i2 = rb < cut2 ? 1.0e4f : (float)(ri * ri), i6 = i2 * i2 * i2;
 #pragma unroll
           for (int v = 0; v < V; ++v) {
             const float2 p = slf[v][i];
-            const float s2 = p.x * ir2;
-            const float s6 = s2 * s2 * s2;
-            accf[k][v] += p.y * s6 * (s6 - 1.0f);
+            accf[k][v] += i6 * fmaf(p.x, i6, -p.y);
           }
         } else {
-          const double ir2 = r2 < cut2 ? 1.0 / cut2 : ri * ri;
+          const double i2 = rb < cut2 ? 1.0e4 : ri * ri, i6 = i2 * i2 * i2;
 #pragma unroll
           for (int v = 0; v < V; ++v) {
             const double2 p = sl[v][i];
-            const double s2 = p.x * ir2;
-            const double s6 = s2 * s2 * s2;
-            acc[k][v] += p.y * s6 * (s6 - 1.0);
+            acc[k][v] = fma(i6, fma(p.x, i6, -p.y), acc[k][v]);
           }
         }
-        if (r2 >= 1600.0) {                 // r >= 40 A: e^-r is below FP64 resolution
+        if (rb >= far2) {                   // r >= 40 A: e^-r is below FP64 resolution
           afr[k] += at.w * ri;
           continue;
         }
@@ -225,63 +241,67 @@ __global__ void k_phase_rows(int nx, int ny, int nz, double bx, double by, doubl
 }
 
 // fk on the owner half j < N/2 (cal_Coulomb.cu:125-149): the phase
-// e^{-ik.R} is the product of the three per-axis rows.  A block covers whole
-// x rows (or one row segment when nx > blockDim): per atom tile, the y-z
-// phase product of each of the block's rows is formed once in shared memory,
-// and each thread adds q e^{-i kx X} (yz) with one coalesced row load.
-constexpr int kRowsMax = 10;    // rows a block of min(256, 8 nx) points can touch
+// e^{-ik.R} is the product of the three per-axis rows.  A block covers
+// blockDim.x neighbouring kx of kRows rows (iy, iz); per atom tile the rows'
+// 4 pi q e^{-i ky Y} e^{-i kz Z} are formed once in shared memory, and each
+// thread adds e^{-i kx X} times them to its kRows points: one 16-byte load of
+// the x phase per atom for 4 kRows FP64 fused multiply-adds (one point per
+// thread read it for every point: 13 ms at 256^3 with 846 atoms, now 2.5).
+constexpr int kRows = 8;
 
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(128)
 k_potential_k(int nx, int ny, int nz, double bx, double by, double bz,
               const double *__restrict__ atoms_all, const int *__restrict__ aoff,
               const int *__restrict__ acnt, double ubeta,
               const double2 *__restrict__ ph_all, double2 *__restrict__ fkh) {
-  __shared__ double sq[kTile];
-  __shared__ double2 syz[kRowsMax][kTile];
-  const long long nh = (long long)nx * ny * nz / 2;
-  const int sb = blockIdx.y;
+  __shared__ double2 syz[kRows][kTile];
+  const int rows = ny * (nz / 2);
+  const int sb = blockIdx.z;
   const double *__restrict__ atoms = atoms_all + 8 * (size_t)aoff[sb];
   const int natom = acnt[sb];
   const double2 *__restrict__ ph = ph_all + (size_t)aoff[sb] * (nx + ny + nz);
-  fkh += (size_t)sb * nh;
-  const long long jb = (long long)blockIdx.x * blockDim.x;      // first point of the block
-  const long long j = jb + threadIdx.x;
-  const long long jj = j < nh ? j : nh - 1;
-  const int ix = (int)(jj % nx);
-  const long long row = jj / nx, row0 = jb / nx;
-  const int lrow = (int)(row - row0);                           // row within the block
-  const int nrows = (int)(min(nh - 1, jb + (long long)blockDim.x - 1) / nx - row0) + 1;
-  const int iy = (int)(row % ny), iz = (int)(row / ny);
-  const double kx = 2.0 * kPi * (ix - nx / 2.0 + 0.5) / bx;
-  const double ky = 2.0 * kPi * (iy - ny / 2.0 + 0.5) / by;
-  const double kz = 2.0 * kPi * (iz - nz / 2.0 + 0.5) / bz;
-  const double rk2 = kx * kx + ky * ky + kz * kz;
-  const double rk4i = 1.0 / (rk2 * (rk2 + 1.0));
+  fkh += (size_t)sb * nx * rows;
+  const int ix = blockIdx.y * blockDim.x + threadIdx.x, row0 = blockIdx.x * kRows;
+  const bool live = ix < nx;
   const int L = nx + ny + nz;
-  double re = 0.0, im = 0.0;
+  double re[kRows], im[kRows];
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) re[r] = im[r] = 0.0;
   for (int t0 = 0; t0 < natom; t0 += kTile) {
     const int m = min(kTile, natom - t0);
     __syncthreads();
-    for (int i = threadIdx.x; i < kTile; i += blockDim.x)
-      sq[i] = i < m ? 4.0 * kPi * atoms[8 * (size_t)(t0 + i) + 3] : 0.0;
-    for (int e = threadIdx.x; e < nrows * m; e += blockDim.x) {
-      const int r = e / m, i = e - r * m;
-      const long long rw = row0 + r;
-      const int y = (int)(rw % ny), z = (int)(rw / ny);
+    for (int e = threadIdx.x; e < kRows * m; e += blockDim.x) {
+      const int r = e / m, i = e - r * m, rw = min(row0 + r, rows - 1), y = rw % ny, z = rw / ny;
       const double2 *rowp = ph + (size_t)(t0 + i) * L;
+      const double q = 4.0 * kPi * atoms[8 * (size_t)(t0 + i) + 3];
       const double2 py = rowp[nx + y], pz = rowp[nx + ny + z];
-      syz[r][i] = make_double2(py.x * pz.x - py.y * pz.y, py.x * pz.y + py.y * pz.x);
+      syz[r][i] = make_double2(q * (py.x * pz.x - py.y * pz.y), q * (py.x * pz.y + py.y * pz.x));
     }
     __syncthreads();
+    const double2 *px0 = ph + (size_t)t0 * L + (live ? ix : 0);
+#pragma unroll 4
     for (int i = 0; i < m; ++i) {
-      const double2 px = ph[(size_t)(t0 + i) * L + ix];
-      const double2 yz = syz[lrow][i];
-      const double cr = px.x * yz.x - px.y * yz.y, ci = px.x * yz.y + px.y * yz.x;
-      re += sq[i] * cr;      // + 4 pi q cos(k.R)
-      im += sq[i] * ci;      // - 4 pi q sin(k.R)
+      const double2 px = px0[(size_t)i * L];
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) {            // + 4 pi q cos(k.R), - 4 pi q sin(k.R)
+        const double2 yz = syz[r][i];
+        re[r] = fma(px.x, yz.x, fma(-px.y, yz.y, re[r]));
+        im[r] = fma(px.x, yz.y, fma(px.y, yz.x, im[r]));
+      }
     }
   }
-  if (j < nh) fkh[j] = make_double2(re * rk4i * ubeta, im * rk4i * ubeta);
+  if (!live) return;
+  const double kx = 2.0 * kPi * (ix - nx / 2.0 + 0.5) / bx;
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) {
+    const int rw = row0 + r;
+    if (rw >= rows) break;
+    const double ky = 2.0 * kPi * (rw % ny - ny / 2.0 + 0.5) / by;
+    const double kz = 2.0 * kPi * (rw / ny - nz / 2.0 + 0.5) / bz;
+    const double rk2 = kx * kx + ky * ky + kz * kz;
+    const double rk4i = 1.0 / (rk2 * (rk2 + 1.0));
+    fkh[(size_t)rw * nx + ix] = make_double2(re[r] * rk4i * ubeta, im[r] * rk4i * ubeta);
+  }
 }
 
 template <int V>
@@ -354,9 +374,10 @@ int compute_potentials(Context &c) {
     return RISM3D_CUDA_ERROR;
   k_phase_rows<<<(unsigned)((L * c.natom + 255) / 256), 256, 0, c.stream>>>(
       c.nx, c.ny, c.nz, c.prm.box[0], c.prm.box[1], c.prm.box[2], c.d_atoms, c.natom, ph);
-  const int thr = c.nx >= 32 ? kThreads : 8 * c.nx;        // at most kRowsMax rows per block
-  long long blocks = (c.n / 2 + thr - 1) / thr;
-  k_potential_k<<<dim3((unsigned)blocks, c.nb), thr, 0, c.stream>>>(
+  const int thr = std::min(128, (c.nx + 31) / 32 * 32);
+  const dim3 gk((unsigned)((c.ny * (c.nz / 2) + kRows - 1) / kRows),
+                (unsigned)((c.nx + thr - 1) / thr), c.nb);
+  k_potential_k<<<gk, thr, 0, c.stream>>>(
       c.nx, c.ny, c.nz, c.prm.box[0], c.prm.box[1], c.prm.box[2], c.d_atoms,
       c.d_atom_off, c.d_atom_cnt, ubeta, ph, c.d_fkh);
   cudaFreeAsync(ph, c.stream);
