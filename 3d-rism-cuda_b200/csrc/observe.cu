@@ -95,10 +95,17 @@ constexpr int kAtomsPerBlock = 128;
 constexpr int kPtsTile = 128;
 
 // part layout: [chunk][atom][2V + 6]: SE_LJ[v], SE_ES[v] (rho_v applied),
-// grad LJ xyz, grad ES xyz (sum over v of rho_v * ...).  One FP64 rsqrt per
-// (point, atom) gives 1/r, r and 1/r^2; the cutoff r < sigma_uv/2 of the
-// reference is tested on r, with the correctly rounded sqrt only for points
-// within 1e-12 of the cutoff radius.
+// grad LJ xyz, grad ES xyz (sum over v of rho_v * ...).  The cutoff
+// r < sigma_uv/2 of the reference is tested on r, with the correctly rounded
+// sqrt only for points within 1e-12 of the cutoff radius.
+//
+// Bound by FP64 issue, so the pairs beyond every cutoff of their atom (all but
+// a few thousand per atom) take as few operations as they can, 36 with forces
+// and two sites instead of 80: rho_v g_v and sum_v q_v rho_v g_v are formed
+// once per point, r^-6 (A r^-6 - B) shares its terms between energy and force,
+// constant factors wait for the end, and the cutoff test compares bit patterns.
+// Pairs near a cutoff, at r = 0 or off the number range take the plain form.
+// 128^3, 300 atoms, two sites, forces: 4.99 -> 2.81 ms.
 template <int V, int GRAD>
 __global__ void __launch_bounds__(kAtomsPerBlock)
 k_atom_integrals(int nx, int ny, int nz, double drx, double dry, double drz,
@@ -112,8 +119,8 @@ k_atom_integrals(int nx, int ny, int nz, double drx, double dry, double drz,
   const double *__restrict__ atoms = atoms_all + 8 * (size_t)aoff[sb];
   const int natom = acnt[sb];
   g += (size_t)sb * V * (size_t)nx * ny * nz;
-  __shared__ double4 pp[kPtsTile];          // x y z
-  __shared__ double pg[V][kPtsTile];
+  __shared__ double4 pp[kPtsTile];          // x y z, sum_v q_v rho_v g_v
+  __shared__ double pg[V][kPtsTile];        // rho_v g_v
   const long long n = (long long)nx * ny * nz;
   const int ia = blockIdx.x * kAtomsPerBlock + threadIdx.x;
   const bool live = ia < natom;
@@ -122,16 +129,20 @@ k_atom_integrals(int nx, int ny, int nz, double drx, double dry, double drz,
     const double *a = atoms + 8 * (size_t)ia;
     X = a[0]; Y = a[1]; Z = a[2]; qu = a[3]; su = a[4]; eu = a[5];
   }
-  double s6v[V], e4[V], qq[V], hs[V];
+  double A[V], B[V], hs[V], hmax = 0.0;        // 4 eps sigma^12, 4 eps sigma^6
 #pragma unroll
   for (int v = 0; v < V; ++v) {
     const double sg = (su + sv.sig[v]) * 0.5;  // cal_LJ.cu:28
-    const double sg2 = sg * sg;
-    s6v[v] = sg2 * sg2 * sg2;
-    e4[v] = 4.0 * sqrt(eu * sv.eps[v]);        // cal_LJ.cu:29
-    qq[v] = qu * sv.q[v] * cc;
+    const double sg2 = sg * sg, s6 = sg2 * sg2 * sg2;
+    B[v] = 4.0 * sqrt(eu * sv.eps[v]) * s6;    // cal_LJ.cu:29
+    A[v] = B[v] * s6;
     hs[v] = sg * 0.5;
+    hmax = fmax(hmax, fabs(hs[v]));
   }
+  // r^2 in [far, infinity) on bit patterns
+  const long long far = __double_as_longlong(fmax(hmax * hmax * (1.0 + 1.0e-9), 1.0e-8));
+  const unsigned long long span =
+      (unsigned long long)(0x7ff0000000000000LL - far);
   double acc[NA];
 #pragma unroll
   for (int k = 0; k < NA; ++k) acc[k] = 0.0;
@@ -144,10 +155,15 @@ k_atom_integrals(int nx, int ny, int nz, double drx, double dry, double drz,
       if (j < j1) {
         const long long r = j / nx;
         const int ix = (int)(j - r * nx), iy = (int)(r % ny), iz = (int)(r / ny);
-        pp[i] = make_double4((ix - nx / 2) * drx, (iy - ny / 2) * dry,   // cal_euv.cu:45-47
-                             (iz - nz / 2) * drz, 0.0);
+        double w = 0.0;
 #pragma unroll
-        for (int v = 0; v < V; ++v) pg[v][i] = g[(size_t)v * n + j];
+        for (int v = 0; v < V; ++v) {
+          const double gr = g[(size_t)v * n + j] * sv.rho[v];
+          pg[v][i] = gr;
+          w = fma(sv.q[v], gr, w);
+        }
+        pp[i] = make_double4((ix - nx / 2) * drx, (iy - ny / 2) * dry,   // cal_euv.cu:45-47
+                             (iz - nz / 2) * drz, w);
       } else {
         pp[i] = make_double4(1.0e30, 1.0e30, 1.0e30, 0.0);
 #pragma unroll
@@ -160,25 +176,42 @@ k_atom_integrals(int nx, int ny, int nz, double drx, double dry, double drz,
     for (int i = 0; i < m; ++i) {
       const double4 p = pp[i];
       const double dx = p.x - X, dy = p.y - Y, dz = p.z - Z;
-      const double r2 = dx * dx + dy * dy + dz * dz;
-      const double ri = rsqrt_nr<2>(r2);
-      const double r1 = r2 * ri;
-      const double ir2 = ri * ri;
-      const double ir6 = ir2 * ir2 * ir2;
+      const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+      if ((unsigned long long)(__double_as_longlong(r2) - far) < span) {
+        const double ri = rsqrt_3(r2), i2 = ri * ri, i6 = i2 * i2 * i2;
+        double f = 0.0;
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const double gr = pg[v][i], w = gr * i6, t = fma(A[v], i6, -B[v]);
+          acc[v] = fma(w, t, acc[v]);
+          acc[V + v] = fma(gr, ri, acc[V + v]);
+          if (GRAD) f = fma(w, fma(A[v], i6, t), f);
+        }
+        if (GRAD) {
+          const double e = p.w * (ri * i2);
+          f *= i2;
+          acc[2 * V + 0] = fma(f, dx, acc[2 * V + 0]);
+          acc[2 * V + 1] = fma(f, dy, acc[2 * V + 1]);
+          acc[2 * V + 2] = fma(f, dz, acc[2 * V + 2]);
+          acc[2 * V + 3] = fma(e, dx, acc[2 * V + 3]);
+          acc[2 * V + 4] = fma(e, dy, acc[2 * V + 4]);
+          acc[2 * V + 5] = fma(e, dz, acc[2 * V + 5]);
+        }
+        continue;
+      }
+      const double ri = rsqrt_nr<2>(r2), r1 = r2 * ri, i2 = ri * ri, i6 = i2 * i2 * i2;
 #pragma unroll
       for (int v = 0; v < V; ++v) {
-        bool inside = !(r1 >= hs[v]);           // r = 0 gives NaN: inside
+        bool inside = !(r1 >= hs[v]);         // NaN: inside
         if (fabs(r1 - hs[v]) < 1.0e-12 * hs[v]) inside = sqrt(r2) < hs[v];
         if (inside) continue;                 // cutoff r < sigma/2
-        const double gv = pg[v][i];
-        const double rs6i = s6v[v] * ir6;
-        acc[v] += e4[v] * rs6i * (rs6i - 1.0) * gv;
-        acc[V + v] += qq[v] * ri * gv;
+        const double gr = pg[v][i], w = gr * i6, t = fma(A[v], i6, -B[v]);
+        acc[v] += w * t;
+        acc[V + v] += gr * ri;
         if (GRAD) {
-          const double ulj = 6.0 * e4[v] * rs6i * ir2 * (2.0 * rs6i - 1.0) * gv * sv.rho[v];
-          const double uco = qq[v] * ri * ir2 * gv * sv.rho[v];
-          acc[2 * V + 0] += ulj * dx; acc[2 * V + 1] += ulj * dy; acc[2 * V + 2] += ulj * dz;
-          acc[2 * V + 3] += uco * dx; acc[2 * V + 4] += uco * dy; acc[2 * V + 5] += uco * dz;
+          const double f = w * fma(A[v], i6, t) * i2, e = sv.q[v] * gr * (ri * i2);
+          acc[2 * V + 0] += f * dx; acc[2 * V + 1] += f * dy; acc[2 * V + 2] += f * dz;
+          acc[2 * V + 3] += e * dx; acc[2 * V + 4] += e * dy; acc[2 * V + 5] += e * dz;
         }
       }
     }
@@ -187,11 +220,14 @@ k_atom_integrals(int nx, int ny, int nz, double drx, double dry, double drz,
     double *o = part + ((size_t)blockIdx.y * natom_tot + aoff[sb] + ia) * NA;
 #pragma unroll
     for (int v = 0; v < V; ++v) {
-      o[v] = acc[v] * sv.rho[v];
-      o[V + v] = acc[V + v] * sv.rho[v];
+      o[v] = acc[v];
+      o[V + v] = acc[V + v] * (qu * sv.q[v] * cc);
     }
 #pragma unroll
-    for (int k = 2 * V; k < NA; ++k) o[k] = acc[k];
+    for (int k = 0; k < 3; ++k) {
+      o[2 * V + k] = 6.0 * acc[2 * V + k];
+      o[2 * V + 3 + k] = (qu * cc) * acc[2 * V + 3 + k];
+    }
   }
 }
 

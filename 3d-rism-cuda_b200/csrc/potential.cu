@@ -80,17 +80,6 @@ __device__ __forceinline__ double exp_neg(double x) {
 constexpr int kPts = 2;          // 4: 256^3 24.1 -> 22.5 ms, but 128^3 2.03 -> 2.09, spills
 constexpr int kBrick = 8;        // brick edge (points); x: 4 threads x kPts
 
-// 1/sqrt(x), x > 0 normal: the hardware approximation y (relative error below
-// 2^-20) and one third-order step y (1 + e/2 + 3 e^2/8), e = 1 - x y^2; what
-// is dropped, 5 e^3 / 16, is below 1e-18.  The approximation's low word is
-// zero, so y y is exact and e has no rounding to speak of.  x = 0 gives NaN.
-__device__ __forceinline__ double rsqrt_3(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y * y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
 template <int V, bool MIX>
 __global__ void __launch_bounds__(kThreads)
 k_potential_r(int nx, int ny, int nz, int bricks_x, int bricks_y, double drx, double dry,

@@ -77,6 +77,17 @@ __device__ __forceinline__ double rsqrt_nr(double x) {
   for (int s = 0; s < STEPS; ++s) y = y * (1.5 - 0.5 * x * y * y);
   return y;
 }
+
+// 1/sqrt(x), x > 0 normal: the hardware approximation y (relative error below
+// 2^-20) and one third-order step y (1 + e/2 + 3 e^2/8), e = 1 - x y^2; what
+// is dropped, 5 e^3 / 16, is below 1e-18.  The approximation's low word is
+// zero, so y y is exact and e has no rounding to speak of.  x = 0 gives NaN.
+__device__ __forceinline__ double rsqrt_3(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y * y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
 #endif
 
 // Per charge-up stage constants, read by the kernels through a pointer so
