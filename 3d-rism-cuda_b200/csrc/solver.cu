@@ -1328,7 +1328,8 @@ __global__ void __launch_bounds__(kThreads) k_pass_a_pipe(IterArgs<T> a0) {
 // c_i = <R, d_i> and a_ij = <d_i, d_j> (d_i = R - R_i, weights 1/rho_v) over
 // the filled slots; the finalize solves a s = c in FP64 and adds the AN2
 // bias mp to the newest slot; pass A applies t = y + sum_i s_i (Y_i - y),
-// y = t + m R.  With M = 2 this is AN2's update (anderson.cu:35-63), and the
+// y = t + m R.  With M = 2 this is AN2's update (anderson.cu:35-63; it runs
+// as AN2 where that has the folded iteration), and the
 // elimination below runs in the order of the reference's 2 x 2 solve
 // (leg, anderson.cu:87-112).  Sums: [0] R^2, [1 + i] c_i, [1 + kDmMax + tri]
 // a_ij (packed upper triangle).

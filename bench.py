@@ -121,6 +121,12 @@ def iter_bytes_per_point(V, s):
     return {"pass_a": 9 * V * s, "pass_k": 2 * V * s + 8, "pass_r": 5 * V * s}
 
 
+def folded_bytes_per_point(V, s):
+    """The same of the three kernels with the 3D transforms folded in: plane A,
+    z lines, plane R (cubic cells, two or four sites)."""
+    return {"pass_a": 8 * V * s, "pass_k": 2 * V * s + 8, "pass_r": 6 * V * s}
+
+
 def fused_pipeline_bytes_per_iter(n, V, s, s_lr=None):
     """N (31 V s + 5 s_lr + 4): minimal fused pipeline of the per-site design;
     the long-range Coulomb grids (e, fr, fk) stay FP64 (s_lr = 8) in the
@@ -253,23 +259,23 @@ def run_ours(args, rank, world, dist):
     # the solve stream; run after the results were read)
     n = ctrl.grid[0] * ctrl.grid[1] * ctrl.grid[2]
     V = sv.natv
-    bpp32 = iter_bytes_per_point(V, 4)
-    bpp64 = iter_bytes_per_point(V, 8)
+    # the opt-in RISM3D_XFFT form of the FP32 passes: cuFFT then transforms along
+    # z only (kernel id 14, one strided C2C pass: 16 B/point read + write of the
+    # packed site pair)
     kern = {}
-    for name, kid, bpp in (("pass_a_fp32", 10, bpp32["pass_a"]), ("pass_k_fp32", 11, bpp32["pass_k"]),
-                           ("pass_r_fp32", 12, bpp32["pass_r"])):
-        ms = mixed.time_kernel(kid, 20)
-        kern[name] = {"ms": ms, "gbs": bpp * n / ms / 1e6}
-    # the FP32 iteration folds the x and y axes of its transforms into passes
-    # A, K and R when the cell allows (256^3 here); cuFFT then transforms
-    # along z only (kernel id 14, one strided C2C pass: 16 B/point read +
-    # write of the packed site pair)
     fused = True
     try:
         ms = mixed.time_kernel(14, 20)
         kern["fft_z_fp32"] = {"ms": ms, "gbs": 2 * 8 * ((V + 1) // 2) * n / ms / 1e6}
     except R.RismError:
         fused = False
+    folded = os.environ.get("RISM3D_FUSED") != "0"        # both cells here have that form
+    bpp32 = folded_bytes_per_point(V, 4) if folded and not fused else iter_bytes_per_point(V, 4)
+    bpp64 = folded_bytes_per_point(V, 8) if folded else iter_bytes_per_point(V, 8)
+    for name, kid, bpp in (("pass_a_fp32", 10, bpp32["pass_a"]), ("pass_k_fp32", 11, bpp32["pass_k"]),
+                           ("pass_r_fp32", 12, bpp32["pass_r"])):
+        ms = mixed.time_kernel(kid, 20)
+        kern[name] = {"ms": ms, "gbs": bpp * n / ms / 1e6}
     for name, kid, bpp in (("pass_a_fp64", 0, bpp64["pass_a"]), ("pass_k_fp64", 1, bpp64["pass_k"]),
                            ("pass_r_fp64", 2, bpp64["pass_r"])):
         ms = fp64.time_kernel(kid, 20)
@@ -305,10 +311,17 @@ def run_ours(args, rank, world, dist):
                        "(context, file reads, solve, .xmu), as the reference executable is timed"}
     dom = "pass_a_fp32"
     achieved = kern[dom]["gbs"]
-    dom_kernel = ("k_pass_ax<float> (FP32 pass A with the x-axis DFTs: inverse x-DFT of the "
-                  "last OZ result, AN2 update, closure, forward x-DFT)" if fused else
-                  "k_pass_a<float> (FP32 pass A: AN2 update + closure + forward pack)")
-    traffic_pp = read_traffic("k_pass_ax_fp32" if fused else "k_pass_a_fp32")
+    if fused:
+        dom_name, dom_kernel = "k_pass_ax_fp32", (
+            "k_pass_ax<float> (FP32 pass A with the x-axis DFTs: inverse x-DFT of the "
+            "last OZ result, AN2 update, closure, forward x-DFT)")
+    elif folded:
+        dom_name, dom_kernel = "k_plane_a_fp32", (
+            "k_plane_a<float> (FP32 plane A: AN2 update, closure, x- and y-DFT of each xy plane)")
+    else:
+        dom_name, dom_kernel = "k_pass_a_fp32", (
+            "k_pass_a<float> (FP32 pass A: AN2 update + closure + forward pack)")
+    traffic_pp = read_traffic(dom_name)
     dmu = abs(rm["sfe_sc"] - r64["sfe_sc"])
     out = {
         "metric": METRIC, "value": ms_mixed / 1e3 / world, "unit": "s/solve",

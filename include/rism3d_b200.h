@@ -206,8 +206,11 @@ long long rism3d_kernel_launches(const rism3d_ctx *ctx);
  * context stream and report the mean device time per launch (CUDA events).
  * which: 0/1/2 = FP64 pass A / pass K / pass R, 10/11/12 = the FP32
  * versions (MIXED contexts), 13/15 = FP32 pass A / pass R of the
- * refinement form (MIXED, after a solve), 20 = real-space potential kernel.  The
- * iteration kernels run on the current state with an AN2 update armed, so
+ * refinement form (MIXED, after a solve), 20 = real-space potential kernel.
+ * Where the iteration is the three kernels with the transforms folded in, pass
+ * A is plane A (with the x- and y-DFT), pass K the z lines (with the z-DFT both
+ * ways) and pass R plane R (with the inverse y- and x-DFT).  The iteration
+ * kernels run on the current state with an AN2 update armed, so
  * the stored solution is invalid afterwards (solve again to restore it). */
 int rism3d_time_kernel(rism3d_ctx *ctx, int which, int reps, double *ms_per_launch);
 
