@@ -328,7 +328,7 @@ int context_init(Context &c, const rism3d_params *p, int nb, std::string &err) {
   c.nred_blocks = (int)(nbk < 148 * 8 ? nbk : 148 * 8);
   ok = ok && cuda_ok(c, cudaMalloc(&c.d_part, sizeof(double) * 64 * c.nred_blocks * nb), "alloc partials") &&
        cuda_ok(c, cudaMalloc(&c.d_count, sizeof(unsigned) * (nb + 1)), "alloc counter") &&
-       cuda_ok(c, cudaMemset(c.d_count, 0, sizeof(unsigned) * (nb + 1)), "zero counter");
+       cuda_ok(c, cudaMemsetAsync(c.d_count, 0, sizeof(unsigned) * (nb + 1), c.stream), "zero counter");
   for (Timer *t : {&c.tm_setup, &c.tm_iter, &c.tm_obs}) {
     cudaEventCreate(&t->a);
     cudaEventCreate(&t->b);
@@ -514,11 +514,11 @@ int rism3d_set_rmdft(rism3d_ctx *x, const double *cvk, int ntab2, const double *
   if (!cuda_ok(c, cudaMalloc(&c.d_rm_ccoef, sizeof(double) * cc.size()), "alloc RMDFT") ||
       !cuda_ok(c, cudaMalloc(&c.d_rm_k2, sizeof(double) * ntab2), "alloc RMDFT") ||
       !cuda_ok(c, cudaMalloc(&c.d_rm_hcoef, sizeof(double) * hc.size()), "alloc RMDFT") ||
-      !cuda_ok(c, cudaMemcpy(c.d_rm_ccoef, cc.data(), sizeof(double) * cc.size(),
+      !cuda_ok(c, stream_copy(c, c.d_rm_ccoef, cc.data(), sizeof(double) * cc.size(),
                              cudaMemcpyHostToDevice), "copy RMDFT") ||
-      !cuda_ok(c, cudaMemcpy(c.d_rm_k2, k, sizeof(double) * ntab2, cudaMemcpyHostToDevice),
+      !cuda_ok(c, stream_copy(c, c.d_rm_k2, k, sizeof(double) * ntab2, cudaMemcpyHostToDevice),
                "copy RMDFT") ||
-      !cuda_ok(c, cudaMemcpy(c.d_rm_hcoef, hc.data(), sizeof(double) * hc.size(),
+      !cuda_ok(c, stream_copy(c, c.d_rm_hcoef, hc.data(), sizeof(double) * hc.size(),
                              cudaMemcpyHostToDevice), "copy RMDFT"))
     return RISM3D_CUDA_ERROR;
   c.rm_ntab2 = ntab2;

@@ -348,6 +348,14 @@ bool cuda_ok(Context &c, cudaError_t e, const char *what);
 inline cudaError_t pool_alloc(Context &c, void **p, size_t bytes) {
   return cudaMallocFromPoolAsync(p, bytes, c.pool, c.stream);
 }
+// Copy on the context's stream, complete on return.  Copies on the legacy
+// stream do not serve: that stream does not order a context's own non-blocking
+// one, and a small copy from pageable memory may return before it has landed.
+inline cudaError_t stream_copy(Context &c, void *dst, const void *src, size_t bytes,
+                               cudaMemcpyKind kind) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, c.stream);
+  return e == cudaSuccess ? cudaStreamSynchronize(c.stream) : e;
+}
 // message returned by rism3d_last_error(NULL) (context-free entry points)
 void set_create_error(const std::string &msg);
 bool cufft_ok(Context &c, cufftResult r, const char *what);

@@ -2230,7 +2230,7 @@ int run_phase(Context &c, cufftHandle plan, T *t, T *U, T *Y, T *RP,
     if (cuda_ok(c, cudaMemcpyAsync(&s0, c.d_state, sizeof(DevState), cudaMemcpyDeviceToHost, c.stream), "state") &&
         cuda_ok(c, cudaStreamSynchronize(c.stream), "state") && s0.iter > 0) {
       std::vector<double> hr(std::min(s0.iter, c.hist_cap));
-      if (cuda_ok(c, cudaMemcpy(hr.data(), c.d_hist, sizeof(double) * hr.size(), cudaMemcpyDeviceToHost), "history"))
+      if (cuda_ok(c, stream_copy(c, hr.data(), c.d_hist, sizeof(double) * hr.size(), cudaMemcpyDeviceToHost), "history"))
         for (size_t i = 0; i < hr.size(); ++i) printf(" Step = %d Reside = %g\n", (int)i + 1, hr[i]);
     }
   }
@@ -2470,7 +2470,7 @@ int time_kernel_t(Context &c, int which, int reps, double *ms) {
   a.tw = (const typename Cx<T>::t *)(fp64 ? (void *)c.d_tw : (void *)c.d_twf);
   DevState saved, run;
   if (!cuda_ok(c, cudaStreamSynchronize(c.stream), "time_kernel")) return RISM3D_CUDA_ERROR;
-  cudaMemcpy(&saved, c.d_state, sizeof(DevState), cudaMemcpyDeviceToHost);
+  stream_copy(c, &saved, c.d_state, sizeof(DevState), cudaMemcpyDeviceToHost);
   run = saved;
   run.done = 0; run.after_done = 0; run.mode = 2; run.count = 0; run.upd_slot = 0;
   run.measure = 1;
@@ -2481,7 +2481,7 @@ int time_kernel_t(Context &c, int which, int reps, double *ms) {
   if (three) set_fused_args<T>(c, a);
   run.rotate = three ? 1 : 0;
   run.rp[0] = 0; run.rp[1] = 1; run.rp[2] = 2;
-  cudaMemcpy(c.d_state, &run, sizeof(DevState), cudaMemcpyHostToDevice);
+  stream_copy(c, c.d_state, &run, sizeof(DevState), cudaMemcpyHostToDevice);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -2539,7 +2539,7 @@ int time_kernel_t(Context &c, int which, int reps, double *ms) {
   cudaEventElapsedTime(&t, e0, e1);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  cudaMemcpy(c.d_state, &saved, sizeof(DevState), cudaMemcpyHostToDevice);
+  stream_copy(c, c.d_state, &saved, sizeof(DevState), cudaMemcpyHostToDevice);
   c.solved = false;
   c.have_forces = false;
   if (!cuda_ok(c, e, "time_kernel")) return RISM3D_CUDA_ERROR;
@@ -2715,7 +2715,7 @@ int setup_fused_iteration(Context &c) {
   if (!cuda_ok(c, cudaMalloc(&base, h + r64 + r32 + sc + o64 + o32), "alloc folded iteration"))
     return RISM3D_CUDA_ERROR;
   c.d_fused = base;
-  if (!cuda_ok(c, cudaMemcpy(base, head.data(), head.size(), cudaMemcpyHostToDevice), "copy roots"))
+  if (!cuda_ok(c, stream_copy(c, base, head.data(), head.size(), cudaMemcpyHostToDevice), "copy roots"))
     return RISM3D_CUDA_ERROR;
   c.d_roots = (double2 *)base;
   c.f_roots = (float2 *)(c.d_roots + nr);
@@ -2819,7 +2819,7 @@ int setup_fused_axes(Context &c) {
     roots[m] = make_float2((float)cos(ang), (float)-sin(ang));
   }
   if (!cuda_ok(c, cudaMalloc(&c.d_xroots, sizeof(float2) * c.nx), "alloc roots") ||
-      !cuda_ok(c, cudaMemcpy(c.d_xroots, roots.data(), sizeof(float2) * c.nx, cudaMemcpyHostToDevice),
+      !cuda_ok(c, stream_copy(c, c.d_xroots, roots.data(), sizeof(float2) * c.nx, cudaMemcpyHostToDevice),
                "copy roots"))
     return RISM3D_CUDA_ERROR;
   // transforms along z: one per (x, y) column, stride nx ny, columns adjacent
@@ -2942,9 +2942,9 @@ int upload_chi(Context &c) {
     }
     std::vector<float> xs32(xs.begin(), xs.end());     // the FP32 passes' copy
     if (!cuda_ok(c, cudaMalloc(&c.d_xs, sizeof(double) * xs.size()), "chi table alloc") ||
-        !cuda_ok(c, cudaMemcpy(c.d_xs, xs.data(), sizeof(double) * xs.size(), cudaMemcpyHostToDevice), "chi table copy") ||
+        !cuda_ok(c, stream_copy(c, c.d_xs, xs.data(), sizeof(double) * xs.size(), cudaMemcpyHostToDevice), "chi table copy") ||
         !cuda_ok(c, cudaMalloc(&c.d_xs32, sizeof(float) * xs32.size()), "chi table alloc") ||
-        !cuda_ok(c, cudaMemcpy(c.d_xs32, xs32.data(), sizeof(float) * xs32.size(), cudaMemcpyHostToDevice), "chi table copy"))
+        !cuda_ok(c, stream_copy(c, c.d_xs32, xs32.data(), sizeof(float) * xs32.size(), cudaMemcpyHostToDevice), "chi table copy"))
       return RISM3D_CUDA_ERROR;
     c.nxs = nidx;
   }
