@@ -565,7 +565,7 @@ int adjoint_one_launch(Context &c, const T *G, const T *w, T *xi, T *Lxi, T *ys,
   a.invvol = 1.0 / c.vol; a.dv = c.dv;
   a.fkh = c.d_fkh; a.nofk = 1;
   a.sp = sp0;
-  a.bar = c.d_bar;
+  a.delay = c.stage_delay;
   a.scr = S.get<CT>((size_t)clusters * N * N);
   fused::AdjointState h{};
   h.best = 1e300;
@@ -574,8 +574,7 @@ int adjoint_one_launch(Context &c, const T *G, const T *w, T *xi, T *Lxi, T *ys,
   if (!a.scr || !g.st) { c.err = "adjoint: out of device memory"; return RISM3D_CUDA_ERROR; }
   g.G = G; g.w = w; g.xi = xi; g.Lxi = Lxi; g.ys = ys; g.rs = rs; g.part = part;
   g.eta = eta; g.tol = tol; g.maxit = maxit;
-  if (!cuda_ok(c, cudaMemcpyAsync(g.st, &h, sizeof(h), cudaMemcpyHostToDevice, c.stream), "adjoint") ||
-      !cuda_ok(c, cudaMemsetAsync(c.d_bar, 0, sizeof(unsigned), c.stream), "adjoint"))
+  if (!cuda_ok(c, cudaMemcpyAsync(g.st, &h, sizeof(h), cudaMemcpyHostToDevice, c.stream), "adjoint"))
     return RISM3D_CUDA_ERROR;
   if (!launch(g, nullptr, c.stream)) {
     cuda_ok(c, cudaGetLastError(), "adjoint solve launch");
@@ -585,8 +584,8 @@ int adjoint_one_launch(Context &c, const T *G, const T *w, T *xi, T *Lxi, T *ys,
   if (!cuda_ok(c, cudaMemcpyAsync(&h, g.st, sizeof(h), cudaMemcpyDeviceToHost, c.stream), "adjoint") ||
       !cuda_ok(c, cudaStreamSynchronize(c.stream), "adjoint"))
     return RISM3D_CUDA_ERROR;
+  if (h.bar != 0) { c.err = "adjoint: a device-side wait gave up"; return RISM3D_CUDA_ERROR; }
   if (h.done == 2) { c.err = "adjoint solve diverged"; return RISM3D_DIVERGED; }
-  if (h.done == 5 || h.fault) { c.err = "adjoint: a device-side wait gave up"; return RISM3D_CUDA_ERROR; }
   it = h.it;
   stalled = h.done == 4;
   done = true;

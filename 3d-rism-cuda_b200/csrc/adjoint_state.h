@@ -11,8 +11,9 @@ constexpr int kAdjDepth = 6;   // Anderson history of the adjoint solve
 
 struct AdjointState {
   int done;        // 0 running, 1 converged, 2 diverged, 3 step limit, 4 stalled
-                   // at the FP32 floor, 5 a barrier gave up
-  int fault;       // a block saw a barrier give up
+                   // at the FP32 floor
+  unsigned bar;    // arrival count of the barriers: zero again once every block
+                   // has left, else a wait gave up
   int it, ns, slot, since_best;
   double best, bnorm;
   double gram[kAdjDepth * kAdjDepth];

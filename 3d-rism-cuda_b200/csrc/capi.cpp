@@ -324,6 +324,10 @@ int context_init(Context &c, const rism3d_params *p, int nb, std::string &err) {
   // RISM3D_HOST_LOOP=1: drive iterations from the host (one graph launch per
   // iteration) instead of the device-side loop, e.g. for per-launch profiling
   if (const char *e = getenv("RISM3D_HOST_LOOP")) c.no_device_loop = e[0] == '1';
+  // RISM3D_STAGE_DELAY=ns: blocks of a whole-phase launch sleep up to this long
+  // before each stage (debugging; results must not depend on it)
+  if (const char *e = getenv("RISM3D_STAGE_DELAY"))
+    c.stage_delay = (unsigned)std::min(std::max(atoi(e), 0), 1000000);
   long long nbk = (c.n + 255) / 256;
   c.nred_blocks = (int)(nbk < 148 * 8 ? nbk : 148 * 8);
   ok = ok && cuda_ok(c, cudaMalloc(&c.d_part, sizeof(double) * 64 * c.nred_blocks * nb), "alloc partials") &&

@@ -809,10 +809,24 @@ __global__ void __launch_bounds__(ZShape<T, N, V>::TH, (ZShape<T, N, V>::MINB)) 
 // arrays are only ever touched by the SM that wrote them; the transform
 // buffer, the exchange planes and the sums go through L2.
 //
-// Arrival count of one solute's blocks, with a bound on the wait: false when
-// the other blocks never came (the caller reports it and returns).
+// Debugging aid (RISM3D_STAGE_DELAY): a block sleeps up to `delay` ns before a
+// stage, another time in each block and stage, so that results which depend on
+// the blocks' relative speed show.
+__device__ __forceinline__ void stage_delay(unsigned delay, unsigned salt) {
+  const unsigned h = (blockIdx.x * 2654435761u) ^ (salt * 2246822519u) ^ (blockIdx.y * 40503u);
+  __nanosleep((h >> 8) % delay);
+}
+
+// The arrival count of one solute's blocks is zero at every launch: the last
+// block to leave the kernel (leave_barrier) clears it, and after a wait that
+// gave up the host side does.  A launch on a count left over from another
+// would run through every barrier without waiting.
+//
+// Arrival and wait, with a bound on the wait: false when the other blocks
+// never came (the caller leaves without counting itself out, which is how the
+// host side learns of it).
 constexpr unsigned kBarrierPolls = 1u << 24;
-__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned target) {
+__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned target, unsigned delay) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -822,9 +836,17 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned target) {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
     } while ((int)(v - target) < 0 && ++polls < kBarrierPolls);   // the count may wrap
     ok = (int)(v - target) >= 0;
+    if (delay) stage_delay(delay, target);
   }
   __syncthreads();
   return ok != 0;
+}
+
+// One thread of each block, after its last barrier (`target`, 0 before the
+// first): the last of the nblk blocks, which no other polls any more, clears
+// the count.
+__device__ __forceinline__ void leave_barrier(unsigned *bar, unsigned target, unsigned nblk) {
+  if (atomicAdd(bar, 1u) == target + nblk - 1u) atomicExch(bar, 0u);
 }
 
 // byte offset of the tables: after the largest of the stages' exchanges
@@ -854,29 +876,30 @@ __global__ void __launch_bounds__(Lines<N>::TH, (Lines<N>::template minp<T, V>()
   const unsigned nblk = gridDim.x;
   unsigned target = 0;
   bool ok = true;
+  if (a.delay && threadIdx.x == 0) stage_delay(a.delay, target);
+  __syncthreads();
   while (!ss.done) {
     planes_a<T, N, V, REF, WIDE>(a, &ss, sm, tw, roots, hnc);
-    if (!(ok = grid_barrier(bar, target += nblk))) break;
+    if (!(ok = grid_barrier(bar, target += nblk, a.delay))) break;
 #pragma unroll 1
     for (int tile = blockIdx.x; tile < ZShape<T, N, V>::TILES; tile += nblk) {
       zline_tile<T, N, V, WIDE, true>(a, sm, roots, N, N, tile);
       __syncthreads();
     }
-    if (!(ok = grid_barrier(bar, target += nblk))) break;
+    if (!(ok = grid_barrier(bar, target += nblk, a.delay))) break;
     planes_r<T, N, V, REF, WIDE>(a, &ss, sm, tw, roots, hnc);
-    if (!(ok = grid_barrier(bar, target += nblk))) break;
+    if (!(ok = grid_barrier(bar, target += nblk, a.delay))) break;
     finalize_block(&ss, a.part, (int)nblk, (double)a.n * V, blockIdx.x == 0 ? a.hist : nullptr,
                    a.hist_cap);
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    if (!ok) a.st->fault = 1;
     if (blockIdx.x == 0) {
-      if (!ok) ss.fault = 1;
       if (!ok) ss.done = 2;
       ss.after_done = 1;
       *a.st = ss;
     }
+    if (ok) leave_barrier(bar, target, nblk);
   }
 }
 

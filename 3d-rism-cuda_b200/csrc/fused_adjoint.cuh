@@ -311,29 +311,30 @@ __global__ void __launch_bounds__(Lines<N>::TH, (Lines<N>::template minp<T, V>()
   for (int i = threadIdx.x; i < N; i += blockDim.x) roots[i] = g.it.roots[i];
   if (threadIdx.x == 0) s = *g.st;
   __syncthreads();
-  const unsigned nblk = gridDim.x;
-  unsigned target = 0;
+  const unsigned nblk = gridDim.x, delay = g.it.delay;
+  unsigned *bar = &g.st->bar, target = 0;
   bool ok = true;
+  if (delay && threadIdx.x == 0) stage_delay(delay, target);
+  __syncthreads();
   while (!s.done) {
     adjoint_forward<T, N, V>(g, &s, sm, tw, roots);
-    if (!(ok = grid_barrier(g.it.bar, target += nblk))) break;
+    if (!(ok = grid_barrier(bar, target += nblk, delay))) break;
 #pragma unroll 1
     for (int tile = blockIdx.x; tile < ZShape<T, N, V>::TILES; tile += nblk) {
       zline_tile<T, N, V, false, true>(g.it, sm, roots, N, N, tile);
       __syncthreads();
     }
-    if (!(ok = grid_barrier(g.it.bar, target += nblk))) break;
+    if (!(ok = grid_barrier(bar, target += nblk, delay))) break;
     adjoint_residual<T, N, V>(g, &s, sm, tw, roots);
-    if (!(ok = grid_barrier(g.it.bar, target += nblk))) break;
+    if (!(ok = grid_barrier(bar, target += nblk, delay))) break;
     adjoint_finalize(&s, g.part, (int)nblk, g.tol, g.maxit, sizeof(T) == 4);
   }
   if (threadIdx.x == 0) {
     if (blockIdx.x == 0) {
-      if (!ok) s.done = 5;
-      *g.st = s;
-    } else if (!ok) {
-      g.st->fault = 1;
+      g.st->done = s.done;
+      g.st->it = s.it;
     }
+    if (ok) leave_barrier(bar, target, nblk);
   }
 }
 

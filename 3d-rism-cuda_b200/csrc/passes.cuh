@@ -50,6 +50,7 @@ struct IterArgs {
   int nb;                   // solutes
   unsigned *gcount;         // solutes whose plane R is done (nb > 1)
   unsigned *bar;            // arrival counts of a whole-phase launch [nb]
+  unsigned delay;           // longest sleep of a block before a stage (ns; debugging)
 };
 
 namespace {

@@ -48,8 +48,9 @@ struct DevState {
   int restart_next;  // (solute 0) FP64 phase starts a fresh AN2 history
   int rotate;      // 1: plane R's residual slots are renamed, not copied:
   int rp[3];       // slots of history entries 0 and 1, and the free one
-  int fault;       // a device-side wait gave up (a bulk or tile copy never
-                   // arrived): the loop was stopped and the solve reports it
+  int fault;       // a device-side wait gave up (a bulk or tile copy or a
+                   // barrier's other blocks never came): the loop was stopped
+                   // and the solve reports it
   double best;     // best rms of this run (stagnation watch)
   double conv;
   double m, mp;    // AN2 mixing factor and bias
@@ -259,6 +260,8 @@ struct Context {
   // node): one launch runs a whole phase; null when the driver refuses it
   cudaGraphExec_t loop64 = nullptr, loop32 = nullptr, loop32r = nullptr;
   bool no_device_loop = false;
+  unsigned stage_delay = 0;     // RISM3D_STAGE_DELAY: longest sleep of a block before
+                                // a stage of a whole-phase launch (ns; debugging)
   double *d_hist = nullptr;     // per-iteration rms (verbose single solves)
   int hist_cap = 0;
   unsigned *d_bar = nullptr;    // arrival counts of whole-phase launches [nb]

@@ -1854,7 +1854,6 @@ void launch_fused(Context &c, const IterArgs<T> &a, bool ref, int which = -1) {
   const fused::Vtable<T> tab = fused::table<T>(c.nx, c.natv);
   IterArgs<T> ar = a;
   ar.nblocks = (which == 4 ? f.cp[ref ? 1 : 0] : f.cr[ref ? 1 : 0]) * f.nc;
-  if (which == 4) cudaMemsetAsync(c.d_bar, 0, sizeof(unsigned) * c.nb, c.stream);
   for (int k = 0; k < 5; ++k)
     if (which < 0 ? k < 3 : which == k) tab.launch(f, k, ref, hnc, c.nb, ar, c.stream);
 }
@@ -2044,8 +2043,11 @@ __global__ void k_phase_begin(DevState *st, int nb, int kind, double conv, int m
   }
 }
 
-// End of a phase: step counters, and the flags the next phases read.
-__global__ void k_phase_end(DevState *st, int nb, int kind, int fp32, int again, int maxstep) {
+// End of a phase: step counters, and the flags the next phases read.  bar: the
+// arrival counts of a whole-phase launch; one that is not back at zero means
+// that a block's wait gave up.
+__global__ void k_phase_end(DevState *st, int nb, int kind, int fp32, int again, int maxstep,
+                            unsigned *bar) {
   __shared__ int any_div;
   if (threadIdx.x == 0) any_div = 0;
   __syncthreads();
@@ -2057,6 +2059,10 @@ __global__ void k_phase_end(DevState *st, int nb, int kind, int fp32, int again,
     s.stage_iter += steps;
     s.total_iter += steps;
     if (fp32) s.total32 += steps;
+    if (bar && bar[b]) {
+      s.fault = 1;
+      bar[b] = 0u;
+    }
     if (s.done == 2) atomicOr(&any_div, 1);
   }
   __syncthreads();
@@ -2111,6 +2117,7 @@ void set_fused_args(Context &c, IterArgs<T> &a) {
   a.xo = (const T *)(sizeof(T) == 8 ? (void *)c.d_xo : (void *)c.d_xo32);
   a.gcount = c.d_count + c.nb;
   a.bar = c.d_bar;
+  a.delay = c.stage_delay;
 }
 
 // One phase: the device-side loop graph when available (no host sync), else
@@ -2222,7 +2229,7 @@ int run_phase(Context &c, cufftHandle plan, T *t, T *U, T *Y, T *RP,
     c.launches += 2;
   }
   k_phase_end<<<1, 128, 0, c.stream>>>(c.d_state, nb, kind, sizeof(T) == 4 ? 1 : 0,
-                                       again ? 1 : 0, c.prm.maxstep);
+                                       again ? 1 : 0, c.prm.maxstep, one ? c.d_bar : nullptr);
   c.launches += 1;
   // progress lines of the reference (iterate.cu:63), from the device record
   if (status == RISM3D_OK && c.prm.verbose && nb == 1 && c.d_hist) {
@@ -2261,7 +2268,8 @@ int refine_base(Context &c, bool again) {
     return RISM3D_CUFFT_ERROR;
   k_refine_base<V, CLOS><<<bb, kThreads, 0, c.stream>>>(a, c.f_R0, c.f_x0, c.f_t, c.f_Y,
                                                          again ? 1 : 0);
-  k_phase_end<<<1, 128, 0, c.stream>>>(c.d_state, nb, kBase64, 0, again ? 1 : 0, c.prm.maxstep);
+  k_phase_end<<<1, 128, 0, c.stream>>>(c.d_state, nb, kBase64, 0, again ? 1 : 0, c.prm.maxstep,
+                                       nullptr);
   c.launches += 6;
   return cuda_ok(c, cudaGetLastError(), "refine base") ? RISM3D_OK : RISM3D_CUDA_ERROR;
 }
@@ -2417,7 +2425,7 @@ int solve_v(Context &c, int chargeup) {
   bodies = fs[0].bodies;
   for (const DevState &x : fs)
     if (x.fault) {
-      c.err = "a device-side wait gave up: a bulk or tile copy never arrived";
+      c.err = "a device-side wait gave up: a copy or a barrier's other blocks never came";
       status = RISM3D_CUDA_ERROR;
     }
   c.launches += (c.split64 || c.split32 ? 5 : c.fu64.on ? 3 : 4) * bodies;
