@@ -584,6 +584,7 @@ int adjoint_one_launch(Context &c, const T *G, const T *w, T *xi, T *Lxi, T *ys,
   if (!cuda_ok(c, cudaMemcpyAsync(&h, g.st, sizeof(h), cudaMemcpyDeviceToHost, c.stream), "adjoint") ||
       !cuda_ok(c, cudaStreamSynchronize(c.stream), "adjoint"))
     return RISM3D_CUDA_ERROR;
+  if (h.done == 5) { c.err = "adjoint: launched without its clusters"; return RISM3D_CUDA_ERROR; }
   if (h.bar != 0) { c.err = "adjoint: a device-side wait gave up"; return RISM3D_CUDA_ERROR; }
   if (h.done == 2) { c.err = "adjoint solve diverged"; return RISM3D_DIVERGED; }
   it = h.it;

@@ -11,7 +11,7 @@ constexpr int kAdjDepth = 6;   // Anderson history of the adjoint solve
 
 struct AdjointState {
   int done;        // 0 running, 1 converged, 2 diverged, 3 step limit, 4 stalled
-                   // at the FP32 floor
+                   // at the FP32 floor, 5 launched without its clusters
   unsigned bar;    // arrival count of the barriers: zero again once every block
                    // has left, else a wait gave up
   int it, ns, slot, since_best;

@@ -132,6 +132,11 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;\n"
                ::: "memory");
 }
+__device__ __forceinline__ unsigned cluster_ctas() {
+  unsigned n;
+  asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
+  return n;
+}
 // Threads that share a row: the R2 consecutive threads of stage 1 also do its
 // R1 stage-2 items (s = t, t + R2, ...), so that where R2 divides a warp the
 // row exchange needs no block barrier.
@@ -392,8 +397,8 @@ __device__ __forceinline__ void planes_a(const IterArgs<T> &a, const DevState *s
 }
 
 template <typename T, int N, int V, bool REF>
-__global__ void __launch_bounds__(Lines<N>::TH, (Lines<N>::template minb<T>()))
-    k_plane_a(IterArgs<T> a0, bool hnc) {
+__global__ void __cluster_dims__(Lines<N>::NC, 1, 1)
+    __launch_bounds__(Lines<N>::TH, (Lines<N>::template minb<T>())) k_plane_a(IterArgs<T> a0, bool hnc) {
   extern __shared__ __align__(16) unsigned char fused_sm[];
   const IterArgs<T> a = solute_view<T, V>(a0);
   if (a.st->done) return;
@@ -553,8 +558,8 @@ __device__ __forceinline__ void finish_cycle(const IterArgs<T> &a0, const IterAr
 }
 
 template <typename T, int N, int V, bool REF>
-__global__ void __launch_bounds__(Lines<N>::TH, (Lines<N>::template minb<T>()))
-    k_plane_r(IterArgs<T> a0, bool hnc) {
+__global__ void __cluster_dims__(Lines<N>::NC, 1, 1)
+    __launch_bounds__(Lines<N>::TH, (Lines<N>::template minb<T>())) k_plane_r(IterArgs<T> a0, bool hnc) {
   extern __shared__ __align__(16) unsigned char fused_sm[];
   const IterArgs<T> a = solute_view<T, V>(a0);
   DevState *st = a.st;
@@ -609,7 +614,8 @@ __device__ __forceinline__ void final_row(const IterArgs<T> &a, const CxT<T> *li
 }
 
 template <typename T, int N, int V, bool REF>
-__global__ void __launch_bounds__(Lines<N>::TH) k_plane_final(IterArgs<T> a0, bool hnc) {
+__global__ void __cluster_dims__(Lines<N>::NC, 1, 1) __launch_bounds__(Lines<N>::TH)
+    k_plane_final(IterArgs<T> a0, bool hnc) {
   typedef CxT<T> C;
   using L = Lines<N>;
   constexpr int R2 = L::R2, LB = L::LB, P = (V + 1) / 2;
@@ -857,14 +863,22 @@ template <typename T, int N, int V> __host__ __device__ constexpr size_t tables_
 }
 
 template <typename T, int N, int V, bool REF>
-__global__ void __launch_bounds__(Lines<N>::TH, (Lines<N>::template minp<T, V>()))
-    k_phase(IterArgs<T> a0, bool hnc) {
+__global__ void __cluster_dims__(Lines<N>::NC, 1, 1)
+    __launch_bounds__(Lines<N>::TH, (Lines<N>::template minp<T, V>())) k_phase(IterArgs<T> a0, bool hnc) {
   typedef CxT<T> C;
   extern __shared__ __align__(16) unsigned char fused_sm[];
   constexpr bool WIDE = Lines<N>::template minp<T, V>() == 1 && Lines<N>::template minb<T>() > 1;
   __shared__ DevState ss;
   C *sm = reinterpret_cast<C *>(fused_sm);
   const IterArgs<T> a = solute_view<T, V>(a0);
+  if (cluster_ctas() != Lines<N>::NC) {            // see the launches
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      a.st->fault = 2;
+      a.st->done = 2;
+      a.st->after_done = 1;
+    }
+    return;
+  }
   // the phase and root tables, read at every stage, stay in shared memory
   // (every barrier's acquire empties L1)
   C *tw = reinterpret_cast<C *>(fused_sm + tables_at<T, N, V>()), *roots = tw + 3 * N;
@@ -904,6 +918,11 @@ __global__ void __launch_bounds__(Lines<N>::TH, (Lines<N>::template minp<T, V>()
 }
 
 // ---------------------------------------------------------------- launches
+// The plane kernels carry their cluster size (__cluster_dims__), not the
+// launch: ncu replays a cooperative launch without its attributes, and with
+// clusters of one CTA plane_sync orders nothing -- a 32^3 solve then ran its
+// 10000 steps without converging.  The two whole-phase kernels check it.
+//
 // Clusters of a plane kernel: one per plane, at most what is resident at once
 // (a cluster then walks its planes with one scratch plane).
 template <typename K>
@@ -913,11 +932,6 @@ int plane_clusters(K kernel, int nc, int threads, size_t smem, int planes) {
   cfg.gridDim = dim3(nc);
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim = {(unsigned)nc, 1, 1};
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
   if (cudaOccupancyMaxActiveClusters(&num, kernel, &cfg) != cudaSuccess || num < 1) {
     cudaGetLastError();
     return 0;
@@ -933,18 +947,11 @@ cudaError_t launch_plane(K kernel, int nclusters, int nc, int nb, int threads, s
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[2] = {};
-  int na = 0;
-  if (nc > 1) {
-    at[na].id = cudaLaunchAttributeClusterDimension;
-    at[na++].val.clusterDim = {(unsigned)nc, 1, 1};
-  }
-  if (cooperative) {
-    at[na].id = cudaLaunchAttributeCooperative;
-    at[na++].val.cooperative = 1;
-  }
-  cfg.attrs = at;
-  cfg.numAttrs = na;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeCooperative;
+  at.val.cooperative = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = cooperative ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 

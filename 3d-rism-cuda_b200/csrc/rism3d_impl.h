@@ -49,8 +49,9 @@ struct DevState {
   int rotate;      // 1: plane R's residual slots are renamed, not copied:
   int rp[3];       // slots of history entries 0 and 1, and the free one
   int fault;       // a device-side wait gave up (a bulk or tile copy or a
-                   // barrier's other blocks never came): the loop was stopped
-                   // and the solve reports it
+                   // barrier's other blocks never came), or 2: the kernel ran
+                   // without its clusters; the loop was stopped and the solve
+                   // reports it
   double best;     // best rms of this run (stagnation watch)
   double conv;
   double m, mp;    // AN2 mixing factor and bias

@@ -2425,7 +2425,8 @@ int solve_v(Context &c, int chargeup) {
   bodies = fs[0].bodies;
   for (const DevState &x : fs)
     if (x.fault) {
-      c.err = "a device-side wait gave up: a copy or a barrier's other blocks never came";
+      c.err = x.fault == 2 ? "a whole-phase kernel was launched without its clusters"
+                           : "a device-side wait gave up: a copy or a barrier's other blocks never came";
       status = RISM3D_CUDA_ERROR;
     }
   c.launches += (c.split64 || c.split32 ? 5 : c.fu64.on ? 3 : 4) * bodies;
