@@ -1826,10 +1826,11 @@ void launch_iteration_dm(Context &c, const IterArgs<float> &a, cufftHandle plan)
   k_pass_r_dm<V, CLOS><<<a.nblocks, kThreads, 0, c.stream>>>(a, c.dm_depth);
 }
 
-// One iteration (or with which >= 0 one of its kernels) in the three-kernel
-// form (fused.cuh).
+// One iteration (or with which >= 0 one of its kernels) in the folded form
+// (fused.cuh).  The launches report their errors here, once: the callers pass
+// them on.
 template <typename T>
-void launch_split(Context &c, const IterArgs<T> &a, bool ref, int which) {
+[[nodiscard]] cudaError_t launch_split(Context &c, const IterArgs<T> &a, bool ref, int which) {
   int lines = 1;
   const fused::SplitRun<T> run[3] = {fused::split_table<T>(c.nx, c.natv, &lines),
                                      fused::split_table<T>(c.ny, c.natv, nullptr),
@@ -1838,36 +1839,37 @@ void launch_split(Context &c, const IterArgs<T> &a, bool ref, int which) {
   const int hnc = c.prm.closure == RISM3D_HNC;
   IterArgs<T> ar = a;
   ar.nblocks = (int)(((long long)c.ny * c.nz * ((c.natv + 1) / 2) + lines - 1) / lines);
-  if (which == 3) run[0](5, 0, ref, hnc, c.nb, ar, c.stream);
-  else
-    for (int k = 0; k < 5; ++k) run[axis[k]](k, axis[k], ref, hnc, c.nb, ar, c.stream);
+  cudaError_t e = cudaSuccess;
+  if (which == 3) return run[0](5, 0, ref, hnc, c.nb, ar, c.stream);
+  for (int k = 0; k < 5 && e == cudaSuccess; ++k)
+    e = run[axis[k]](k, axis[k], ref, hnc, c.nb, ar, c.stream);
+  return e;
 }
 
 template <typename T>
-void launch_fused(Context &c, const IterArgs<T> &a, bool ref, int which = -1) {
-  if (sizeof(T) == 8 ? c.split64 : c.split32) {  // which: -1 a cycle, 3 the pass after the loop
-    launch_split<T>(c, a, ref, which);
-    return;
-  }
+[[nodiscard]] cudaError_t launch_fused(Context &c, const IterArgs<T> &a, bool ref, int which = -1) {
+  cudaGetLastError();                            // an earlier call's error is not this launch's
+  if (sizeof(T) == 8 ? c.split64 : c.split32)    // which: -1 a cycle, 3 the pass after the loop
+    return launch_split<T>(c, a, ref, which);
   const FusedPlan &f = sizeof(T) == 8 ? c.fu64 : c.fu32;
   const int hnc = c.prm.closure == RISM3D_HNC;
   const fused::Vtable<T> tab = fused::table<T>(c.nx, c.natv);
   IterArgs<T> ar = a;
   ar.nblocks = (which == 4 ? f.cp[ref ? 1 : 0] : f.cr[ref ? 1 : 0]) * f.nc;
-  for (int k = 0; k < 5; ++k)
-    if (which < 0 ? k < 3 : which == k) tab.launch(f, k, ref, hnc, c.nb, ar, c.stream);
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < 5 && e == cudaSuccess; ++k)
+    if (which < 0 ? k < 3 : which == k) e = tab.launch(f, k, ref, hnc, c.nb, ar, c.stream);
+  return e;
 }
 
 template <typename T, int V, int CLOS, bool REF>
-void launch_iteration(Context &c, const IterArgs<T> &a, cufftHandle plan) {
-  if (a.RPx) {
-    launch_fused<T>(c, a, REF);
-    return;
-  }
+[[nodiscard]] cudaError_t launch_iteration(Context &c, const IterArgs<T> &a, cufftHandle plan) {
+  if (a.RPx) return launch_fused<T>(c, a, REF);
+  cudaGetLastError();
   if constexpr (sizeof(T) == 4 && !REF) {
     if (c.dm_depth && (const void *)a.Y == (const void *)c.f_Ydm) {
       launch_iteration_dm<V, CLOS>(c, a, plan);
-      return;
+      return cudaGetLastError();
     }
   }
   // the fused-axis passes run the plain FP32 bulk; the refinement form
@@ -1878,7 +1880,7 @@ void launch_iteration(Context &c, const IterArgs<T> &a, cufftHandle plan) {
     if (c.xfused) {
       if (c.nx == 256) launch_iteration_x<V, CLOS, REF, 16>(c, a);
       else launch_iteration_x<V, CLOS, REF, 8>(c, a);
-      return;
+      return cudaGetLastError();
     }
   }
   const dim3 ba(wave_blocks(k_pass_a<T, V, CLOS, REF>, a.n, c.nb), c.nb),
@@ -1909,6 +1911,7 @@ void launch_iteration(Context &c, const IterArgs<T> &a, cufftHandle plan) {
   launch_pass_r<T, V, CLOS, REF>(c, a);
   (void)sizeof(C);
   (void)br;
+  return cudaGetLastError();
 }
 
 template <typename T>
@@ -1942,9 +1945,10 @@ cudaGraphExec_t capture(Context &c, const IterArgs<T> &a, cufftHandle plan) {
     cudaGetLastError();
     return nullptr;
   }
-  launch_iteration<T, V, CLOS, REF>(c, a, plan);
+  const cudaError_t el = launch_iteration<T, V, CLOS, REF>(c, a, plan);
   cudaError_t e = cudaStreamEndCapture(c.stream, &g);
-  if (e != cudaSuccess || !g) {
+  if (el != cudaSuccess || e != cudaSuccess || !g) {
+    if (g) cudaGraphDestroy(g);
     cudaGetLastError();
     return nullptr;
   }
@@ -1990,13 +1994,15 @@ cudaGraphExec_t capture_loop(Context &c, const IterArgs<T> &a, cufftHandle plan)
         IterArgs<T> al = a;
         al.cond = h;
         al.loop = 1;
-        launch_iteration<T, V, CLOS, REF>(c, al, plan);
+        ok = launch_iteration<T, V, CLOS, REF>(c, al, plan) == cudaSuccess;
       } else {
-        launch_iteration<T, V, CLOS, REF>(c, a, plan);
+        ok = launch_iteration<T, V, CLOS, REF>(c, a, plan) == cudaSuccess;
         k_loop_cond<<<1, 32, 0, c.stream>>>(h, a.st, c.nb);
+        ok = ok && cudaGetLastError() == cudaSuccess;
       }
+      // a body without its loop test would never end
       cudaGraph_t out = nullptr;
-      ok = cudaStreamEndCapture(c.stream, &out) == cudaSuccess;
+      ok = cudaStreamEndCapture(c.stream, &out) == cudaSuccess && ok;
     }
   }
   if (ok) ok = cudaGraphInstantiate(&x, g, 0) == cudaSuccess;
@@ -2161,12 +2167,9 @@ int run_phase(Context &c, cufftHandle plan, T *t, T *U, T *Y, T *RP,
       cudaEventCreate(&t1);
       cudaEventRecord(t0, c.stream);
     }
-    if (one) {
-      launch_fused<T>(c, a, REF, 4);
-      c.launches += 1;
-    }
-    if (!cuda_ok(c, one ? cudaGetLastError() : cudaGraphLaunch(lx, c.stream), "phase launch"))
+    if (!cuda_ok(c, one ? launch_fused<T>(c, a, REF, 4) : cudaGraphLaunch(lx, c.stream), "phase launch"))
       return RISM3D_CUDA_ERROR;
+    if (one) c.launches += 1;
     if (trace) {
       cudaEventRecord(t1, c.stream);
       DevState s0;
@@ -2190,8 +2193,11 @@ int run_phase(Context &c, cufftHandle plan, T *t, T *U, T *Y, T *RP,
     int launched = 0;
     bool stop = false;
     while (!stop) {
-      if (gx) cudaGraphLaunch(gx, c.stream);
-      else launch_iteration<T, V, CLOS, REF>(c, a, plan);
+      if (!cuda_ok(c, gx ? cudaGraphLaunch(gx, c.stream)
+                         : launch_iteration<T, V, CLOS, REF>(c, a, plan), "iteration launch")) {
+        status = RISM3D_CUDA_ERROR;
+        break;
+      }
       c.launches += 3;
       cudaMemcpyAsync(&c.h_state[(size_t)(launched % kRing) * nb], c.d_state, sizeof(DevState) * nb,
                       cudaMemcpyDeviceToHost, c.stream);
@@ -2214,16 +2220,18 @@ int run_phase(Context &c, cufftHandle plan, T *t, T *U, T *Y, T *RP,
     }
     // drain: one more iteration guarantees the snapshot pass ran
     if (status == RISM3D_OK) {
-      if (gx) cudaGraphLaunch(gx, c.stream);
-      else launch_iteration<T, V, CLOS, REF>(c, a, plan);
+      if (!cuda_ok(c, gx ? cudaGraphLaunch(gx, c.stream)
+                         : launch_iteration<T, V, CLOS, REF>(c, a, plan), "iteration launch"))
+        status = RISM3D_CUDA_ERROR;
       c.launches += 3;
     }
     for (int i = 0; i < kRing; ++i) cudaEventDestroy(ev[i]);
+    if (status != RISM3D_OK) return status;
   }
   // the loop's bodies (4 launches each: passes A, K, R and the loop test)
   // are counted from the device record at the end of the solve
   if (fused) {
-    launch_fused<T>(c, a, REF, 3);
+    if (!cuda_ok(c, launch_fused<T>(c, a, REF, 3), "pass after the loop")) return RISM3D_CUDA_ERROR;
     k_rp_order<T, V><<<dim3(grid_blocks((long long)V * c.n), nb), kThreads, 0, c.stream>>>(
         (long long)V * c.n, a.st, a.RP, a.RPx);
     c.launches += 2;
@@ -2499,10 +2507,12 @@ int time_kernel_t(Context &c, int which, int reps, double *ms) {
             bar = wave_blocks(k_pass_a<T, V, CLOS, true>, a.n, 1),
             bk = wave_blocks(k_kspace<T, V>, a.n / 2, 1);
   cudaEventRecord(e0, c.stream);
+  cudaError_t el = cudaSuccess;                  // of a launch
   bool fused_done = false;
   if (three) {                                   // plane A / z lines / plane R
     const bool ref = which == 13 || which == 15;
-    for (int r = 0; r < reps; ++r) launch_fused<T>(c, a, ref, ref ? which - 13 : which % 10);
+    for (int r = 0; r < reps && el == cudaSuccess; ++r)
+      el = launch_fused<T>(c, a, ref, ref ? which - 13 : which % 10);
     fused_done = true;
   }
   if constexpr (sizeof(T) == 4 && V <= 2) {
@@ -2551,7 +2561,7 @@ int time_kernel_t(Context &c, int which, int reps, double *ms) {
   stream_copy(c, c.d_state, &saved, sizeof(DevState), cudaMemcpyHostToDevice);
   c.solved = false;
   c.have_forces = false;
-  if (!cuda_ok(c, e, "time_kernel")) return RISM3D_CUDA_ERROR;
+  if (!cuda_ok(c, el == cudaSuccess ? e : el, "time_kernel")) return RISM3D_CUDA_ERROR;
   *ms = t / reps;
   return RISM3D_OK;
 }

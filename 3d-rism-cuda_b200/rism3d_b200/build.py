@@ -33,6 +33,7 @@ def _ccbin():
 
 def _flags():
     return (_ccbin() + ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
+                               "-Xcompiler", "-Werror=unused-result",
                                "-I" + os.path.join(ROOT, "include"), "-I" + CSRC])
 
 
