@@ -439,10 +439,23 @@ int blocks_for(long long work) {
 struct Scratch {
   std::vector<void *> ptrs;
   Context &c;
-  explicit Scratch(Context &cc) : c(cc) {}
+  bool must;                   // the call cannot do without: the folded iteration's
+                               // memory is given up for it
+  Scratch(Context &cc, bool need) : c(cc), must(need) {}
   template <typename T> T *get(size_t count) {
     void *p = nullptr;
-    if (pool_alloc(c, &p, sizeof(T) * count) != cudaSuccess) return nullptr;
+    cudaError_t e = pool_alloc(c, &p, sizeof(T) * count);
+    if (e != cudaSuccess) {                      // without what the pool holds unused
+      cudaStreamSynchronize(c.stream);
+      cudaMemPoolTrimTo(c.pool, 0);
+      e = pool_alloc(c, &p, sizeof(T) * count);
+    }
+    if (e != cudaSuccess && must && c.d_fused) {
+      drop_fused_iteration(c);
+      e = pool_alloc(c, &p, sizeof(T) * count);
+    }
+    cudaGetLastError();
+    if (e != cudaSuccess) return nullptr;
     ptrs.push_back(p);
     return (T *)p;
   }
@@ -544,15 +557,18 @@ template <> struct SolveTol<float> { static constexpr double tol = 2.0e-6; };
 
 // The whole Anderson solve as one launch (fused_adjoint.cuh): `done` is set
 // when it ran, with the steps taken; otherwise (no instantiation for the cell,
-// or not on this device) nothing has happened.
+// no room for its exchange planes, or not on this device)
+// nothing has happened.
 template <int V, typename T, typename CT>
 int adjoint_one_launch(Context &c, const T *G, const T *w, T *xi, T *Lxi, T *ys, T *rs,
                        double *part, const StageParams *sp0, CT *buf, double eta, double tol,
-                       int maxit, Scratch &S, bool &done, int &it, bool &stalled) {
+                       int maxit, bool &done, int &it, bool &stalled) {
   done = false;
+  Scratch S(c, false);                           // back in the pool for the back-projection
   if (!c.d_fused || !c.d_xs || c.nx != c.ny || c.nx != c.nz) return RISM3D_OK;   // cubic cells
   const fused::AdjointLaunch<T> launch = fused::adjoint_table<T>(c.nx, V);
   fused::AdjointArgs<T> g{};
+  g.max_blocks = kDotBlocks;
   int clusters = 0;
   if (!launch || !launch(g, &clusters, c.stream)) return RISM3D_OK;
   const size_t N = c.nx;
@@ -571,14 +587,14 @@ int adjoint_one_launch(Context &c, const T *G, const T *w, T *xi, T *Lxi, T *ys,
   h.best = 1e300;
   h.bnorm = -1.0;
   g.st = S.get<fused::AdjointState>(1);
-  if (!a.scr || !g.st) { c.err = "adjoint: out of device memory"; return RISM3D_CUDA_ERROR; }
+  if (!a.scr || !g.st) return RISM3D_OK;
   g.G = G; g.w = w; g.xi = xi; g.Lxi = Lxi; g.ys = ys; g.rs = rs; g.part = part;
   g.eta = eta; g.tol = tol; g.maxit = maxit;
   if (!cuda_ok(c, cudaMemcpyAsync(g.st, &h, sizeof(h), cudaMemcpyHostToDevice, c.stream), "adjoint"))
     return RISM3D_CUDA_ERROR;
   if (!launch(g, nullptr, c.stream)) {
-    cuda_ok(c, cudaGetLastError(), "adjoint solve launch");
-    return RISM3D_CUDA_ERROR;
+    cudaGetLastError();
+    return RISM3D_OK;
   }
   c.launches += 1;
   if (!cuda_ok(c, cudaMemcpyAsync(&h, g.st, sizeof(h), cudaMemcpyDeviceToHost, c.stream), "adjoint") ||
@@ -603,7 +619,7 @@ int adjoint_v(Context &c, double *dq, double *dsig, double *deps, double *dR) {
   const int P = (V + 1) / 2, gb = blocks_for(n), gt = blocks_for(tot);
   const int A = c.natom;
   constexpr bool F32 = sizeof(T) == 4;
-  Scratch S(c);
+  Scratch S(c, true);
   double *w64 = S.get<double>(tot), *tmp = S.get<double>(tot), *Om = S.get<double>(n);
   T *G = S.get<T>(tot), *xi = S.get<T>(tot), *Lxi = S.get<T>(tot);
   T *w = F32 ? S.get<T>(tot) : (T *)w64;
@@ -676,7 +692,7 @@ int adjoint_v(Context &c, double *dq, double *dsig, double *deps, double *dR) {
   bool stalled = false;
   // one launch where the cell has an instantiation, else driven from here
   bool one = false;
-  rc = adjoint_one_launch<V, T>(c, G, w, xi, Lxi, ys, rs, dpart, sp0, bufT, eta, tol, maxit, S,
+  rc = adjoint_one_launch<V, T>(c, G, w, xi, Lxi, ys, rs, dpart, sp0, bufT, eta, tol, maxit,
                                 one, it, stalled);
   if (rc != RISM3D_OK) return rc;
   for (; !one && it < maxit; ++it) {

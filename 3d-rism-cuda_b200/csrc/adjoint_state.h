@@ -27,6 +27,7 @@ struct AdjointArgs {
   T *xi, *Lxi;                 // [V][N]
   T *ys, *rs;                  // histories [kAdjDepth][V][N]
   double *part;                // dots of every block
+  int max_blocks;              // that it has room for
   AdjointState *st;
   double eta, tol;
   int maxit;

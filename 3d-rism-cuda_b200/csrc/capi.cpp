@@ -64,6 +64,23 @@ bool cufft_ok(Context &c, cufftResult r, const char *what) {
   return false;
 }
 
+void drop_graphs(Context &c) {
+  for (cudaGraphExec_t *g : {&c.graph64, &c.graph32, &c.graph32r, &c.loop64, &c.loop32, &c.loop32r}) {
+    if (*g) cudaGraphExecDestroy(*g);
+    *g = nullptr;
+  }
+}
+
+void drop_fused_iteration(Context &c) {
+  if (c.stream) cudaStreamSynchronize(c.stream);
+  drop_graphs(c);
+  if (c.d_fused) cudaFree(c.d_fused);
+  c.d_fused = nullptr;
+  c.d_RPx = nullptr; c.f_RPx = nullptr; c.d_scr = nullptr; c.d_roots = nullptr; c.f_roots = nullptr;
+  c.d_bar = nullptr; c.d_xo = nullptr; c.d_xo32 = nullptr; c.split64 = c.split32 = false;
+  c.fu64.on = c.fu32.on = false;
+}
+
 void free_device(Context &c) {
   void *ptrs[] = {c.d_u, c.d_e, c.d_fr, c.d_fkh, c.d_atoms, c.d_tw, c.d_twf,
                   c.d_U, c.d_t, c.d_Y, c.d_RP, c.d_buf, c.d_h, c.d_g,
@@ -86,14 +103,6 @@ void free_device(Context &c) {
   c.d_atom_off = c.d_atom_cnt = nullptr;
   if (c.h_state) cudaFreeHost(c.h_state);
   c.h_state = nullptr;
-  if (c.graph64) cudaGraphExecDestroy(c.graph64);
-  if (c.graph32) cudaGraphExecDestroy(c.graph32);
-  if (c.graph32r) cudaGraphExecDestroy(c.graph32r);
-  c.graph64 = c.graph32 = c.graph32r = nullptr;
-  for (cudaGraphExec_t *g : {&c.loop64, &c.loop32, &c.loop32r}) {
-    if (*g) cudaGraphExecDestroy(*g);
-    *g = nullptr;
-  }
   if (c.d_hist) cudaFree(c.d_hist);
   c.d_hist = nullptr;
   c.hist_cap = 0;
@@ -112,11 +121,7 @@ void free_device(Context &c) {
   c.d_fkt = nullptr;
   delete c.ky_map;
   c.ky_map = nullptr;
-  if (c.d_fused) cudaFree(c.d_fused);
-  c.d_fused = nullptr;
-  c.d_RPx = nullptr; c.f_RPx = nullptr; c.d_scr = nullptr; c.d_roots = nullptr; c.f_roots = nullptr;
-  c.d_bar = nullptr; c.d_xo = nullptr; c.d_xo32 = nullptr; c.split64 = c.split32 = false;
-  c.fu64.on = c.fu32.on = false;
+  drop_fused_iteration(c);
   if (c.plan64) cufftDestroy(c.plan64);
   if (c.plan32) cufftDestroy(c.plan32);
   if (c.plan1) cufftDestroy(c.plan1);

@@ -352,7 +352,9 @@ bool adjoint_launch(const AdjointArgs<T> &g, int *clusters, cudaStream_t st) {
     cudaGetLastError();
     return false;
   }
-  const int ncl = plane_clusters(k_adjoint_solve<T, N, V>, L::NC, L::TH, s, N * ((V + 1) / 2));
+  const int planes = N * ((V + 1) / 2), room = g.max_blocks / L::NC;
+  const int ncl = plane_clusters(k_adjoint_solve<T, N, V>, L::NC, L::TH, s,
+                                 planes < room ? planes : room);
   if (ncl < 1) return false;
   if (clusters) {                                  // asked for the count only
     *clusters = ncl;

@@ -314,6 +314,9 @@ int upload_chi(Context &c);                       // solver.cu
 // decide on and set up the fused-axis FP32 passes (plan, roots, limits)
 int setup_fused_axes(Context &c);                 // solver.cu
 int setup_fused_iteration(Context &c);            // solver.cu: three-kernel iteration
+void drop_graphs(Context &c);                     // capi.cpp: the captured iterations
+// gives back what the folded iteration holds; the passes take over
+void drop_fused_iteration(Context &c);            // capi.cpp
 int setup_kspace_tma(Context &c);                 // solver.cu: TMA fused pass K
 int fused_fk_columns(Context &c);                 // solver.cu: fk copy for it
 int setup_pipe_r(Context &c);                     // solver.cu: pipelined pass R

@@ -2731,8 +2731,10 @@ int setup_fused_iteration(Context &c) {
                r32 = mixed ? up(sizeof(float) * vn) : 0, sc = up(scr), o64 = up(sizeof(double) * oct),
                o32 = mixed ? up(sizeof(float) * oct) : 0;
   unsigned char *base = nullptr;
-  if (!cuda_ok(c, cudaMalloc(&base, h + r64 + r32 + sc + o64 + o32), "alloc folded iteration"))
-    return RISM3D_CUDA_ERROR;
+  if (cudaMalloc(&base, h + r64 + r32 + sc + o64 + o32) != cudaSuccess) {
+    cudaGetLastError();                            // the passes need none of it
+    return RISM3D_OK;
+  }
   c.d_fused = base;
   if (!cuda_ok(c, stream_copy(c, base, head.data(), head.size(), cudaMemcpyHostToDevice), "copy roots"))
     return RISM3D_CUDA_ERROR;
@@ -2930,13 +2932,7 @@ int upload_chi(Context &c) {
       spline_coefficients(xp.data(), &c.xvv_host[((size_t)va * V + vb) * nt], nt,
                           &tab[(size_t)(va * V + vb) * 4], (size_t)V * V * 4);
   // the captured iteration graphs embed the table pointers
-  if (c.graph64) { cudaGraphExecDestroy(c.graph64); c.graph64 = nullptr; }
-  if (c.graph32) { cudaGraphExecDestroy(c.graph32); c.graph32 = nullptr; }
-  if (c.graph32r) { cudaGraphExecDestroy(c.graph32r); c.graph32r = nullptr; }
-  for (cudaGraphExec_t *g : {&c.loop64, &c.loop32, &c.loop32r}) {
-    if (*g) cudaGraphExecDestroy(*g);
-    *g = nullptr;
-  }
+  drop_graphs(c);
   // Cubic cells: evaluate the spline once per distinct |k|^2 (the sorted
   // unique-|k| table of initialize_g.cu:31-43, indexed directly).
   if (c.d_xs) { cudaFree(c.d_xs); c.d_xs = nullptr; c.nxs = 0; }
