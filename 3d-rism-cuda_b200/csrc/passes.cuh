@@ -47,6 +47,7 @@ struct IterArgs {
   const T *xo;              // non-cubic: chi_ab [nz/2][ny/2][nx/2][V*V], by |2 i + 1| per axis
   cudaGraphConditionalHandle cond;  // loop body: the while node to steer
   int loop;                 // 1: plane R runs the loop test itself
+  int body_kernels;         // kernels of one cycle in this form
   int nb;                   // solutes
   unsigned *gcount;         // solutes whose plane R is done (nb > 1)
   unsigned *bar;            // arrival counts of a whole-phase launch [nb]
@@ -472,7 +473,8 @@ __device__ void finalize_block(DevState *st, const double *part, int nblocks,
 // End of one device-side loop body: keep looping while any solute is still
 // running or has not yet had the idle pass after its stop (the snapshot);
 // the body count is bounded by the phase's step limit plus a margin.
-__device__ __forceinline__ void loop_test(cudaGraphConditionalHandle h, DevState *st, int nb) {
+__device__ __forceinline__ void loop_test(cudaGraphConditionalHandle h, DevState *st, int nb,
+                                          int body_kernels) {
   bool more = false;
   int cap = 1;                 // the largest step budget left to any solute
   for (int b = 0; b < nb; ++b) {
@@ -480,7 +482,7 @@ __device__ __forceinline__ void loop_test(cudaGraphConditionalHandle h, DevState
     cap = max(cap, __ldcg(&st[b].maxstep));
   }
   const int loops = ++st[0].loops;
-  st[0].bodies += 1;
+  st[0].launched += body_kernels;
   cap = cap < 1000000 ? cap : 1000000;
   if (loops >= cap + 4) more = false;
   cudaGraphSetConditional(h, more ? 1u : 0u);
@@ -497,7 +499,7 @@ __device__ __forceinline__ void loop_test_all(const IterArgs<T> &a0) {
     *a0.gcount = 0u;
     __threadfence();
   }
-  loop_test(a0.cond, a0.st, a0.nb);
+  loop_test(a0.cond, a0.st, a0.nb, a0.body_kernels);
 }
 
 }  // namespace

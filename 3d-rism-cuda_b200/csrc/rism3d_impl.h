@@ -40,7 +40,7 @@ struct DevState {
   int watch;       // 1: stop as stalled (done = 4) when progress stops
   int since;       // steps since the best rms last improved by 10 %
   int loops;       // device-side loop: bodies run in this launch (solute 0)
-  int bodies;      // device-side loop bodies of the whole solve (solute 0)
+  int launched;    // kernels of the device-side loops of the whole solve (solute 0)
   int stage_iter;  // steps of this charge-up stage, all phases
   int total_iter;  // steps of the solve, all stages and phases
   int total32;     // of which FP32

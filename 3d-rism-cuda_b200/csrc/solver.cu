@@ -1962,7 +1962,7 @@ cudaGraphExec_t capture(Context &c, const IterArgs<T> &a, cufftHandle plan) {
 }
 
 __global__ void k_loop_cond(cudaGraphConditionalHandle h, DevState *st, int nb) {
-  if (threadIdx.x == 0) loop_test(h, st, nb);
+  if (threadIdx.x == 0) loop_test(h, st, nb, 4);   // passes A, K, R and this
 }
 
 // One whole phase as a single graph: a while node whose body is one
@@ -2120,6 +2120,7 @@ void set_fused_args(Context &c, IterArgs<T> &a) {
   a.scr = (typename Cx<T>::t *)c.d_scr;
   a.scr_n = (long long)std::max(std::max(f.cr[0], f.cr[1]), std::max(f.cp[0], f.cp[1])) * c.nx * c.nx;
   a.nb = c.nb;
+  a.body_kernels = (sizeof(T) == 8 ? c.split64 : c.split32) ? 5 : 3;
   a.xo = (const T *)(sizeof(T) == 8 ? (void *)c.d_xo : (void *)c.d_xo32);
   a.gcount = c.d_count + c.nb;
   a.bar = c.d_bar;
@@ -2198,7 +2199,7 @@ int run_phase(Context &c, cufftHandle plan, T *t, T *U, T *Y, T *RP,
         status = RISM3D_CUDA_ERROR;
         break;
       }
-      c.launches += 3;
+      c.launches += fused ? a.body_kernels : 3;
       cudaMemcpyAsync(&c.h_state[(size_t)(launched % kRing) * nb], c.d_state, sizeof(DevState) * nb,
                       cudaMemcpyDeviceToHost, c.stream);
       cudaEventRecord(ev[launched % kRing], c.stream);
@@ -2223,13 +2224,13 @@ int run_phase(Context &c, cufftHandle plan, T *t, T *U, T *Y, T *RP,
       if (!cuda_ok(c, gx ? cudaGraphLaunch(gx, c.stream)
                          : launch_iteration<T, V, CLOS, REF>(c, a, plan), "iteration launch"))
         status = RISM3D_CUDA_ERROR;
-      c.launches += 3;
+      c.launches += fused ? a.body_kernels : 3;
     }
     for (int i = 0; i < kRing; ++i) cudaEventDestroy(ev[i]);
     if (status != RISM3D_OK) return status;
   }
-  // the loop's bodies (4 launches each: passes A, K, R and the loop test)
-  // are counted from the device record at the end of the solve
+  // the kernels of the loop's bodies are counted from the device record at the
+  // end of the solve
   if (fused) {
     if (!cuda_ok(c, launch_fused<T>(c, a, REF, 3), "pass after the loop")) return RISM3D_CUDA_ERROR;
     k_rp_order<T, V><<<dim3(grid_blocks((long long)V * c.n), nb), kThreads, 0, c.stream>>>(
@@ -2278,7 +2279,7 @@ int refine_base(Context &c, bool again) {
                                                          again ? 1 : 0);
   k_phase_end<<<1, 128, 0, c.stream>>>(c.d_state, nb, kBase64, 0, again ? 1 : 0, c.prm.maxstep,
                                        nullptr);
-  c.launches += 6;
+  c.launches += 5;
   return cuda_ok(c, cudaGetLastError(), "refine base") ? RISM3D_OK : RISM3D_CUDA_ERROR;
 }
 
@@ -2425,19 +2426,17 @@ int solve_v(Context &c, int chargeup) {
       !cuda_ok(c, cudaStreamSynchronize(c.stream), "solve"))
     return RISM3D_CUDA_ERROR;
   int total = 0, total32 = 0;
-  long long bodies = 0;
   for (const DevState &x : fs) {
     total = std::max(total, x.total_iter);
     total32 = std::max(total32, x.total32);
   }
-  bodies = fs[0].bodies;
   for (const DevState &x : fs)
     if (x.fault) {
       c.err = x.fault == 2 ? "a whole-phase kernel was launched without its clusters"
                            : "a device-side wait gave up: a copy or a barrier's other blocks never came";
       status = RISM3D_CUDA_ERROR;
     }
-  c.launches += (c.split64 || c.split32 ? 5 : c.fu64.on ? 3 : 4) * bodies;
+  c.launches += fs[0].launched;
   c.res.rms = fs[0].rms;
   if (nb > 1) {
     c.bres.assign(nb, rism3d_result{});
