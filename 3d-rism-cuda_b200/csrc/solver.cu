@@ -1831,6 +1831,8 @@ void launch_iteration_dm(Context &c, const IterArgs<float> &a, cufftHandle plan)
 // them on.
 template <typename T>
 [[nodiscard]] cudaError_t launch_split(Context &c, const IterArgs<T> &a, bool ref, int which) {
+  // which: 0 rows A and columns, 1 z lines, 2 inverse columns and rows R
+  static const int first[3] = {0, 2, 3}, last[3] = {2, 3, 5};
   int lines = 1;
   const fused::SplitRun<T> run[3] = {fused::split_table<T>(c.nx, c.natv, &lines),
                                      fused::split_table<T>(c.ny, c.natv, nullptr),
@@ -1841,7 +1843,7 @@ template <typename T>
   ar.nblocks = (int)(((long long)c.ny * c.nz * ((c.natv + 1) / 2) + lines - 1) / lines);
   cudaError_t e = cudaSuccess;
   if (which == 3) return run[0](5, 0, ref, hnc, c.nb, ar, c.stream);
-  for (int k = 0; k < 5 && e == cudaSuccess; ++k)
+  for (int k = which < 0 ? 0 : first[which]; k < (which < 0 ? 5 : last[which]) && e == cudaSuccess; ++k)
     e = run[axis[k]](k, axis[k], ref, hnc, c.nb, ar, c.stream);
   return e;
 }
@@ -2491,11 +2493,11 @@ int time_kernel_t(Context &c, int which, int reps, double *ms) {
   run.done = 0; run.after_done = 0; run.mode = 2; run.count = 0; run.upd_slot = 0;
   run.measure = 1;
   run.s1 = 0.25; run.s2 = 0.25;
-  // the three-kernel iteration, where the solve runs it (14 is a transform)
-  const bool three = which != 14 && !(fp64 ? c.split64 : c.split32) && (fp64 ? c.fu64.on : c.fu32.on) &&
-                     !(!fp64 && which < 13 && (c.dm_depth || c.xfused));
-  if (three) set_fused_args<T>(c, a);
-  run.rotate = three ? 1 : 0;
+  // the folded iteration, where the solve runs it (14 is a transform)
+  const bool folded = which != 14 && (fp64 ? c.fu64.on : c.fu32.on) &&
+                      !(!fp64 && which < 13 && (c.dm_depth || c.xfused));
+  if (folded) set_fused_args<T>(c, a);
+  run.rotate = folded ? 1 : 0;
   run.rp[0] = 0; run.rp[1] = 1; run.rp[2] = 2;
   stream_copy(c, c.d_state, &run, sizeof(DevState), cudaMemcpyHostToDevice);
   cudaEvent_t e0, e1;
@@ -2508,8 +2510,10 @@ int time_kernel_t(Context &c, int which, int reps, double *ms) {
   cudaEventRecord(e0, c.stream);
   cudaError_t el = cudaSuccess;                  // of a launch
   bool fused_done = false;
-  if (three) {                                   // plane A / z lines / plane R
+  int kernels = 1;                               // per repetition
+  if (folded) {                                  // rows and columns / z lines / columns and rows
     const bool ref = which == 13 || which == 15;
+    if ((fp64 ? c.split64 : c.split32) && which % 10 != 1) kernels = 2;
     for (int r = 0; r < reps && el == cudaSuccess; ++r)
       el = launch_fused<T>(c, a, ref, ref ? which - 13 : which % 10);
     fused_done = true;
@@ -2517,7 +2521,7 @@ int time_kernel_t(Context &c, int which, int reps, double *ms) {
   if constexpr (sizeof(T) == 4 && V <= 2) {
     // the fused-axis passes the FP32 solve runs (ids as below; 14: one
     // cuFFT transform along z)
-    if (c.xfused && which != 14 && !three) {
+    if (c.xfused && which != 14 && !folded) {
       if (c.nx == 256) time_fused<V, CLOS, 16>(c, a, which, reps);
       else time_fused<V, CLOS, 8>(c, a, which, reps);
       fused_done = true;
@@ -2551,7 +2555,7 @@ int time_kernel_t(Context &c, int which, int reps, double *ms) {
     }
   }
   cudaEventRecord(e1, c.stream);
-  c.launches += reps;
+  c.launches += (long long)reps * kernels;
   cudaError_t e = cudaEventSynchronize(e1);
   float t = 0;
   cudaEventElapsedTime(&t, e0, e1);

@@ -207,10 +207,12 @@ long long rism3d_kernel_launches(const rism3d_ctx *ctx);
  * which: 0/1/2 = FP64 pass A / pass K / pass R, 10/11/12 = the FP32
  * versions (MIXED contexts), 13/15 = FP32 pass A / pass R of the
  * refinement form (MIXED, after a solve), 20 = real-space potential kernel.
- * Where the iteration is the three kernels with the transforms folded in, pass
- * A is plane A (with the x- and y-DFT), pass K the z lines (with the z-DFT both
- * ways) and pass R plane R (with the inverse y- and x-DFT).  The iteration
- * kernels run on the current state with an AN2 update armed, so
+ * Where the iteration has the transforms folded in, pass A is the stage with
+ * the x- and y-DFT (plane A, or rows A and columns), pass K the z lines (with
+ * the z-DFT both ways) and pass R the stage with the inverse y- and x-DFT
+ * (plane R, or inverse columns and rows R).  A cell whose solve runs a whole
+ * phase in one launch is timed by the same three stages as kernels of their
+ * own.  The iteration kernels run on the current state with an AN2 update armed, so
  * the stored solution is invalid afterwards (solve again to restore it). */
 int rism3d_time_kernel(rism3d_ctx *ctx, int which, int reps, double *ms_per_launch);
 

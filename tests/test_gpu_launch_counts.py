@@ -88,3 +88,22 @@ def test_gradient_runs_in_one_launch(monkeypatch, edge, precision):
     n = s.kernel_launches() - n0
     s.close()
     assert n < 40, n
+
+
+@pytest.mark.parametrize("dims,precision,want", [((48, 60, 72), 0, (2, 1, 2)), ((72,) * 3, 0, (2, 1, 2)),
+                                                 ((100,) * 3, 1, (2, 1, 2)), ((128,) * 3, 0, (1, 1, 1)),
+                                                 ((100,) * 3, 0, (1, 1, 1))])
+def test_timed_stages_are_those_of_the_solve(monkeypatch, dims, precision, want):
+    """time_kernel runs the kernels of the cell's own form: rows and columns of
+    the split form together."""
+    monkeypatch.setenv("RISM3D_FUSED", "1")
+    s = _solver(dims, WATER, maxstep=5, precision=precision)
+    s.solve(allow_unconverged=True)
+    got = []
+    for which in ((0, 1, 2) if precision == 0 else (10, 11, 12)):
+        n0 = s.kernel_launches()
+        assert s.time_kernel(which, 4) > 0
+        got.append((s.kernel_launches() - n0) // 4)
+    r = s.solve(allow_unconverged=True)                  # and a solve works after it
+    s.close()
+    assert tuple(got) == want and r["iterations"] >= 5
