@@ -638,12 +638,7 @@ int adjoint_v(Context &c, double *dq, double *dsig, double *deps, double *dR) {
     c.err = "adjoint: out of device memory";
     return RISM3D_CUDA_ERROR;
   }
-  if (F32 && !c.plan32) {                       // FP64 context: the FP32 plan, made once
-    int dims[3] = {c.nz, c.ny, c.nx};
-    if (!cufft_ok(c, cufftPlanMany(&c.plan32, 3, dims, nullptr, 1, (int)n, nullptr, 1, (int)n,
-                                   CUFFT_C2C, P), "cufftPlanMany C2C"))
-      return RISM3D_CUFFT_ERROR;
-  }
+  if (!ensure_plan64(c) || (F32 && !ensure_plan32(c))) return RISM3D_CUFFT_ERROR;
   StageParams zero{}, q{};
   for (int v = 0; v < V; ++v) q.qcf[v] = c.qv[v] * c.cf_final;
   DevState run{};

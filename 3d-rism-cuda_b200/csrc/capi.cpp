@@ -129,6 +129,41 @@ void free_device(Context &c) {
   c.plans_ok = false;
 }
 
+// one batched 3D plan over the site pairs of all solutes; x is the fastest axis
+static bool make_plan(Context &c, cufftHandle &plan, cufftType type, const char *what) {
+  if (plan) return true;
+  int dims[3] = {c.nz, c.ny, c.nx};
+  const int np = (int)c.n, nbat = (c.natv + 1) / 2 * c.nb;
+  auto make = [&] {
+    if (cufft_ok(c, cufftPlanMany(&plan, 3, dims, nullptr, 1, np, nullptr, 1, np, type, nbat), what))
+      return true;
+    plan = 0;
+    return false;
+  };
+  if (make()) return true;
+  if (!c.d_fused) return false;
+  drop_fused_iteration(c);                       // room for the work area
+  cudaGetLastError();
+  return make();
+}
+
+bool ensure_plan64(Context &c) { return make_plan(c, c.plan64, CUFFT_Z2Z, "cufftPlanMany Z2Z"); }
+bool ensure_plan32(Context &c) { return make_plan(c, c.plan32, CUFFT_C2C, "cufftPlanMany C2C"); }
+
+int ensure_passes(Context &c) {
+  const bool mixed = c.prm.precision == RISM3D_MIXED, folded = c.d_fused != nullptr,
+             lib64 = !c.fu64.on, lib32 = mixed && (!c.fu32.on || c.dm_depth || c.xfused);
+  // the refinement's FP64 base cycle runs the passes in either form
+  if (((lib64 || mixed) && !ensure_plan64(c)) || (lib32 && !ensure_plan32(c)))
+    return RISM3D_CUFFT_ERROR;
+  if (folded && !c.d_fused) return ensure_passes(c);      // given up for a plan
+  if ((lib64 || lib32) && !c.pipe_asked) {
+    c.pipe_asked = true;
+    return setup_pipe_r(c);
+  }
+  return RISM3D_OK;
+}
+
 int fetch_grid(Context &c, int which, double *host) {
   const size_t n = (size_t)c.n, V = (size_t)c.natv;
   auto get = [&](const double *d, double *h, size_t cnt) {
@@ -204,23 +239,12 @@ static int alloc_state(Context &c) {
          A((void **)&c.f_R0, sizeof(float) * V * n, "alloc R0 32") &&
          A((void **)&c.f_x0, sizeof(float) * V * n, "alloc x0 32");
   if (!ok) return RISM3D_CUDA_ERROR;
-  // batched 3D plans over the site pairs; x is the fastest axis
-  // one batched plan over all site pairs of all solutes
-  int dims[3] = {c.nz, c.ny, c.nx};
-  const int np = (int)c.n, nbat = (int)(P * c.nb);
-  if (!cufft_ok(c, cufftPlanMany(&c.plan64, 3, dims, nullptr, 1, np, nullptr, 1, np,
-                                 CUFFT_Z2Z, nbat), "cufftPlanMany Z2Z"))
-    return RISM3D_CUFFT_ERROR;
-  if (mixed && !cufft_ok(c, cufftPlanMany(&c.plan32, 3, dims, nullptr, 1, np, nullptr, 1,
-                                          np, CUFFT_C2C, nbat), "cufftPlanMany C2C"))
-    return RISM3D_CUFFT_ERROR;
   if (mixed) {
     const int rc = setup_fused_axes(c);
     if (rc != RISM3D_OK) return rc;
   }
   {
-    int rc = setup_pipe_r(c);
-    if (rc == RISM3D_OK) rc = setup_fused_iteration(c);
+    const int rc = setup_fused_iteration(c);
     if (rc != RISM3D_OK) return rc;
   }
   // depth-M Anderson for the plain FP32 bulk (opt-in, single solutes); depth 2
@@ -238,13 +262,11 @@ static int alloc_state(Context &c) {
       c.dm_depth = M;
     }
   }
+  const int rc = ensure_passes(c);
+  if (rc != RISM3D_OK) return rc;
   c.plans_ok = true;
   return RISM3D_OK;
 }
-
-extern "C" {
-
-}  // extern "C"
 
 namespace rism3d {
 

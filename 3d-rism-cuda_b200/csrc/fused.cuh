@@ -973,45 +973,66 @@ struct Kernels {
   static constexpr size_t phase_smem() {
     return tables_at<T, N, V>() + 4 * N * sizeof(CxT<T>);
   }
-  // attributes and cluster counts; false when the device cannot run them
-  static bool setup(FusedPlan &f, int nb) {
+  // Attributes and cluster counts; false when the device cannot run them.  Only
+  // the kernels that the cell will launch are touched: each costs 1-4 ms the
+  // first time in a process, when the driver loads it.
+  static bool setup(FusedPlan &f, int nb, bool host) {
     const size_t s = L::template smem<T>();
-    cudaError_t e = allow(k_plane_a<T, N, V, false>, s);
-    if (e == cudaSuccess) e = allow(k_plane_r<T, N, V, false>, s);
-    if (e == cudaSuccess) e = allow(k_plane_final<T, N, V, false>, s);
-    if constexpr (ONE)
-      if (e == cudaSuccess) e = allow(k_phase<T, N, V, false>, phase_smem());
-    if (e == cudaSuccess) e = allow(k_zline<T, N, V>, Z::smem());
-    if constexpr (sizeof(T) == 4) {
-      if (e == cudaSuccess) e = allow(k_plane_a<T, N, V, true>, s);
-      if (e == cudaSuccess) e = allow(k_plane_r<T, N, V, true>, s);
+    f.nc = L::NC;
+    cudaError_t e = allow(k_plane_final<T, N, V, false>, s);
+    if constexpr (sizeof(T) == 4)
       if (e == cudaSuccess) e = allow(k_plane_final<T, N, V, true>, s);
-      if constexpr (ONE)
-        if (e == cudaSuccess) e = allow(k_phase<T, N, V, true>, phase_smem());
+    // clusters of one phase launch: resident ones shared by the nb solutes
+    if constexpr (ONE) {
+      if (!host) {
+        if (e == cudaSuccess) e = allow(k_phase<T, N, V, false>, phase_smem());
+        if (e == cudaSuccess)
+          f.cp[0] = plane_clusters(k_phase<T, N, V, false>, L::NC, L::TH, phase_smem(), 1 << 30) / nb;
+        f.cp[1] = f.cp[0];
+        if constexpr (sizeof(T) == 4) {
+          if (e == cudaSuccess) e = allow(k_phase<T, N, V, true>, phase_smem());
+          if (e == cudaSuccess)
+            f.cp[1] = plane_clusters(k_phase<T, N, V, true>, L::NC, L::TH, phase_smem(), 1 << 30) / nb;
+        }
+        for (int r = 0; r < 2; ++r) f.cp[r] = f.cp[r] < N * P ? f.cp[r] : N * P;
+      }
     }
     if (e != cudaSuccess) {
       cudaGetLastError();
       return false;
     }
-    f.ca[0] = plane_clusters(k_plane_a<T, N, V, false>, L::NC, L::TH, s, N * P);
-    f.cr[0] = plane_clusters(k_plane_r<T, N, V, false>, L::NC, L::TH, s, N * P);
+    if ((f.cp[0] == 0 || f.cp[1] == 0) && !setup_planes(f, N * P)) return false;
+    for (int r = 0; r < 2; ++r) {
+      f.cs = f.cs > f.cp[r] ? f.cs : f.cp[r];
+      f.cs = f.cs > f.cr[r] ? f.cs : f.cr[r];
+    }
+    return true;
+  }
+  // the same of the kernels of a cycle; room: exchange planes
+  static bool setup_planes(FusedPlan &f, int room) {
+    const size_t s = L::template smem<T>();
+    cudaError_t e = allow(k_plane_a<T, N, V, false>, s);
+    if (e == cudaSuccess) e = allow(k_plane_r<T, N, V, false>, s);
+    if (e == cudaSuccess) e = allow(k_zline<T, N, V>, Z::smem());
     if constexpr (sizeof(T) == 4) {
-      f.ca[1] = plane_clusters(k_plane_a<T, N, V, true>, L::NC, L::TH, s, N * P);
-      f.cr[1] = plane_clusters(k_plane_r<T, N, V, true>, L::NC, L::TH, s, N * P);
-    } else {
-      f.ca[1] = f.ca[0];
-      f.cr[1] = f.cr[0];
+      if (e == cudaSuccess) e = allow(k_plane_a<T, N, V, true>, s);
+      if (e == cudaSuccess) e = allow(k_plane_r<T, N, V, true>, s);
     }
-    f.nc = L::NC;
-    // clusters of one phase launch: resident ones shared by the nb solutes
-    if constexpr (ONE) {
-      f.cp[0] = plane_clusters(k_phase<T, N, V, false>, L::NC, L::TH, phase_smem(), 1 << 30) / nb;
-      f.cp[1] = f.cp[0];
-      if constexpr (sizeof(T) == 4)
-        f.cp[1] = plane_clusters(k_phase<T, N, V, true>, L::NC, L::TH, phase_smem(), 1 << 30) / nb;
-      for (int r = 0; r < 2; ++r) f.cp[r] = f.cp[r] < N * P ? f.cp[r] : N * P;
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return false;
     }
-    return f.ca[0] > 0 && f.cr[0] > 0 && f.ca[1] > 0 && f.cr[1] > 0;
+    const int planes = N * P, rp = planes < room ? planes : room;
+    f.ca[0] = plane_clusters(k_plane_a<T, N, V, false>, L::NC, L::TH, s, planes);
+    f.cr[0] = plane_clusters(k_plane_r<T, N, V, false>, L::NC, L::TH, s, rp);
+    f.ca[1] = f.ca[0];
+    f.cr[1] = f.cr[0];
+    if constexpr (sizeof(T) == 4) {
+      f.ca[1] = plane_clusters(k_plane_a<T, N, V, true>, L::NC, L::TH, s, planes);
+      f.cr[1] = plane_clusters(k_plane_r<T, N, V, true>, L::NC, L::TH, s, rp);
+    }
+    f.planes = f.ca[0] > 0 && f.cr[0] > 0 && f.ca[1] > 0 && f.cr[1] > 0;
+    return f.planes;
   }
   // which: 0 plane A, 1 z lines, 2 plane R, 3 the pass after the loop, 4 a
   // whole phase
@@ -1034,7 +1055,7 @@ struct Kernels {
       if (which == 4)
         return launch_plane(k_phase<T, N, V, REF>, f.cp[REF], L::NC, nb, L::TH, phase_smem(),
                             st, true, a, hnc);
-    const int ncl = which == 0 ? f.ca[REF] : f.cr[REF];
+    const int ncl = which == 0 ? f.ca[REF] : which == 2 ? f.cr[REF] : f.cs;
     return launch_plane(which == 0   ? k_plane_a<T, N, V, REF>
                         : which == 2 ? k_plane_r<T, N, V, REF>
                                      : k_plane_final<T, N, V, REF>,
@@ -1045,10 +1066,10 @@ struct Kernels {
 template <typename T, int N>
 Vtable<T> table_v(int V) {
   switch (V) {
-    case 2: return {Kernels<T, N, 2>::setup, Kernels<T, N, 2>::launch};
-    case 4: return {Kernels<T, N, 4>::setup, Kernels<T, N, 4>::launch};
+    case 2: return {Kernels<T, N, 2>::setup, Kernels<T, N, 2>::setup_planes, Kernels<T, N, 2>::launch};
+    case 4: return {Kernels<T, N, 4>::setup, Kernels<T, N, 4>::setup_planes, Kernels<T, N, 4>::launch};
   }
-  return {nullptr, nullptr};
+  return {};
 }
 
 }  // namespace fused

@@ -11,7 +11,7 @@ template <> Vtable<float> table_a<float>(int N, int V) {
     case 40: return table_v<float, 40>(V);
     case 48: return table_v<float, 48>(V);
   }
-  return {nullptr, nullptr};
+  return {};
 }
 
 }  // namespace fused

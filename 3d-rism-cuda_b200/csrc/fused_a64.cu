@@ -11,7 +11,7 @@ template <> Vtable<double> table_a<double>(int N, int V) {
     case 40: return table_v<double, 40>(V);
     case 48: return table_v<double, 48>(V);
   }
-  return {nullptr, nullptr};
+  return {};
 }
 
 }  // namespace fused

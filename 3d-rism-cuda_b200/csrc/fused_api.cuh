@@ -43,13 +43,15 @@ inline Form cubic_form(int N, bool fp64) {
   return kLibrary;
 }
 
-// set-up (attributes, cluster counts; false: not on this device) and launch
-// of kernel 0 (plane A), 1 (z lines), 2 (plane R), 3 (the pass after the loop) or 4 (a
+// set-up (attributes, cluster counts; false: not on this device) for nb solutes
+// and, where not part of it, of the kernels of a cycle; launch of kernel 0 (plane A), 1 (z lines), 2 (plane R), 3 (the pass after the loop) or 4 (a
 // whole phase) of one (T, edge, sites)
 template <typename T>
 struct Vtable {
-  bool (*setup)(FusedPlan &, int);
-  cudaError_t (*launch)(const FusedPlan &, int, bool, int, int, const IterArgs<T> &, cudaStream_t);
+  bool (*setup)(FusedPlan &, int nb, bool host_driven) = nullptr;
+  bool (*planes)(FusedPlan &, int room) = nullptr;
+  cudaError_t (*launch)(const FusedPlan &, int, bool, int, int, const IterArgs<T> &,
+                        cudaStream_t) = nullptr;
 };
 
 // one translation unit per group of edges: up to 48, 60-80, above

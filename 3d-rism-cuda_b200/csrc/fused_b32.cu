@@ -11,7 +11,7 @@ template <> Vtable<float> table_b<float>(int N, int V) {
     case 72: return table_v<float, 72>(V);
     case 80: return table_v<float, 80>(V);
   }
-  return {nullptr, nullptr};
+  return {};
 }
 
 }  // namespace fused

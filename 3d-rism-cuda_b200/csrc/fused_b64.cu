@@ -10,7 +10,7 @@ template <> Vtable<double> table_b<double>(int N, int V) {
     case 64: return table_v<double, 64>(V);
     case 80: return table_v<double, 80>(V);
   }
-  return {nullptr, nullptr};
+  return {};
 }
 
 }  // namespace fused

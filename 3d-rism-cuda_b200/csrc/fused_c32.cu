@@ -10,7 +10,7 @@ template <> Vtable<float> table_c<float>(int N, int V) {
     case 128: return table_v<float, 128>(V);
     case 256: return table_v<float, 256>(V);
   }
-  return {nullptr, nullptr};
+  return {};
 }
 
 }  // namespace fused

@@ -10,7 +10,7 @@ template <> Vtable<double> table_c<double>(int N, int V) {
     case 160: return table_v<double, 160>(V);
     case 256: return table_v<double, 256>(V);
   }
-  return {nullptr, nullptr};
+  return {};
 }
 
 }  // namespace fused

@@ -134,6 +134,8 @@ struct FusedPlan {
   int ca[2] = {0, 0};         // clusters of plane A: plain, refinement form
   int cr[2] = {0, 0};         // clusters of plane R
   int cp[2] = {0, 0};         // clusters per solute of a whole-phase launch (0: none)
+  int cs = 0;                 // exchange planes per solute
+  bool planes = false;        // the kernels of a cycle are set up (ca, cr)
 };
 
 struct Timer {
@@ -233,6 +235,7 @@ struct Context {
   int dm_depth = 0;
   float *f_Ydm = nullptr, *f_RPdm = nullptr;
   bool pipe_r = false;       // pass R as the cp.async pipeline (natv <= 2)
+  bool pipe_asked = false;   // setup_pipe_r has run
   bool bulk_r = false;       // pass R as the bulk-copy (cp.async.bulk) stream
   bool xfused = false;
   cufftHandle plan32z = 0;
@@ -320,6 +323,11 @@ void drop_fused_iteration(Context &c);            // capi.cpp
 int setup_kspace_tma(Context &c);                 // solver.cu: TMA fused pass K
 int fused_fk_columns(Context &c);                 // solver.cu: fk copy for it
 int setup_pipe_r(Context &c);                     // solver.cu: pipelined pass R
+// cuFFT plans and pass R's set-up, where a phase of the solve runs the passes;
+// called at set-up and before a solve
+int ensure_passes(Context &c);                    // capi.cpp
+bool ensure_plan64(Context &c);                   // capi.cpp: 3D transforms of all site pairs
+bool ensure_plan32(Context &c);
 // spline.cc:4-43: natural cubic spline through (xp[k], yp[k]), k < np; writes
 // {y_k, b_k, c_k, d_k} (y + b t + c t^2 + d t^3 on interval k; zero
 // coefficients on the last knot) to out[k * stride + 0..3]

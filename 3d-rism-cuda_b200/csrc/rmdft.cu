@@ -252,6 +252,7 @@ int rmdft_v(Context &c) {
                                    CUFFT_Z2Z, 1), "cufftPlanMany RMDFT"))
       return RISM3D_CUFFT_ERROR;
   }
+  if (!ensure_plan64(c)) return RISM3D_CUFFT_ERROR;
   if (!cufft_ok(c, cufftSetStream(c.plan1, c.stream), "cufftSetStream") ||
       !cufft_ok(c, cufftSetStream(c.plan64, c.stream), "cufftSetStream"))
     return RISM3D_CUFFT_ERROR;

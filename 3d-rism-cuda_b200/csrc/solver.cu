@@ -1853,9 +1853,10 @@ template <typename T>
   cudaGetLastError();                            // an earlier call's error is not this launch's
   if (sizeof(T) == 8 ? c.split64 : c.split32)    // which: -1 a cycle, 3 the pass after the loop
     return launch_split<T>(c, a, ref, which);
-  const FusedPlan &f = sizeof(T) == 8 ? c.fu64 : c.fu32;
+  FusedPlan &f = sizeof(T) == 8 ? c.fu64 : c.fu32;
   const int hnc = c.prm.closure == RISM3D_HNC;
   const fused::Vtable<T> tab = fused::table<T>(c.nx, c.natv);
+  if (which < 3 && !f.planes && !tab.planes(f, f.cs)) return cudaErrorInvalidConfiguration;
   IterArgs<T> ar = a;
   ar.nblocks = (which == 4 ? f.cp[ref ? 1 : 0] : f.cr[ref ? 1 : 0]) * f.nc;
   cudaError_t e = cudaSuccess;
@@ -2120,7 +2121,7 @@ void set_fused_args(Context &c, IterArgs<T> &a) {
   a.RPx = (T *)(sizeof(T) == 8 ? (void *)c.d_RPx : (void *)c.f_RPx);
   a.roots = (const typename Cx<T>::t *)(sizeof(T) == 8 ? (void *)c.d_roots : (void *)c.f_roots);
   a.scr = (typename Cx<T>::t *)c.d_scr;
-  a.scr_n = (long long)std::max(std::max(f.cr[0], f.cr[1]), std::max(f.cp[0], f.cp[1])) * c.nx * c.nx;
+  a.scr_n = (long long)f.cs * c.nx * c.nx;
   a.nb = c.nb;
   a.body_kernels = (sizeof(T) == 8 ? c.split64 : c.split32) ? 5 : 3;
   a.xo = (const T *)(sizeof(T) == 8 ? (void *)c.d_xo : (void *)c.d_xo32);
@@ -2150,7 +2151,8 @@ int run_phase(Context &c, cufftHandle plan, T *t, T *U, T *Y, T *RP,
   k_phase_begin<<<1, 128, 0, c.stream>>>(c.d_state, nb, kind, conv, c.prm.maxstep,
                                          watch ? 1 : 0, c.prm.an2_count, fused ? 1 : 0, again ? 1 : 0);
   c.launches += 1;
-  if (!cufft_ok(c, cufftSetStream(plan, c.stream), "cufftSetStream")) return RISM3D_CUFFT_ERROR;
+  if (!fused && !cufft_ok(c, cufftSetStream(plan, c.stream), "cufftSetStream"))
+    return RISM3D_CUFFT_ERROR;
   if (c.plan32z && !cufft_ok(c, cufftSetStream(c.plan32z, c.stream), "cufftSetStream"))
     return RISM3D_CUFFT_ERROR;
   int status = RISM3D_OK;
@@ -2159,6 +2161,12 @@ int run_phase(Context &c, cufftHandle plan, T *t, T *U, T *Y, T *RP,
   // one launch for the phase (not while iterations are driven from the host)
   const bool one = fused && !c.no_device_loop &&
                    (sizeof(T) == 8 ? c.fu64 : c.fu32).cp[REF ? 1 : 0] > 0;
+  FusedPlan &f = sizeof(T) == 8 ? c.fu64 : c.fu32;
+  if (fused && !one && !f.planes && !(sizeof(T) == 8 ? c.split64 : c.split32) &&
+      !fused::table<T>(c.nx, c.natv).planes(f, f.cs)) {      // before a capture
+    c.err = "the folded iteration's kernels cannot run on this device";
+    return RISM3D_CUDA_ERROR;
+  }
   if (!one && !lx && !c.no_device_loop) {
     lx = capture_loop<T, V, CLOS, REF>(c, a, plan);
     if (!lx) c.no_device_loop = true;
@@ -2681,8 +2689,13 @@ int setup_fused_iteration(Context &c) {
               f32 = !mixed ? fused::kLibrary : cubic ? fused::cubic_form(c.nx, false) : fused::kSplit;
   const fused::Vtable<double> t64 = fused::table<double>(c.nx, V);
   const fused::Vtable<float> t32 = fused::table<float>(c.nx, V);
-  if (f64 == fused::kPlanes && (!t64.setup || !t64.setup(c.fu64, c.nb))) f64 = fused::kLibrary;
-  if (f32 == fused::kPlanes && (!t32.setup || !t32.setup(c.fu32, c.nb))) f32 = fused::kLibrary;
+  const bool host = c.no_device_loop;
+  // this file's module is loaded here (50 ms, once in a process), not in the
+  // first solve
+  cudaFuncAttributes at;
+  cudaFuncGetAttributes(&at, k_init_t);
+  if (f64 == fused::kPlanes && (!t64.setup || !t64.setup(c.fu64, c.nb, host))) f64 = fused::kLibrary;
+  if (f32 == fused::kPlanes && (!t32.setup || !t32.setup(c.fu32, c.nb, host))) f32 = fused::kLibrary;
   // the split form: kernels of every axis' edge
   int lines = 1;
   auto split_ok = [&](auto zero) {
@@ -2701,14 +2714,11 @@ int setup_fused_iteration(Context &c) {
   };
   if (f64 == fused::kSplit && !split_ok(0.0)) f64 = fused::kLibrary;
   if (f32 == fused::kSplit && !split_ok(0.0f)) f32 = fused::kLibrary;
-  auto max_cr = [](const FusedPlan &f) {
-    return (size_t)std::max(std::max(f.cr[0], f.cr[1]), std::max(f.cp[0], f.cp[1]));
-  };
   const bool split = f64 == fused::kSplit || f32 == fused::kSplit;
   const size_t blocks =
-      std::max(std::max(max_cr(c.fu64) * c.fu64.nc, max_cr(c.fu32) * c.fu32.nc),
+      std::max(std::max((size_t)c.fu64.cs * c.fu64.nc, (size_t)c.fu32.cs * c.fu32.nc),
                split ? ((size_t)c.ny * c.nz * ((V + 1) / 2) + lines - 1) / lines : 0);
-  const size_t scr = std::max(max_cr(c.fu64) * sizeof(double2), max_cr(c.fu32) * sizeof(float2)) *
+  const size_t scr = std::max(c.fu64.cs * sizeof(double2), c.fu32.cs * sizeof(float2)) *
                      (size_t)c.nx * c.nx * c.nb;
   const size_t oct = split ? (size_t)(c.n / 8) * V * V : 0;
   if (f64 == fused::kLibrary && f32 == fused::kLibrary) return RISM3D_OK;
@@ -3063,6 +3073,8 @@ int launch_oz_kspace(Context &c, double2 *buf, const StageParams *sp, DevState *
 }
 
 int run_solve(Context &c, int chargeup) {
+  const int rc = ensure_passes(c);
+  if (rc != RISM3D_OK) return rc;
   switch (c.natv) {
     case 1: return solve_c<1>(c, chargeup);
     case 2: return solve_c<2>(c, chargeup);
