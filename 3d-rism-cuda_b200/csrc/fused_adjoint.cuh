@@ -315,22 +315,21 @@ __global__ void __cluster_dims__(Lines<N>::NC, 1, 1)
   for (int i = threadIdx.x; i < N; i += blockDim.x) roots[i] = g.it.roots[i];
   if (threadIdx.x == 0) s = *g.st;
   __syncthreads();
-  const unsigned nblk = gridDim.x, delay = g.it.delay;
-  unsigned *bar = &g.st->bar, target = 0;
-  bool ok = true;
-  if (delay && threadIdx.x == 0) stage_delay(delay, target);
+  __shared__ GridBarrier bar;
+  const unsigned nblk = gridDim.x;
+  if (threadIdx.x == 0) enter_barrier(bar, &g.st->bar, g.it.delay);
   __syncthreads();
   while (!s.done) {
     adjoint_forward<T, N, V>(g, &s, sm, tw, roots);
-    if (!(ok = grid_barrier(bar, target += nblk, delay))) break;
+    if (!grid_barrier(bar)) break;
 #pragma unroll 1
     for (int tile = blockIdx.x; tile < ZShape<T, N, V>::TILES; tile += nblk) {
       zline_tile<T, N, V, false, true>(g.it, sm, roots, N, N, tile);
       __syncthreads();
     }
-    if (!(ok = grid_barrier(bar, target += nblk, delay))) break;
+    if (!grid_barrier(bar)) break;
     adjoint_residual<T, N, V>(g, &s, sm, tw, roots);
-    if (!(ok = grid_barrier(bar, target += nblk, delay))) break;
+    if (!grid_barrier(bar)) break;
     adjoint_finalize(&s, g.part, (int)nblk, g.tol, g.maxit, sizeof(T) == 4);
   }
   if (threadIdx.x == 0) {
@@ -338,7 +337,7 @@ __global__ void __cluster_dims__(Lines<N>::NC, 1, 1)
       g.st->done = s.done;
       g.st->it = s.it;
     }
-    if (ok) leave_barrier(bar, target, nblk);
+    leave_barrier(bar);
   }
 }
 
