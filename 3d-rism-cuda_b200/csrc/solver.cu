@@ -2387,7 +2387,10 @@ int solve_v(Context &c, int chargeup) {
       const double conv = c.prm.convergence;
       double sw = c.prm.mixed_switch > 0 ? c.prm.mixed_switch : std::max(100.0 * conv, 1e-4);
       if (sw < conv) sw = conv;
-      const int rounds = std::max(1, (int)ceil(log(sw / conv) / log(200.0)));
+      // (No residual falls below 1e-16: a tolerance under it, given to use up the
+      // step limit, adds no rounds: 32^3, limit 1500: 1 FP64 step -> 632.)
+      const double goal = std::max(conv, 1e-16);
+      const int rounds = std::max(1, (int)ceil(log(sw / goal) / log(200.0)));
       st = run_phase<float, V, CLOS, false>(c, c.plan32, c.f_t, c.f_U,
                                            c.dm_depth ? c.f_Ydm : c.f_Y,
                                            c.dm_depth ? c.f_RPdm : c.f_RP, c.f_buf,
@@ -2401,7 +2404,7 @@ int solve_v(Context &c, int chargeup) {
       k_promote_base<<<gb, kThreads, 0, c.stream>>>(vn, c.f_t, c.d_state, c.d_t);
       c.launches += 1;
       for (int r = 0; r < rounds && st == RISM3D_OK; ++r) {
-        const double target = r + 1 == rounds ? conv : sw * pow(conv / sw, (r + 1.0) / rounds);
+        const double target = r + 1 == rounds ? conv : sw * pow(goal / sw, (r + 1.0) / rounds);
         st = refine_base<V, CLOS>(c, r > 0);
         if (st == RISM3D_OK)
           st = run_phase<float, V, CLOS, true>(c, c.plan32, c.f_t, c.f_x0, c.f_Y, c.f_RP, c.f_buf,

@@ -197,3 +197,15 @@ def test_potentials_of_odd_site_counts(sites, precision):
         e4 = 4.0 * beta * np.sqrt(eps * sv.epsv[v])
         want, size = (e4 * (s6 * s6 - s6)).sum(axis=1), (e4 * (s6 * s6 + s6)).sum(axis=1)
         assert np.all(np.abs(got[v] - want) <= (257 + 10) * unit * size)
+
+
+def test_unreachable_tolerance_leaves_steps_to_fp64(monkeypatch):
+    """A tolerance below any residual (to use up the step limit): the rounds end
+    at the rounding floor, and it is FP64 steps that reach the limit (a phase
+    that finds it used up takes one step more)."""
+    monkeypatch.setenv("RISM3D_FUSED", "1")
+    s = _solver((32,) * 3, WATER, precision=1, convergence=1e-300, maxstep=1500)
+    r = s.solve(allow_unconverged=True)
+    s.close()
+    assert r["status"] == 6 and r["iterations"] == 1500
+    assert r["iterations"] - r["iterations_fp32"] > 6 + 1       # more than the bases and a step
