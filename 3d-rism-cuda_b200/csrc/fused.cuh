@@ -1,5 +1,5 @@
 // One iteration in three kernels, with the 3D transforms folded in (cubic
-// cells whose edge N = R1 R2 has an instantiation, up to four solvent sites):
+// cells whose edge N = R1 R2 has an instantiation, two or four solvent sites):
 //
 //   k_plane_a  update + closure + packing of one xy plane, x- and y-DFT
 //   k_zline    z-DFT, OZ product of every mirror pair, inverse z-DFT
@@ -285,7 +285,7 @@ __device__ __forceinline__ void rows_inverse(const CxT<T> *src, CxT<T> *line, in
 // twiddled, then its x-DFT to dst.
 template <typename T, int N, int V, bool REF, bool WIDE>
 __device__ __forceinline__ void update_row(const IterArgs<T> &a, const DevState *st, CxT<T> *line,
-                                           int t, bool live, bool two, size_t base, CxT<T> tyz,
+                                           int t, bool live, size_t base, CxT<T> tyz,
                                            int dyz, CxT<T> *dst, const CxT<T> *tw,
                                            const CxT<T> *roots, bool hnc) {
   typedef CxT<T> C;
@@ -310,10 +310,8 @@ __device__ __forceinline__ void update_row(const IterArgs<T> &a, const DevState 
         x0[q] = VW * (t + R2 * (q + NV * c));
         ldv(tv[0][q], pt + x0[q]);
         ldv(uv[0][q], pu + x0[q]);
-        if (two) {
-          ldv(tv[1][q], pt + n + x0[q]);
-          ldv(uv[1][q], pu + n + x0[q]);
-        }
+        ldv(tv[1][q], pt + n + x0[q]);
+        ldv(uv[1][q], pu + n + x0[q]);
       }
       if (mode != 0) {
         T rv[2][NV][VW], y0[2][NV][VW], y1[2][NV][VW];
@@ -321,7 +319,6 @@ __device__ __forceinline__ void update_row(const IterArgs<T> &a, const DevState 
         for (int q = 0; q < NV; ++q)
 #pragma unroll
           for (int b = 0; b < 2; ++b) {
-            if (b && !two) break;
             ldv(rv[b][q], pr + b * n + x0[q]);
             ldv(y0[b][q], p0 + b * n + x0[q]);
             ldv(y1[b][q], p1 + b * n + x0[q]);
@@ -330,7 +327,6 @@ __device__ __forceinline__ void update_row(const IterArgs<T> &a, const DevState 
         for (int q = 0; q < NV; ++q)
 #pragma unroll
           for (int b = 0; b < 2; ++b) {
-            if (b && !two) break;
             T yw[VW];
 #pragma unroll
             for (int k = 0; k < VW; ++k) {
@@ -353,7 +349,7 @@ __device__ __forceinline__ void update_row(const IterArgs<T> &a, const DevState 
           const int x = x0[q] + k;
           C cc;
           cc.x = cfun_rt<REF>(tv[0][q][k], uv[0][q][k], hnc);
-          cc.y = two ? cfun_rt<REF>(tv[1][q][k], uv[1][q][k], hnc) : T(0);
+          cc.y = cfun_rt<REF>(tv[1][q][k], uv[1][q][k], hnc);
           const C kf = cmul(tw[x], tyz);
           const T dir = ((x & 1) ^ dyz) ? T(-1) : T(1);
           C w;
@@ -378,14 +374,13 @@ __device__ __forceinline__ void planes_a(const IterArgs<T> &a, const DevState *s
   const int row_l = threadIdx.x / R2, t = threadIdx.x % R2;
   for (int plane = blockIdx.x / L::NC; plane < N * P; plane += ncl) {
     const int p = plane / N, z = plane % N;
-    const bool two = V % 2 == 0 || 2 * p + 1 < V;
     C *pb = a.buf + (size_t)plane * N * N;
     __syncthreads();                               // the columns' exchange is free
 #pragma unroll 1
     for (int rb = 0; rb < L::SH; rb += LB) {
       const bool live = L::FULL || (row_l < LB && rb + row_l < L::SH);
       const int y = rank * L::SH + (live ? rb + row_l : 0);
-      update_row<T, N, V, REF, WIDE>(a, st, sm + row_l * L::LS, t, live, two,
+      update_row<T, N, V, REF, WIDE>(a, st, sm + row_l * L::LS, t, live,
                                      (size_t)(2 * p) * n + ((size_t)z * N + y) * N,
                                      cmul(tw[N + y], tw[2 * N + z]), (y + z) & 1,
                                      pb + (size_t)y * N, tw, roots, hnc);
@@ -410,7 +405,7 @@ __global__ void __cluster_dims__(Lines<N>::NC, 1, 1)
 // sites v0 and v0 + 1): residuals, their sums, the new residual slot.
 template <typename T, int N, int V, bool REF, bool WIDE>
 __device__ __forceinline__ void residual_row(const IterArgs<T> &a, const DevState *st,
-                                             const CxT<T> *line, int t, bool two, int v0,
+                                             const CxT<T> *line, int t, int v0,
                                              size_t base, CxT<T> tyz, int dyz, const CxT<T> *tw,
                                              bool gram, bool hnc, double (&acc)[6]) {
   typedef CxT<T> C;
@@ -432,7 +427,6 @@ __device__ __forceinline__ void residual_row(const IterArgs<T> &a, const DevStat
       x0[q] = VW * (t + R2 * (q + NV * c));
 #pragma unroll
       for (int b = 0; b < 2; ++b) {
-        if (b && !two) break;
         ldv(tv[b][q], pt + b * n + x0[q]);
         ldv(uv[b][q], pu + b * n + x0[q]);
         ldv(r0[b][q], p0 + b * n + x0[q]);
@@ -455,7 +449,6 @@ __device__ __forceinline__ void residual_row(const IterArgs<T> &a, const DevStat
         const C h = cmul(line[(x / R2) * ST + x % R2], w);
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
-          if (b && !two) break;
           const T R = residual_rt<REF>(b ? h.y : h.x, tv[b][q][k], uv[b][q][k],
                                        REF ? qv[b][q][k] : T(0), hnc);
           rw[b][k] = R;
@@ -474,7 +467,6 @@ __device__ __forceinline__ void residual_row(const IterArgs<T> &a, const DevStat
       }
 #pragma unroll
       for (int b = 0; b < 2; ++b) {
-        if (b && !two) break;
         stv(pr + b * n + x0[q], rw[b]);
       }
     }
@@ -517,7 +509,6 @@ __device__ __forceinline__ void planes_r(const IterArgs<T> &a, const DevState *s
   double acc[6] = {0, 0, 0, 0, 0, 0};
   for (int plane = cl; plane < N * P; plane += ncl) {
     const int p = plane / N, z = plane % N;
-    const bool two = V % 2 == 0 || 2 * p + 1 < V;
     columns<T, N, true, L::FULL>(a.buf + (size_t)plane * N * N + rank * L::SH, scr + rank * L::SH, N, L::SH,
                         sm, roots);
     __syncthreads();                               // the columns' exchange is free
@@ -528,7 +519,7 @@ __device__ __forceinline__ void planes_r(const IterArgs<T> &a, const DevState *s
       const int y = rank * L::SH + (live ? rb + row_l : 0);
       rows_inverse<T, N>(scr + (size_t)y * N, line, t, live, roots);
       if (live)
-        residual_row<T, N, V, REF, WIDE>(a, st, line, t, two, 2 * p,
+        residual_row<T, N, V, REF, WIDE>(a, st, line, t, 2 * p,
                                          (size_t)(2 * p) * n + ((size_t)z * N + y) * N,
                                          cmul(tw[N + y], tw[2 * N + z]), (y + z) & 1, tw, gram,
                                          hnc, acc);
@@ -595,7 +586,6 @@ __device__ __forceinline__ void final_row(const IterArgs<T> &a, const CxT<T> *li
     const C h = cmul(line[(x / R2) * ST + x % R2], w);
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      if (2 * p + q >= V) break;
       const size_t iv = (size_t)(2 * p + q) * n + row + x;
       const T tv = a.t[iv];
       if (snap) {
@@ -982,6 +972,7 @@ struct Kernels {
   using L = Lines<N>;
   using Z = ZShape<T, N, V>;
   static constexpr int P = (V + 1) / 2;
+  static_assert(V % 2 == 0, "whole site pairs");
   // A phase as one launch, by what a step took on a B200 (us, loop of three
   // launches / one launch; V = 2): FP64 N = 32 25 / 16, 64 31 / 23, 80 52 / 41,
   // 128 152 / 132, 160 336 / 320, 256 1022 / 1082; V = 4: 64 47 / 39, 80 109 /

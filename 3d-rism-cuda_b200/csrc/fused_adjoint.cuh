@@ -88,7 +88,6 @@ __device__ __forceinline__ void adjoint_forward(const AdjointArgs<T> &g, const A
   for (int i = 0; i < kAdjDepth; ++i) cf[i] = i < ns ? s->coef[i] : 0.0;
   for (int plane = blockIdx.x / L::NC; plane < N * P; plane += ncl) {
     const int p = plane / N, z = plane % N;
-    const bool two = V % 2 == 0 || 2 * p + 1 < V;
     C *pb = a.buf + (size_t)plane * N * N;
     __syncthreads();                               // the columns' exchange is free
 #pragma unroll 1
@@ -107,7 +106,6 @@ __device__ __forceinline__ void adjoint_forward(const AdjointArgs<T> &g, const A
         for (int b = 0; b < 2; ++b) {
 #pragma unroll
           for (int k = 0; k < VW; ++k) xv[b][k] = T(0);
-          if (b && !two) break;
           const size_t j = base + b * n + x0;
           if (ns == 0) {
             ldv(xv[b], g.xi + j);
@@ -171,7 +169,6 @@ __device__ __forceinline__ void adjoint_residual(const AdjointArgs<T> &g, const 
   for (int i = 0; i <= kAdjDepth; ++i) acc[i] = 0.0;
   for (int plane = cl; plane < N * P; plane += ncl) {
     const int p = plane / N, z = plane % N;
-    const bool two = V % 2 == 0 || 2 * p + 1 < V;
     columns<T, N, true, L::FULL>(a.buf + (size_t)plane * N * N + rank * L::SH, scr + rank * L::SH, N, L::SH,
                         sm, roots);
     __syncthreads();                               // the columns' exchange is free
@@ -200,7 +197,6 @@ __device__ __forceinline__ void adjoint_residual(const AdjointArgs<T> &g, const 
         }
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
-          if (b && !two) break;
           const size_t j = base + b * n + x0;
           T gv[VW], wv[VW], xv[VW], rv[kAdjDepth][VW], lw[VW], rw[VW], yw[VW];
           ldv(gv, g.G + j);

@@ -26,6 +26,20 @@ enum Form { kLibrary, kPlanes, kSplit };
 //         160 238 / 203 / 188   180 365 / 425 / 326   192 372 / 346 / 311
 //         200 488 / 465 / 398   216 528 / 632 / 521   240 833 / 794 / 661
 //         256 817 / 653 / 650
+// Smaller edges, library passes / the planes' one launch:
+//   FP64   32  32 / 15           36  31 / 16           40  34 / 22
+//          48  37 / 21           60  43 / 30
+//   FP32   32  29 / 12           36  32 / 13           40  34 / 16
+//          48  36 / 16           60  39 / 19
+// Four sites, library passes / the form chosen:
+//   FP64   32  35 / 18   36  37 / 26   40  41 / 33   48  48 / 31   60  67 / 53
+//          64  68 / 37   72  96 / 71   80 129 / 90   96 200 / 137 120 329 / 315
+//         128 369 / 311 160 751 / 741 256 2819 / 2368
+//   FP32   32  33 / 14   36  33 / 21   40  35 / 25   48  41 / 22   60  49 / 36
+//          64  51 / 24   72  65 / 42   80  76 / 49   96 119 / 73  120 192 / 186
+//         128 205 / 149 160 398 / 395 256 1493 / 1300
+// Edges with another prime factor than 2, 3 and 5, above 256, and one, three or
+// more than four sites run the library passes.
 // Cells that are not cubic run the split form (72x60x48 50 / - / 41).
 inline Form cubic_form(int N, bool fp64) {
   switch (N) {

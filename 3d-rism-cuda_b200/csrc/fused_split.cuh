@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(Lines<N>::TH, (Lines<N>::template minb<T>()))
   const int p = live ? r / rows : 0, yz = live ? r - p * rows : 0, z = yz / a.ny, y = yz - z * a.ny;
   const size_t base = (size_t)yz * N;
   update_row<T, N, V, REF, false>(a, a.st, reinterpret_cast<C *>(fused_sm) + row_l * L::LS, t, live,
-                                  V % 2 == 0 || 2 * p + 1 < V, (size_t)(2 * p) * a.n + base,
+                                  (size_t)(2 * p) * a.n + base,
                                   cmul(a.tw[N + y], a.tw[N + a.ny + z]), (y + z) & 1,
                                   a.buf + (size_t)p * a.n + base, a.tw, a.roots, hnc);
 }
@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(Lines<N>::TH, (Lines<N>::template minb<T>()))
   double acc[6] = {0, 0, 0, 0, 0, 0};
   rows_inverse<T, N>(a.buf + (size_t)p * a.n + base, line, t, live, a.roots);
   if (live)
-    residual_row<T, N, V, REF, false>(a, a.st, line, t, V % 2 == 0 || 2 * p + 1 < V, 2 * p,
+    residual_row<T, N, V, REF, false>(a, a.st, line, t, 2 * p,
                                       (size_t)(2 * p) * a.n + base,
                                       cmul(a.tw[N + y], a.tw[N + a.ny + z]), (y + z) & 1, a.tw,
                                       a.st->count <= 0, hnc, acc);
@@ -115,6 +115,7 @@ __global__ void __launch_bounds__(ZShape<T, N, V>::TH, (ZShape<T, N, V>::MINB))
 // the row kernels.
 template <typename T, int N, int V>
 struct SplitKernels {
+  static_assert(V % 2 == 0, "whole site pairs");
   using L = Lines<N>;
   using Z = ZShape<T, N, V>;
   template <typename K> static void attr(K k, size_t b, cudaError_t &e) {

@@ -81,8 +81,9 @@ __device__ __forceinline__ double rsqrt_nr(double x) {
 }
 
 // 1/sqrt(x), x > 0 normal: the hardware approximation y (relative error below
-// 2^-20) and one third-order step y (1 + e/2 + 3 e^2/8), e = 1 - x y^2; what
-// is dropped, 5 e^3 / 16, is below 1e-18.  The approximation's low word is
+// 2^-20) and the binomial series of (1 - e)^(-1/2), e = 1 - x y^2, to second
+// order, y (1 + e/2 + 3 e^2/8): a third-order step.  |e| is below 2^-19, and
+// what is dropped, 5 e^3 / 16, below 2.2e-18.  The approximation's low word is
 // zero, so y y is exact and e has no rounding to speak of.  x = 0 gives NaN.
 __device__ __forceinline__ double rsqrt_3(double x) {
   double y;
