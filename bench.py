@@ -127,6 +127,12 @@ def folded_bytes_per_point(V, s):
     return {"pass_a": 8 * V * s, "pass_k": 2 * V * s + 8, "pass_r": 6 * V * s}
 
 
+def transform_bytes_per_point(V, s):
+    """Two 3D library transforms a cycle, three read-write passes each over the
+    packed site pairs (the folded kernels have none)."""
+    return 2 * 3 * 2 * ((V + 1) // 2) * 2 * s
+
+
 def fused_pipeline_bytes_per_iter(n, V, s, s_lr=None):
     """N (31 V s + 5 s_lr + 4): minimal fused pipeline of the per-site design;
     the long-range Coulomb grids (e, fr, fk) stay FP64 (s_lr = 8) in the
@@ -255,8 +261,9 @@ def run_ours(args, rank, world, dist):
     torch.cuda.synchronize()
     s_e2e = max_over_ranks(time.perf_counter() - t0) / args.steps
 
-    # ---- live roofline of the dominant streaming kernels (CUDA events on
-    # the solve stream; run after the results were read)
+    # ---- the stages of a cycle as kernels of their own (CUDA events on the
+    # solve stream; run after the results were read); a phase that runs in one
+    # launch does the same three stages with barriers between them
     n = ctrl.grid[0] * ctrl.grid[1] * ctrl.grid[2]
     V = sv.natv
     # the opt-in RISM3D_XFFT form of the FP32 passes: cuFFT then transforms along
@@ -309,19 +316,28 @@ def run_ours(args, rank, world, dist):
                "reps": args.cli_reps,
                "what": "bin/rism3d-b200 on the same control file, whole-process wall time "
                        "(context, file reads, solve, .xmu), as the reference executable is timed"}
-    dom = "pass_a_fp32"
-    achieved = kern[dom]["gbs"]
-    if fused:
-        dom_name, dom_kernel = "k_pass_ax_fp32", (
-            "k_pass_ax<float> (FP32 pass A with the x-axis DFTs: inverse x-DFT of the "
-            "last OZ result, AN2 update, closure, forward x-DFT)")
-    elif folded:
-        dom_name, dom_kernel = "k_plane_a_fp32", (
-            "k_plane_a<float> (FP32 plane A: AN2 update, closure, x- and y-DFT of each xy plane)")
+    # bytes of a cycle, transforms included, and the rate that the iteration of a
+    # whole solve moves them at (a mixed solve's few FP64 cycles counted as FP32)
+    step32 = sum(bpp32.values()) + (0 if folded and not fused else transform_bytes_per_point(V, 4))
+    step64 = sum(bpp64.values()) + (0 if folded else transform_bytes_per_point(V, 8))
+
+    def rate(r, step):
+        return {"ms_iterate": r["ms_iterate"], "steps": r["iterations"],
+                "model_gbs": step * n * r["iterations"] / (r["ms_iterate"] * 1e6)}
+
+    rates = {"fp64": rate(r64, step64), "mixed": rate(rm, step32)}
+    if folded and not fused:
+        # the FP32 phases are one kernel each: per step, from the solve itself
+        dom_kernel = ("k_phase<float> (a whole FP32 phase in one launch: plane A, z lines and "
+                      "plane R of every step)")
+        achieved, per, dom_bytes = rates["mixed"]["model_gbs"], "step", step32
+        traffic_pp = read_traffic("k_phase_fp32_step")
     else:
-        dom_name, dom_kernel = "k_pass_a_fp32", (
-            "k_pass_a<float> (FP32 pass A: AN2 update + closure + forward pack)")
-    traffic_pp = read_traffic(dom_name)
+        stage = max(("pass_a", "pass_k", "pass_r"), key=lambda k: kern[k + "_fp32"]["ms"])
+        dom_kernel = "FP32 %s%s" % (stage, " with the x-axis DFTs" if fused else "")
+        achieved, per, dom_bytes = kern[stage + "_fp32"]["gbs"], "launch", bpp32[stage]
+        traffic_pp = read_traffic({"pass_a": "k_pass_a_fp32", "pass_k": "k_kspace_fp32",
+                                   "pass_r": "k_pass_r_pipe_fp32"}[stage]) if not fused else None
     dmu = abs(rm["sfe_sc"] - r64["sfe_sc"])
     out = {
         "metric": METRIC, "value": ms_mixed / 1e3 / world, "unit": "s/solve",
@@ -361,7 +377,7 @@ def run_ours(args, rank, world, dist):
         "roofline": {"bound": "hbm", "kernel": dom_kernel, "achieved": achieved, "peak": hbm_peak,
                      "unit": "GB/s", "frac": achieved / hbm_peak,
                      "traffic": None if traffic_pp is None else traffic_pp * n,
-                     "algorithmic_bytes_per_launch": bpp32["pass_a"] * n,
+                     "per": per, "algorithmic_bytes": dom_bytes * n,
                      "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6650"},
         "batch": batch,
         "cli": cli,
@@ -370,20 +386,10 @@ def run_ours(args, rank, world, dist):
                     "outputs": "d mu/d(q, sigma, eps, xyz) of all "
                     "%d atoms" % len(sol.q)},
         "kernels": kern,
-        "bytes_per_iteration": {"fp64": sum(bpp64.values()) * n, "fp32": sum(bpp32.values()) * n,
+        "bytes_per_iteration": {"fp64": step64 * n, "fp32": step32 * n,
                                 "fused_pipeline_fp64": fused_pipeline_bytes_per_iter(n, V, 8),
                                 "fused_pipeline_fp32": fused_pipeline_bytes_per_iter(n, V, 4, 8)},
-        # whole-iteration rate under the per-site byte model N (31 V s + 5 s + 4)
-        # (FP32 bulk: 31 V x 4 B, the long-range terms at 8 B): bytes x steps /
-        # iteration time; above the copy peak means the fused passes move fewer
-        # bytes than that model assumes
-        "iteration_rate": {
-            "fp64": {"ms_iterate": r64["ms_iterate"], "steps": r64["iterations"],
-                     "model_gbs": fused_pipeline_bytes_per_iter(n, V, 8) * r64["iterations"]
-                     / (r64["ms_iterate"] * 1e6)},
-            "mixed": {"ms_iterate": rm["ms_iterate"], "steps": rm["iterations"],
-                      "model_gbs": n * (31 * V * 4 + 5 * 8 + 4) * rm["iterations"]
-                      / (rm["ms_iterate"] * 1e6)}},
+        "iteration_rate": rates,
         "clocks": clocks,
     }
     return out
